@@ -51,6 +51,7 @@ struct RowSink {
     int row;
     double f;
     __device__ void put(int, int, double) {}
+    __device__ void putc(int, int, double) {}
     __device__ void putv(int, int, double) {}
     __device__ void putf(int r, double x) {
         if (r == row) f = x;

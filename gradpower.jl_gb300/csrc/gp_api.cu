@@ -18,6 +18,7 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <set>
 #include <memory>
 #include <stdexcept>
 #include <string>
@@ -1552,6 +1553,20 @@ void build_clusters(gp_layout *L, const gp_problem *pr, const double *z0, const 
         }
         C.row_pos = A.upload(row_pos);
     }
+    C.n_img = A.upload(cp.n_img);
+    C.diff_mask = A.upload(cp.diff_mask);
+    C.base = A.upload(cp.base);
+    C.base_stride = cp.base_stride;
+    C.max_img = cp.max_img;
+    C.max_rb = cp.max_rb;
+    C.const_ptr = A.upload(cp.const_ptr);
+    C.const_ops = A.upload(cp.const_ops);
+    C.full_ptr = A.upload(cp.full_ptr);
+    C.full = A.upload(cp.full);
+    C.sol_ptr = A.upload(cp.sol_ptr);
+    C.sol = A.upload(cp.sol);
+    C.kc = A.alloc<double>((size_t)L->M * std::max(1, C.n_tasks) * gp::kConstSlots * 32);
+    C.img = A.alloc<double>((size_t)2 * L->M * std::max(1, C.n_tasks) * C.max_img * 32);
     C.max_slots = cp.max_slots;
     C.max_w = 1;
     for (int w : cp.cls_W) C.max_w = std::max(C.max_w, w);
@@ -1711,7 +1726,7 @@ int enqueue_solve(gp_layout *L, int variant, int *nfac_out) {
 void enqueue_eval(gp_layout *L, double tol, int itermax, const gp::LoopCtl &ctl) {
     gp::launch_reset_norm(L->P, L->W, L->Mx, L->st);
     mark(L, 0);
-    L->eval_launches = 3 + gp::launch_cluster(L->P, L->W, L->C, L->Mx, 0, L->st);
+    L->eval_launches = 3 + gp::launch_cluster(L->P, L->W, L->C, L->Mx, L->st);
     mark(L, 1);
     gp::launch_network(L->P, L->W, L->Mx, 0, L->st, L->solver == GP_SOLVER_SHARED_WOODBURY ? 1 : 0);
     mark(L, 2);
@@ -1843,7 +1858,6 @@ void ensure_mixed(gp_layout *L) {
     X.fronts = A.alloc<float>(M * L->S.front_total);
     X.lfac = A.alloc<float>(M * L->S.lu_total);
     X.ufac = A.alloc<float>(M * L->S.lu_total);
-    X.kc = A.alloc<double>(M * std::max(1, L->C.n_tasks) * gp::kConstSlots * 32);
     L->zprev = A.alloc<double>(M * L->n_sys);
     L->zprev2 = A.alloc<double>(M * L->n_sys);
     L->zprev3 = A.alloc<double>(M * L->n_sys);
@@ -1891,7 +1905,7 @@ void wb_prepare(gp_layout *L, double dt) {
        "zold");
     ck(cudaMemsetAsync(L->W.active, 1, M, L->st), "memset");
     gp::launch_reset_norm(L->P, L->W, L->Mx, L->st);
-    gp::launch_cluster(L->P, L->W, L->C, L->Mx, 0, L->st);
+    gp::launch_cluster(L->P, L->W, L->C, L->Mx, L->st);
     gp::launch_network(L->P, L->W, L->Mx, 0, L->st);
     gp::launch_dag_begin(L->D, L->st);
     gp::launch_dag_factor<double>(L->P, L->W, L->S, L->D, L->G64, L->S.fronts, L->S.lfac, L->S.ufac, L->d_only0, 1,
@@ -2021,6 +2035,14 @@ void solve_step(gp_layout *L, double dt, double tol, int itermax, bool force_ref
     }
 }
 
+// The cluster programs' constants for a call's time step and, with re-solves
+// to come, for dt = 0 (the parameters may have changed since the last call).
+void cluster_images(gp_layout *L, double dt, bool resolves) {
+    gp::launch_cluster_image(L->P, L->W, L->C, dt, L->st);
+    if (resolves) gp::launch_cluster_image(L->P, L->W, L->C, 0.0, L->st);
+    if (L->C.n_tasks > 0) L->launches += resolves ? 2 : 1;
+}
+
 // Event steps of the current fault table, and per step the scenarios whose
 // faults toggle there (they take a dt = 0 re-solve after that step).
 std::map<int, std::vector<uint8_t>> event_masks(const gp_layout *L) {
@@ -2044,7 +2066,7 @@ void adj_solve(gp_layout *L, const gp::DevAdj &A, const gp::DevClu &Csave, doubl
     launch_set_double(L->W.dt, dt, L->st);
     ck(cudaMemcpyAsync(L->W.zold, L->W.z, M * nsys * sizeof(double), cudaMemcpyDeviceToDevice, L->st), "zold");
     const DevMixed exact{};
-    launch_cluster(L->P, L->W, Csave, exact, 0, L->st);
+    launch_cluster(L->P, L->W, Csave, exact, L->st);
     launch_network(L->P, L->W, exact, 0, L->st);
     launch_adj_rhs(L->P, L->W, Csave, A, L->st);
     launch_dag_begin(L->D, L->st);
@@ -2222,7 +2244,7 @@ int32_t gp_residual(gp_layout *L, const double *zold, double dt, int32_t n_fault
     fill(L, L->W.active, 1, L->M);
     const gp::DevMixed exact{};
     gp::launch_reset_norm(L->P, L->W, exact, L->st);
-    gp::launch_cluster(L->P, L->W, L->C, exact, 1, L->st);
+    gp::launch_cluster_residual(L->P, L->W, L->C, L->st);
     gp::launch_network(L->P, L->W, exact, 1, L->st);
     ck(cudaGetLastError(), "residual launch");
     ck(cudaStreamSynchronize(L->st), "residual");
@@ -2259,11 +2281,6 @@ int32_t gp_integrate(gp_layout *L, const gp_options *opt, int32_t n_faults, cons
     const int M = L->M, ns = opt->n_steps, nsys = L->n_sys;
     set_faults(L, n_faults, faults);
     ensure_graphs(L, opt->newton_tol, opt->itermax, opt->solver);
-    if (L->Mx.on) {
-        // the parameters may have changed since the last integration
-        gp::launch_cluster_const(L->P, L->W, L->C, L->Mx, L->st);
-        L->launches += L->C.n_tasks > 0;
-    }
     ck(cudaMemsetAsync(L->W.status, 0, M * sizeof(int), L->st), "memset");
     // event steps
     std::map<int, int> ev_steps;
@@ -2276,7 +2293,11 @@ int32_t gp_integrate(gp_layout *L, const gp_options *opt, int32_t n_faults, cons
         if (L->h_tr_off_step[e] >= 0) ev_steps[L->h_tr_off_step[e]] = 1;
     }
     if (L->n_tr > 0) ck(cudaMemsetAsync(L->d_tr_on, 0, L->n_tr, L->st), "memset");
-    for (int e = 0; e < L->n_dc; e++) ev_steps[L->h_dc_on_step[e]] = 1;
+    std::set<int> dc_steps;
+    for (int e = 0; e < L->n_dc; e++) {
+        ev_steps[L->h_dc_on_step[e]] = 1;
+        dc_steps.insert(L->h_dc_on_step[e]);
+    }
     if (L->n_dc > 0) ck(cudaMemsetAsync(L->d_dc_flags, 0, L->dc_bytes, L->st), "memset");
     double *d_traj = nullptr;
     const size_t n_it = (size_t)2 * std::max(ns, 1) * M;
@@ -2347,6 +2368,7 @@ int32_t gp_integrate(gp_layout *L, const gp_options *opt, int32_t n_faults, cons
     L->retries = 0;
     for (int i = 0; i < 8; i++) L->ph_ms[i] = 0.0;
     ck(cudaMemsetAsync(L->D.err, 0, sizeof(int), L->st), "memset");
+    cluster_images(L, opt->dt, !ev_steps.empty());
     if (opt->solver == GP_SOLVER_SHARED_WOODBURY) wb_prepare(L, opt->dt);
     // the mixed solver refreshes its kept factors at the first solve and
     // around every event (the dt = 0 re-solve and the step after it); with
@@ -2384,6 +2406,8 @@ int32_t gp_integrate(gp_layout *L, const gp_options *opt, int32_t n_faults, cons
                               L->st);
             gp::launch_disconnects(L->d_dc_on_step, L->d_dc_scen, L->d_dc_idx, L->d_dc_flags, L->W.active, L->n_dc,
                                    k, L->st);
+            // an exciter that went offline changes its cluster's constants
+            if (dc_steps.count(k)) cluster_images(L, opt->dt, true);
             ck(cudaMemcpyAsync(L->W.zold, L->W.z, (size_t)M * nsys * sizeof(double), cudaMemcpyDeviceToDevice,
                                L->st),
                "zold");
@@ -2627,6 +2651,7 @@ int32_t gp_adjoint(gp_layout *L, const gp_options *opt, int32_t n_faults, const 
     ck(cudaEventCreate(&e0), "event");
     ck(cudaEventCreate(&e1), "event");
     ck(cudaEventRecord(e0, L->st), "event");
+    cluster_images(L, opt->dt, !ev.empty());
     // one forward step k; after(0) runs after the regular solve, after(1)
     // after the re-solve of the scenarios whose faults toggle at k
     auto step = [&](int k, auto after) {
@@ -3089,7 +3114,7 @@ extern "C" int32_t gp_residual_static(gp_layout *L, const double *zold, double d
     ck(cudaMemcpyAsync(W.dt, &dt, sizeof(double), cudaMemcpyHostToDevice, st), "dt");
     const gp::DevMixed exact{};
     gp::launch_reset_norm(P, W, exact, st);
-    gp::launch_cluster(P, W, L->C, exact, 1, st);
+    gp::launch_cluster_residual(P, W, L->C, st);
     gp::launch_network(P, W, exact, 1, st);
     ck(cudaGetLastError(), "residual launch");
     ck(cudaMemcpyAsync(f, W.f, M * P.n_sys * sizeof(double), cudaMemcpyDeviceToHost, st), "residual copy");

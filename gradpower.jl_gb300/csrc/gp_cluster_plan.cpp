@@ -13,8 +13,12 @@ namespace {
 
 struct PatSink {
     int ws;
-    std::set<int> *ent;
-    void put(int r, int c, double) { ent->insert((r - ws) * 32 + (c - ws)); }
+    std::set<int> *ent, *var;   // every entry; those that depend on the state
+    void put(int r, int c, double) {
+        ent->insert((r - ws) * 32 + (c - ws));
+        var->insert((r - ws) * 32 + (c - ws));
+    }
+    void putc(int r, int c, double) { ent->insert((r - ws) * 32 + (c - ws)); }
     void putv(int r, int k, double) { ent->insert((r - ws) * 32 + 29 + k); }
     void putf(int r, double) { ent->insert((r - ws) * 32 + 31); }
 };
@@ -23,18 +27,129 @@ struct DenseSink {
     int ws;
     double *a;   // [32*32]
     void put(int r, int c, double v) { a[(r - ws) * 32 + (c - ws)] = v; }
+    void putc(int r, int c, double v) { put(r, c, v); }
     void putv(int r, int k, double v) { a[(r - ws) * 32 + 29 + k] = v; }
     void putf(int r, double v) { a[(r - ws) * 32 + 31] = v; }
 };
 
+// Entries to their slots with the backward-Euler scaling: the constant ones
+// (image) or the state-dependent ones, as the device's two sinks.
 struct SlotSink {
     int ws;
     const short *slot_of;
     double *v;
-    void put(int r, int c, double x) { v[slot_of[(r - ws) * 32 + (c - ws)]] = x; }
-    void putv(int r, int k, double x) { v[slot_of[(r - ws) * 32 + 29 + k]] = x; }
-    void putf(int r, double x) { v[slot_of[(r - ws) * 32 + 31]] = x; }
+    unsigned diff;
+    double dt;
+    bool image;
+    const double *z, *zold;
+    void store(int r, int c, double x) {
+        const bool d = diff >> (r - ws) & 1;
+        if (d) x *= -dt;
+        if (d && r == c) x += 1.0;
+        v[slot_of[(r - ws) * 32 + (c - ws)]] = x;
+    }
+    void put(int r, int c, double x) {
+        if (!image) store(r, c, x);
+    }
+    void putc(int r, int c, double x) {
+        if (image) store(r, c, x);
+    }
+    void putv(int r, int k, double x) {
+        if (image) return;
+        v[slot_of[(r - ws) * 32 + 29 + k]] = diff >> (r - ws) & 1 ? -dt * x : x;
+    }
+    void putf(int r, double x) {
+        if (image) return;
+        v[slot_of[(r - ws) * 32 + 31]] = diff >> (r - ws) & 1 ? z[r] - zold[r] - dt * x : x;
+    }
 };
+
+// One operation on slots, for the scheduler.
+struct SlotOp {
+    int code, d, a, b;   // REC_*; b unused but for FMS
+};
+
+// Schedules `ops` (in program order) for kCluWarps warps: list scheduling by
+// the longest path to the end.  Within a stage no operation reads or writes
+// a slot that another one writes, so the warps need only meet between
+// stages.  The unit of length is one FP64 instruction's time on its pipe; a
+// reciprocal takes about five, and a stage without one takes up to two
+// operations a warp.
+void schedule(const std::vector<SlotOp> &ops, int n_slots, std::vector<CluRec> *out) {
+    const int n = (int)ops.size();
+    std::vector<std::vector<int>> succ(n);
+    std::vector<int> npred(n, 0), last_write(n_slots, -1);
+    std::vector<std::vector<int>> readers(n_slots);
+    auto dep = [&](int from, int to) {
+        if (from >= 0 && from != to) {
+            succ[from].push_back(to);
+            npred[to]++;
+        }
+    };
+    for (int i = 0; i < n; i++) {
+        const SlotOp &o = ops[i];
+        std::vector<int> rd = {o.a};
+        if (o.code == REC_FMS) rd.push_back(o.b);
+        for (int s : rd) dep(last_write[s], i);
+        dep(last_write[o.d], i);
+        for (int r : readers[o.d]) dep(r, i);
+        readers[o.d].clear();
+        for (int s : rd) readers[s].push_back(i);
+        last_write[o.d] = i;
+    }
+    auto len = [&](int i) { return ops[i].code == REC_RCP ? 5 : 1; };
+    std::vector<int> prio(n, 0);
+    for (int i = n - 1; i >= 0; i--) {
+        for (int j : succ[i]) prio[i] = std::max(prio[i], prio[j]);
+        prio[i] += len(i) + 1;
+    }
+    std::vector<int> ready;
+    for (int i = 0; i < n; i++)
+        if (npred[i] == 0) ready.push_back(i);
+    while (!ready.empty()) {
+        std::stable_sort(ready.begin(), ready.end(), [&](int a, int b) { return prio[a] > prio[b]; });
+        const bool rcp = ops[ready[0]].code == REC_RCP;
+        const int cap = rcp ? 5 : 2;
+        std::vector<int> take[kCluWarps], rest;
+        int load[kCluWarps] = {};
+        for (int i : ready) {
+            int w = 0;
+            for (int v = 1; v < kCluWarps; v++)
+                if (load[v] < load[w]) w = v;
+            if (load[w] + len(i) > cap) {
+                rest.push_back(i);
+                continue;
+            }
+            load[w] += len(i);
+            take[w].push_back(i);
+        }
+        for (int w = 0; w < kCluWarps; w++) {
+            std::vector<CluRec> &q = out[w];
+            for (size_t k = 0; k < take[w].size(); k++) {
+                const SlotOp &o = ops[take[w][k]];
+                CluRec r{o.d * 32, o.a * 32, o.b * 32, o.code};
+                CluRec t{0, 0, 0, 0};
+                if (o.code != REC_RCP && k + 1 < take[w].size() && ops[take[w][k + 1]].code == o.code) {
+                    const SlotOp &u = ops[take[w][++k]];
+                    t = CluRec{u.d * 32, u.a * 32, u.b * 32, 0};
+                    r.w |= u.code << 4;
+                }
+                q.push_back(r);
+                q.push_back(t);
+            }
+            if (take[w].empty()) {
+                q.push_back(CluRec{0, 0, 0, 0});
+                q.push_back(CluRec{0, 0, 0, 0});
+            }
+            q[q.size() - 2].w |= REC_SYNC;
+        }
+        for (int w = 0; w < kCluWarps; w++)
+            for (int i : take[w])
+                for (int j : succ[i])
+                    if (--npred[j] == 0) rest.push_back(j);
+        ready.swap(rest);
+    }
+}
 
 DevRef ref(const gp_device_table &T, int k) {
     DevRef d;
@@ -109,15 +224,15 @@ void make_cluster_plan(const gp_problem *pr, const double *z0, const double *u0,
     const int n_sys = net + 2 * pr->n_bus;
     std::vector<double> zz(n_sys, 0.0), uu(std::max(1, pr->n_ctrl), 0.0), pz(std::max(1, pr->n_par), 0.0);
     std::map<std::vector<int>, int> key_to_class;
-    std::vector<std::set<int>> cls_ent;
+    std::vector<std::set<int>> cls_ent, cls_var;
     std::vector<std::vector<int>> cls_loc3;
     pl.cluster_class.assign(pr->n_clusters, -1);
     std::vector<std::vector<int>> members;
     for (int c = 0; c < pr->n_clusters; c++) {
         if (pr->cl_gen[c] < 0) continue;
         const int W = pr->cl_w_size[c], ws = pr->cl_w_start[c];
-        std::set<int> ent;
-        PatSink ps{ws, &ent};
+        std::set<int> ent, var;
+        PatSink ps{ws, &ent, &var};
         double C[6], I[2];
         eval_cluster(pr, c, zz.data(), uu.data(), pz.data(), ps, C, I);
         for (int r = 0; r < W; r++)
@@ -132,12 +247,15 @@ void make_cluster_plan(const gp_problem *pr, const double *z0, const double *u0,
         for (int r = 0; r < W; r++) key.push_back(pr->is_diff[ws + r]);
         key.insert(key.end(), loc3.begin(), loc3.end());
         key.insert(key.end(), ent.begin(), ent.end());
+        key.push_back(-1);
+        key.insert(key.end(), var.begin(), var.end());
         auto it = key_to_class.find(key);
         int cls;
         if (it == key_to_class.end()) {
             cls = (int)cls_ent.size();
             key_to_class[key] = cls;
             cls_ent.push_back(ent);
+            cls_var.push_back(var);
             cls_loc3.push_back(loc3);
             pl.cls_W.push_back(W);
             pl.cls_rep.push_back(c);
@@ -160,6 +278,16 @@ void make_cluster_plan(const gp_problem *pr, const double *z0, const double *u0,
     pl.ops.clear();
     pl.max_slots = 0;
     pl.lu_flops = 0;
+    pl.n_img.clear();
+    pl.diff_mask.clear();
+    pl.const_ptr.assign(1, 0);
+    pl.const_ops.clear();
+    pl.full_ptr.assign(1, 0);
+    pl.sol_ptr.assign(1, 0);
+    pl.full.clear();
+    pl.sol.clear();
+    pl.max_img = pl.max_rb = 1;
+    std::vector<std::vector<unsigned char>> cls_base;
     const double dt_rep = 1.0 / 120.0;
     for (int cls = 0; cls < pl.n_class; cls++) {
         const int W = pl.cls_W[cls], rep = pl.cls_rep[cls], ws = pr->cl_w_start[rep];
@@ -244,12 +372,19 @@ void make_cluster_plan(const gp_problem *pr, const double *z0, const double *u0,
                         if (Q[k][j]) Q[i][j] = 1;
         }
         std::vector<std::vector<int>> slot(W, std::vector<int>(W, -1));
+        // the state-dependent entries last, after the pivot reciprocals
+        std::vector<std::vector<char>> var(W, std::vector<char>(W, 0));
+        for (int e : cls_var[cls]) var[iprow[e / 32]][ipcol[e % 32]] = 1;
         int ns = 0;
         for (int i = 0; i < W; i++)
             for (int j = 0; j < W; j++)
-                if (Q[i][j]) slot[i][j] = ns++;
-        const int inv0 = ns;
-        const int rb = inv0 + W;
+                if (Q[i][j] && !var[i][j]) slot[i][j] = ns++;
+        const int inv0 = ns, n_img = inv0 + W;
+        ns = n_img;
+        for (int i = 0; i < W; i++)
+            for (int j = 0; j < W; j++)
+                if (Q[i][j] && var[i][j]) slot[i][j] = ns++;
+        const int rb = ns;
         const int trash = rb + 3 * W;
         const int nslot = trash + 1;
         short *so = pl.slot_of.data() + (size_t)cls * 1024;
@@ -304,6 +439,72 @@ void make_cluster_plan(const gp_problem *pr, const double *z0, const double *u0,
             for (int i = 0; i < k; i++)
                 if (Q[i][k]) { op(OP_FMS3, i, slot[i][k], k); fl += 3; }
         }
+        // the device's form: operations whose operands depend on the
+        // parameters and the time step alone (const_ops, in program order),
+        // the others, and the solves of the columns with the structural
+        // zeros of the two B columns left out
+        {
+            std::vector<char> cst(rb, 1);
+            for (int k = 0; k < W; k++) cst[inv0 + k] = 0;
+            for (int sl = n_img; sl < rb; sl++) cst[sl] = 0;
+            std::vector<SlotOp> full, sol;
+            for (int q = pl.prog_mid.back(); q < pl.prog_sol.back(); q++) {
+                const CluOp &o = pl.ops[q];
+                const bool c = cst[o.a] && (o.code == OP_RCP || cst[o.d]) && (o.code != OP_FMS || cst[o.b]);
+                cst[o.d] = c;
+                if (c) pl.const_ops.push_back(o);
+                else
+                    full.push_back(SlotOp{o.code == OP_RCP ? REC_RCP : (o.code == OP_MUL ? REC_MUL : REC_FMS), o.d,
+                                          o.a, o.b});
+            }
+            pl.const_ptr.push_back((int)pl.const_ops.size());
+            std::vector<char> nz(3 * W, 0);
+            for (int r = 0; r < W; r++) {
+                nz[iprow[r]] = ent.count(r * 32 + 29) ? 1 : 0;
+                nz[W + iprow[r]] = ent.count(r * 32 + 30) ? 1 : 0;
+                nz[2 * W + iprow[r]] = 1;
+            }
+            for (int q = pl.prog_sol.back(); q < (int)pl.ops.size(); q++) {
+                const CluOp &o = pl.ops[q];
+                const int code = o.code == OP_MUL3 ? REC_MUL : REC_FMS;
+                for (int c = 0; c < 3; c++) {
+                    if (!nz[c * W + (code == REC_FMS ? o.b : o.d)]) continue;
+                    nz[c * W + o.d] = 1;
+                    full.push_back(SlotOp{code, rb + c * W + o.d, o.a, code == REC_FMS ? rb + c * W + o.b : 0});
+                }
+                // (d, b shifted past the LU slots for the dependencies)
+                sol.push_back(SlotOp{code, rb + o.d, o.a, code == REC_FMS ? rb + o.b : 0});
+            }
+            std::vector<CluRec> st[kCluWarps];
+            schedule(full, rb + 3 * W, st);
+            for (int w = 0; w < kCluWarps; w++) {
+                pl.full.insert(pl.full.end(), st[w].begin(), st[w].end());
+                pl.full_ptr.push_back((int)pl.full.size() / 2);
+                st[w].clear();
+            }
+            schedule(sol, rb + W, st);
+            for (int w = 0; w < kCluWarps; w++) {
+                for (CluRec &r : st[w]) {
+                    r.d = std::max(0, r.d - rb * 32);
+                    r.b = std::max(0, r.b - rb * 32);
+                }
+                pl.sol.insert(pl.sol.end(), st[w].begin(), st[w].end());
+                pl.sol_ptr.push_back((int)pl.sol.size() / 2);
+            }
+            std::vector<unsigned char> base(rb, 0);
+            unsigned dm = 0;
+            for (int r = 0; r < W; r++)
+                if (isd[r]) {
+                    dm |= 1u << r;
+                    base[slot[iprow[r]][ipcol[r]]] |= 1;
+                }
+            for (int k = 0; k < W; k++) base[slot[k][k]] |= 2;
+            cls_base.push_back(base);
+            pl.diff_mask.push_back(dm);
+            pl.n_img.push_back(n_img);
+            pl.max_img = std::max(pl.max_img, n_img);
+            pl.max_rb = std::max(pl.max_rb, rb);
+        }
         pl.prog_ptr.push_back((int)pl.ops.size());
         pl.rhs_base.push_back(rb);
         pl.nslot.push_back(nslot);
@@ -312,6 +513,10 @@ void make_cluster_plan(const gp_problem *pr, const double *z0, const double *u0,
         for (int t = 0; t < 3; t++) pl.pos3[(size_t)cls * 3 + t] = ipcol[cls_loc3[cls][t]];
         pl.lu_flops += fl * (int64_t)members[cls].size();
     }
+    pl.base_stride = pl.max_rb;
+    pl.base.assign((size_t)std::max(1, pl.n_class) * pl.base_stride, 0);
+    for (int cls = 0; cls < pl.n_class; cls++)
+        std::copy(cls_base[cls].begin(), cls_base[cls].end(), pl.base.begin() + (size_t)cls * pl.base_stride);
     // warp tasks: 32 clusters of one class, the classes with the most slots
     // (the longest programs) first, so that the warps that start last are
     // the short ones
@@ -339,43 +544,48 @@ double host_cluster_run(const gp_problem *pr, const ClusterPlan &pl, int c, cons
     if (cls < 0) throw std::runtime_error("trivial cluster has no program");
     const int W = pl.cls_W[cls], ws = pr->cl_w_start[c];
     std::vector<double> v(pl.nslot[cls], 0.0);
-    SlotSink s{ws, pl.slot_of.data() + (size_t)cls * 1024, v.data()};
-    double C[6], I[2];
-    eval_cluster(pr, c, z, u0, p, s, C, I);
     const int rb = pl.rhs_base[cls];
     double *R0 = v.data() + rb, *R1 = R0 + W, *R2 = R1 + W;
-    for (int q = pl.prog_ptr[cls]; q < pl.prog_mid[cls]; q++) {
-        const CluOp &o = pl.ops[q];
-        if (o.code == OP_SCL) v[o.d] *= -dt;
-        else if (o.code == OP_DIAG) v[o.d] += 1.0;
-        else if (o.code == OP_BEF) v[o.d] = z[ws + o.a] - zold[ws + o.a] - dt * v[o.d];
-        if ((o.code == OP_BEF || o.code == OP_ROW) && f_out) f_out[o.a] = v[o.d];
+    // the constant entries and their part of the factorisation, taken at
+    // another state (as on the device, whose image is of an earlier one): an
+    // entry wrongly marked constant shows
+    std::vector<double> z_img(z, z + pr->n_diff + pr->n_alg + 2 * pr->n_bus);
+    for (double &x : z_img) x = 0.37 - 0.6 * x;
+    const unsigned char *base = pl.base.data() + (size_t)cls * pl.base_stride;
+    for (int s = 0; s < rb; s++)
+        if (base[s] & 1) v[s] = 1.0;
+    double C[6], I[2];
+    SlotSink si{ws, pl.slot_of.data() + (size_t)cls * 1024, v.data(), pl.diff_mask[cls], dt, true, z, zold};
+    eval_cluster(pr, c, z_img.data(), u0, p, si, C, I);
+    for (int q = pl.const_ptr[cls]; q < pl.const_ptr[cls + 1]; q++) {
+        const CluOp &o = pl.const_ops[q];
+        if (o.code == OP_RCP) v[o.d] = 1.0 / v[o.a];
+        else if (o.code == OP_MUL) v[o.d] *= v[o.a];
+        else v[o.d] -= v[o.a] * v[o.b];
     }
+    // the state-dependent entries and the residual
+    si.image = false;
+    eval_cluster(pr, c, z, u0, p, si, C, I);
     double fmax = 0.0;
     for (int j = 0; j < W; j++) fmax = std::max(fmax, std::fabs(R2[j]));
-    for (int q = pl.prog_mid[cls]; q < pl.prog_ptr[cls + 1]; q++) {
-        const CluOp &o = pl.ops[q];
-        switch (o.code) {
-        case OP_RCP: v[o.d] = 1.0 / v[o.a]; break;
-        case OP_MUL: v[o.d] *= v[o.a]; break;
-        case OP_FMS: v[o.d] -= v[o.a] * v[o.b]; break;
-        case OP_FMS3: {
-            const double l = v[o.a];
-            R0[o.d] -= l * R0[o.b];
-            R1[o.d] -= l * R1[o.b];
-            R2[o.d] -= l * R2[o.b];
-            break;
-        }
-        case OP_MUL3: {
-            const double l = v[o.a];
-            R0[o.d] *= l;
-            R1[o.d] *= l;
-            R2[o.d] *= l;
-            break;
-        }
-        default: break;
-        }
-    }
+    if (f_out)
+        for (int r = 0; r < W; r++) f_out[r] = v[pl.slot_of[(size_t)cls * 1024 + r * 32 + 31]];
+    // the staged operations, stage by stage, the last warp's share first
+    int pos[kCluWarps];
+    for (int w = 0; w < kCluWarps; w++) pos[w] = pl.full_ptr[(size_t)cls * kCluWarps + w];
+    while (pos[0] < pl.full_ptr[(size_t)cls * kCluWarps + 1])
+        for (int w = kCluWarps - 1; w >= 0; w--)
+            for (bool more = true; more;) {
+                const CluRec *r = pl.full.data() + 2 * (size_t)pos[w]++;
+                for (int h = 0; h < 2; h++) {
+                    const int code = h ? r[0].w >> 4 & 15 : r[0].w & 15;
+                    double &d = v[r[h].d / 32];
+                    if (code == REC_FMS) d -= v[r[h].a / 32] * v[r[h].b / 32];
+                    else if (code == REC_MUL) d *= v[r[h].a / 32];
+                    else if (code == REC_RCP) d = 1.0 / v[r[h].a / 32];
+                }
+                more = !(r[0].w & REC_SYNC);
+            }
     for (int j = 0; j < W; j++) {
         const int st = pl.perm_col[(size_t)cls * 32 + j];
         yx[st] = R2[j];

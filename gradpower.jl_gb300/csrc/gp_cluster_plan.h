@@ -27,6 +27,25 @@ struct ClusterPlan {
     std::vector<int> prog_ptr, prog_mid, prog_sol, rhs_base, nslot, perm_col, pos3;
     std::vector<CluOp> ops;
     int64_t lu_flops = 0;                            // per scenario, all clusters (FMA count)
+    // The device's form of the programs.  Slots of a class: [0, n_img) the
+    // LU entries no state-dependent Jacobian entry falls on, and the pivot
+    // reciprocals (kept per scenario, with the constant part of the
+    // factorisation done: const_ops); [n_img, rhs_base) the state-dependent
+    // LU entries; then the three right-hand-side columns.
+    std::vector<int> n_img;                          // [n_class]
+    std::vector<unsigned> diff_mask;                 // [n_class] bit r: local row r is differential
+    std::vector<unsigned char> base;                 // [class][max rhs_base] bit 0: a differential row's diagonal
+                                                     // entry, bit 1: a pivot
+    int base_stride = 1;
+    std::vector<int> const_ptr;                      // [n_class+1]
+    std::vector<CluOp> const_ops;
+    // the rest of the factorisation with the three solves (full), and one
+    // solve alone (sol: column 2's operations, slots relative to rhs_base +
+    // 2 W for d and b), each scheduled for kCluWarps warps in stages with a
+    // barrier after each: per (class, warp) a stream of record pairs
+    std::vector<int> full_ptr, sol_ptr;              // [n_class * kCluWarps + 1], in record pairs
+    std::vector<CluRec> full, sol;
+    int max_img = 1, max_rb = 1;
 };
 
 void make_cluster_plan(const gp_problem *pr, const double *z0, const double *u0, const double *p,

@@ -127,6 +127,18 @@ struct DevClu {
     const int *row_pos;         // [class][32] position of local row r in the program
     int max_slots;
     int max_w;                  // widest class
+    // the scheduled programs and the parts kept over an integration (see
+    // gp_cluster_plan.h and cluster_kernel)
+    const int *n_img;           // [n_class]
+    const unsigned *diff_mask;  // [n_class]
+    const unsigned char *base;  // [class][base_stride]
+    int base_stride, max_img, max_rb;
+    const int *const_ptr;       // [n_class+1]
+    const CluOp *const_ops;
+    const int *full_ptr, *sol_ptr;   // [n_class * kCluWarps + 1] record pairs
+    const CluRec *full, *sol;
+    double *kc;                 // [M][n_tasks][kConstSlots][32] parameter constants of the cluster devices
+    double *img;                // [2][M][n_tasks][max_img][32] constant slots for the call's dt and for dt = 0
     // adjoint: when set, the cluster kernel also saves its FP64 LU values
     // ([M][n_tasks][n_save][32]) and the coupling rows C ([M][n_cl][6])
     double *save_lu, *save_cc;
@@ -163,7 +175,6 @@ struct DevMixed {
     float *cc;             // [M][n_cl][6] coupling rows of the network equations
     float *fronts;         // [M][front_total] reduced-system fronts (update matrices for the assembly)
     float *lfac, *ufac;    // [M][lu_total] solve-ordered FP32 factors (DevSym::lu_off)
-    double *kc;            // [M][n_tasks][kConstSlots][32] parameter constants of the cluster devices
 };
 
 // Dataflow schedule of the multifrontal factorisation and solves
@@ -328,11 +339,13 @@ void launch_disconnects(const int *on_step, const int *scen, const int *idx, uin
 // Parameter products of the ZIP loads for network_kernel; rerun whenever
 // the parameter vectors change.
 void launch_zip_const(const DevProblem &P, const DevWork &W, double *out, cudaStream_t st);
-// Parameter constants of the cluster devices for cluster_keep_kernel.
-void launch_cluster_const(const DevProblem &P, const DevWork &W, const DevClu &C, const DevMixed &Mx,
-                          cudaStream_t st);
-int launch_cluster(const DevProblem &P, const DevWork &W, const DevClu &C, const DevMixed &Mx, int want_f,
-                    cudaStream_t st);
+// Parameter constants and constant slots of the cluster programs for the
+// time step dt (the call's, or 0 for the re-solves): before the first
+// evaluation of a call with that time step, and again after a disconnection.
+void launch_cluster_image(const DevProblem &P, const DevWork &W, const DevClu &C, double dt, cudaStream_t st);
+int launch_cluster(const DevProblem &P, const DevWork &W, const DevClu &C, const DevMixed &Mx, cudaStream_t st);
+// The clusters' residual rows alone (the parity probes).
+void launch_cluster_residual(const DevProblem &P, const DevWork &W, const DevClu &C, cudaStream_t st);
 // skip_s: the entries of S are not needed (shared-factor Woodbury path)
 void launch_network(const DevProblem &P, const DevWork &W, const DevMixed &Mx, int want_f, cudaStream_t st,
                     int skip_s = 0);

@@ -1,12 +1,11 @@
 // Device kernels of the batched backward-Euler Newton step.
 //
-//  cluster_kernel  one warp per (generator cluster, scenario): evaluates
+//  cluster_kernel  one lane per (generator cluster, scenario): evaluates
 //                  the cluster's residual rows and Jacobian block
 //                  [A_k | B_k] (src/kernels/{genrou,ieesgo,tgov1,sexs,
 //                  esdc1a,ieeest}.jl), applies the backward-Euler scaling
-//                  (src/dynamics.jl:366-391, 481-500), factors A_k with
-//                  partial pivoting held in registers (one row per lane) and
-//                  returns A_k^-1 f_k, A_k^-1 B_k and the Schur terms
+//                  (src/dynamics.jl:366-391, 481-500), factors A_k by its
+//                  class's static-pivot sparse program and returns A_k^-1 f_k, A_k^-1 B_k and the Schur terms
 //                  C_k A_k^-1 B_k, C_k A_k^-1 f_k (src/schur.jl:195-247,
 //                  324-346) — the reference's gather + cuBLAS getrf/getrs
 //                  sequence (ext/GradPowerCUDAExt/GradPowerCUDAExt.jl:1825-1887,
@@ -47,23 +46,30 @@ __device__ __forceinline__ unsigned long long norm_bits(double v) {
 }
 
 // ---------------------------------------------------------------------------
-// cluster kernel: one lane per (cluster, scenario), 32 clusters of one
-// pattern class per warp; the class program does the backward-Euler scaling,
-// the static-pivot sparse LU and the solves for [B(:,vr) B(:,vi) f].
+// cluster kernels: one lane per (cluster, scenario), 32 clusters of one
+// pattern class per warp task, a task run by the kCluWarps warps of a CTA.
+//
+// What bounds them.  GB300's FP64 pipe takes 64 cycles of an SM
+// sub-partition per warp instruction (19 per SM with all four busy, both
+// whatever the active lanes), so a task on one warp is a serial chain of its
+// FP64 instructions at 64 cycles each plus the shared-memory round trips
+// between them, and the FP64 instruction count is what the throughput limit
+// is made of.  Hence
+//  - the entries of a cluster block that depend on the parameters and the
+//    time step alone, and the part of the factorisation that only touches
+//    them, are computed once per integration (cluster_image_kernel; the
+//    reciprocals of parameters likewise, DevClu::kc);
+//  - the devices of a cluster are evaluated by different warps, and the
+//    rest of the factorisation and the three solves is scheduled on the host
+//    over the four warps in stages (gp_cluster_plan.cpp), so that a task
+//    uses all four sub-partitions;
+//  - structurally zero operations on the two B columns are left out.
+// Every slot receives the operations it always did, in the same order.
+// Measured, one FP64 evaluation, one warp a task and the whole program each
+// time -> this: one cluster (2 buses) 60 -> 23 us, 25,600 clusters (2,000
+// buses x 64) 180 -> 73 us, 40,000 (70,000 buses x 8) 203 -> 88 us; the
+// mixed solver's (mostly kept factors) 70,000 x 8 85 -> 58 us.
 // ---------------------------------------------------------------------------
-
-struct LaneSink {
-    double *v;             // vals[slot * 32 + lane]
-    const short *slot_of;  // class map, local (r, c) -> slot
-    int ws, lane;
-    __device__ __forceinline__ void put(int r, int c, double x) {
-        v[(int)slot_of[(r - ws) * 32 + (c - ws)] * 32 + lane] = x;
-    }
-    __device__ __forceinline__ void putv(int r, int k, double x) {
-        v[(int)slot_of[(r - ws) * 32 + 29 + k] * 32 + lane] = x;
-    }
-    __device__ __forceinline__ void putf(int r, double x) { v[(int)slot_of[(r - ws) * 32 + 31] * 32 + lane] = x; }
-};
 
 __device__ __forceinline__ DevRef devref(const DTab &T, int k) {
     DevRef d;
@@ -77,95 +83,202 @@ __device__ __forceinline__ DevRef devref(const DTab &T, int k) {
     return d;
 }
 
-// The cluster's device table entries are read first, all together, so that
-// their round trips overlap instead of each device's starting after the
-// previous device's equations.
-template <class Sink, class KP = ComputeK>
-__device__ __forceinline__ void eval_cluster(const DevProblem &P, int c, const double *z, const double *u0,
-                                             const double *p, Sink &sink, double Cc[6], double Ic[2],
-                                             const KP &kc = KP(), bool exc_on = true) {
-    const int gt = P.cl_gov_type[c], et0 = P.cl_exc_type[c], ip = P.cl_pss[c];
-    const int ig = P.cl_gen[c], igv = P.cl_gov[c], iex = P.cl_exc[c];
-    const int et = exc_on ? et0 : -1;   // an offline exciter's states hold
-    const DevRef dg = devref(P.dev[0], ig);
-    DevRef dgv{}, dex{}, dps{};
-    if (gt == 1 || gt == 2) dgv = devref(P.dev[gt], igv);
-    if (et == 3 || et == 4) dex = devref(P.dev[et], iex);
-    if (ip >= 0) dps = devref(P.dev[5], ip);
-    genrou_eval(dg, P.net, z, u0, p, sink, Cc, Ic, kc);
-    if (gt == 1) ieesgo_eval(dgv, z, p, sink, kc);
-    else if (gt == 2) tgov1_eval(dgv, z, p, sink, kc);
-    if (et == 3) sexs_eval(dex, P.net, z, p, sink, kc);
-    else if (et == 4) esdc1a_eval(dex, P.net, z, p, sink, kc);
-    if (ip >= 0) ieeest_eval(dps, z, p, sink, kc);
+// The warps' shares of a cluster's evaluation: 0 the machine's flux rows, 1
+// its network-frame rows (C, I) and the exciter, 2 the governor, 3 the
+// stabiliser.  `off` receives the entries of an offline exciter.
+template <class Sink, class Off, class KP>
+__device__ __forceinline__ void eval_share(const DevProblem &P, int c, int share, const double *z, const double *u0,
+                                           const double *p, Sink &sink, Off &off, double Cc[6], double Ic[2],
+                                           const KP &kc, bool exc_on) {
+    if (share == 0) {
+        genrou_flux(devref(P.dev[0], P.cl_gen[c]), z, u0, p, sink, kc);
+    } else if (share == 1) {
+        const int et = P.cl_exc_type[c], iex = P.cl_exc[c];
+        const DevRef dg = devref(P.dev[0], P.cl_gen[c]);
+        DevRef dex{};
+        if (et == 3 || et == 4) dex = devref(P.dev[et], iex);
+        genrou_stator(dg, P.net, z, sink, Cc, Ic);
+        if (exc_on) {
+            if (et == 3) sexs_eval(dex, P.net, z, p, sink, kc);
+            else if (et == 4) esdc1a_eval(dex, P.net, z, p, sink, kc);
+        } else {
+            if (et == 3) sexs_eval(dex, P.net, z, p, off, kc);
+            else if (et == 4) esdc1a_eval(dex, P.net, z, p, off, kc);
+        }
+    } else if (share == 2) {
+        const int gt = P.cl_gov_type[c], igv = P.cl_gov[c];
+        if (gt == 1) ieesgo_eval(devref(P.dev[1], igv), z, p, sink, kc);
+        else if (gt == 2) tgov1_eval(devref(P.dev[2], igv), z, p, sink, kc);
+    } else {
+        const int ip = P.cl_pss[c];
+        if (ip >= 0) ieeest_eval(devref(P.dev[5], ip), z, p, sink, kc);
+    }
 }
 
-// Sink that drops every entry (the evaluation of the parameter constants).
-struct NullSink {
+__device__ __forceinline__ bool exciter_on(const DevProblem &P, int m, int c) {
+    return !P.exc_off || !P.exc_off[(size_t)m * P.n_cl + c];
+}
+
+// Image of the constant entries: the slot keeps the entry with the
+// backward-Euler scaling (rows of the class's differential mask) and the
+// diagonal's one.  ON false: an offline exciter, whose rows hold (the
+// entries are zero, the diagonal one).
+template <bool ON>
+struct ImageSink {
+    double *v;             // vals[slot * 32 + lane]
+    const short *slot_of;  // class map, local (r, c) -> slot
+    int ws, lane;
+    unsigned diff;
+    double dt;
     __device__ __forceinline__ void put(int, int, double) {}
+    __device__ __forceinline__ void putc(int r, int c, double x) {
+        const int lr = r - ws;
+        const bool d = diff >> lr & 1;
+        double y = ON ? x : 0.0;
+        if (d) y = __dmul_rn(y, -dt);
+        if (d && r == c) y = __dadd_rn(y, 1.0);
+        v[(int)slot_of[lr * 32 + (c - ws)] * 32 + lane] = y;
+    }
     __device__ __forceinline__ void putv(int, int, double) {}
     __device__ __forceinline__ void putf(int, double) {}
 };
 
-// Parameter constants of every cluster's devices for every scenario, stored
-// for cluster_keep_kernel (they depend on the parameters alone; run once per
-// integration, after the parameters are set).
-__global__ void __launch_bounds__(32) cluster_const_kernel(DevProblem P, DevWork W, DevClu Cl, DevMixed Mx) {
+// State-dependent entries, the B columns and the backward-Euler residual
+// (its norm in nb).  Same scaling as ImageSink.
+template <bool ON>
+struct LaneSink {
+    double *v;
+    const short *slot_of;
+    const double *z, *zold;
+    int ws, lane;
+    unsigned diff;
+    double dt;
+    unsigned long long *nb;
+    __device__ __forceinline__ void put(int r, int c, double x) {
+        const int lr = r - ws;
+        const bool d = diff >> lr & 1;
+        double y = ON ? x : 0.0;
+        if (d) y = __dmul_rn(y, -dt);
+        if (d && r == c) y = __dadd_rn(y, 1.0);
+        v[(int)__ldg(slot_of + lr * 32 + (c - ws)) * 32 + lane] = y;
+    }
+    __device__ __forceinline__ void putc(int, int, double) {}
+    __device__ __forceinline__ void putv(int r, int k, double x) {
+        const int lr = r - ws;
+        double y = ON ? x : 0.0;
+        if (diff >> lr & 1) y = __dmul_rn(y, -dt);
+        v[(int)__ldg(slot_of + lr * 32 + 29 + k) * 32 + lane] = y;
+    }
+    __device__ __forceinline__ void putf(int r, double x) {
+        const int lr = r - ws;
+        double y = ON ? x : 0.0;
+        if (diff >> lr & 1) y = z[r] - zold[r] - dt * y;
+        v[(int)__ldg(slot_of + lr * 32 + 31) * 32 + lane] = y;
+        const unsigned long long t = norm_bits(y);
+        *nb = t > *nb ? t : *nb;
+    }
+};
+
+// Once per integration, one warp per (task, scenario): the parameter
+// constants (DevClu::kc) and, for the call's time step (which = 0) and the
+// dt = 0 re-solves (which = 1), the constant slots with their part of the
+// factorisation done.  Rerun after a disconnection.
+__global__ void __launch_bounds__(32) cluster_image_kernel(DevProblem P, DevWork W, DevClu Cl, double dt, int which) {
+    extern __shared__ double vals[];
     const int task = blockIdx.x, m = blockIdx.y, lane = threadIdx.x;
-    if (lane >= Cl.task_count[task]) return;
-    const int c = Cl.order[Cl.task_first[task] + lane];
-    const double *z = W.z + (size_t)m * P.n_sys;
-    double Cc[6], Ic[2];
-    NullSink sink;
-    RecordK rk{Mx.kc + (((size_t)m * Cl.n_tasks + task) * kConstSlots) * 32 + lane, 32};
-    eval_cluster(P, c, z, W.u0 + (size_t)m * P.n_ctrl, W.p + (size_t)m * P.n_par, sink, Cc, Ic, rk);
+    const int cls = Cl.task_class[task];
+    const bool act = lane < Cl.task_count[task];
+    const int c = Cl.order[Cl.task_first[task] + (act ? lane : 0)];
+    const int rb = Cl.rhs_base[cls], n_img = Cl.n_img[cls];
+    const unsigned char *base = Cl.base + (size_t)cls * Cl.base_stride;
+    // (idle lanes factor an identity, so that none divides by zero)
+    for (int s = 0; s < rb; s++) vals[s * 32 + lane] = base[s] & (act ? 1 : 2) ? 1.0 : 0.0;
+    if (act) {
+        const short *so = Cl.slot_of + (size_t)cls * 1024;
+        const int ws = P.cl_w_start[c];
+        const unsigned diff = Cl.diff_mask[cls];
+        ImageSink<true> on{vals, so, ws, lane, diff, dt};
+        ImageSink<false> off{vals, so, ws, lane, diff, dt};
+        const double *z = W.z + (size_t)m * P.n_sys, *u0 = W.u0 + (size_t)m * P.n_ctrl,
+                     *p = W.p + (size_t)m * P.n_par;
+        double Cc[6], Ic[2];
+        const bool exc = exciter_on(P, m, c);
+        const RecordK rk{Cl.kc + (((size_t)m * Cl.n_tasks + task) * kConstSlots) * 32 + lane, 32};
+        for (int s = 0; s < kCluWarps; s++) eval_share(P, c, s, z, u0, p, on, off, Cc, Ic, rk, exc);
+    }
+    for (int q = Cl.const_ptr[cls]; q < Cl.const_ptr[cls + 1]; q++) {
+        const CluOp o = Cl.const_ops[q];
+        double *d = vals + o.d * 32 + lane;
+        if (o.code == OP_RCP) *d = recip(vals[o.a * 32 + lane]);
+        else if (o.code == OP_MUL) *d *= vals[o.a * 32 + lane];
+        else *d -= vals[o.a * 32 + lane] * vals[o.b * 32 + lane];
+    }
+    double *img = Cl.img + ((((size_t)which * P.M + m) * Cl.n_tasks + task) * Cl.max_img) * 32 + lane;
+    for (int s = 0; s < n_img; s++) img[(size_t)s * 32] = vals[s * 32 + lane];
 }
 
-// The factorisation part of a class program and the solves of the three
-// right-hand-side columns R0, R1 (B) and R2 (f), on one lane's slots.
+// A staged stream of record pairs (CluRec) by one of the task's warps: v0 +
+// offsets for d and b, va + offsets for a.  The next pair is read ahead.
 template <class T>
-__device__ __forceinline__ void clu_program(T *vals, T *R0, T *R1, T *R2, const CluOp *ops, int qm, int q1,
-                                            int lane) {
-    for (int q = qm; q < q1; q++) {
-        const CluOp o = ops[q];
-        switch (o.code) {
-        case OP_RCP:
-            vals[o.d * 32 + lane] = recip(vals[o.a * 32 + lane]);
-            break;
-        case OP_MUL:
-            vals[o.d * 32 + lane] *= vals[o.a * 32 + lane];
-            break;
-        case OP_FMS:
-            vals[o.d * 32 + lane] -= vals[o.a * 32 + lane] * vals[o.b * 32 + lane];
-            break;
-        case OP_FMS3: {
-            const T l = vals[o.a * 32 + lane];
-            R0[o.d * 32 + lane] -= l * R0[o.b * 32 + lane];
-            R1[o.d * 32 + lane] -= l * R1[o.b * 32 + lane];
-            R2[o.d * 32 + lane] -= l * R2[o.b * 32 + lane];
-            break;
+__device__ __forceinline__ void run_stages(const int4 *q, int n, T *v0, const T *va, int lane) {
+    v0 += lane;
+    va += lane;
+    int4 r0 = __ldg(q), r1 = __ldg(q + 1);
+    for (int i = 0; i < n; i++) {
+        const int4 c0 = r0, c1 = r1;
+        if (i + 1 < n) {
+            r0 = __ldg(q + 2 * i + 2);
+            r1 = __ldg(q + 2 * i + 3);
         }
-        case OP_MUL3: {
-            const T l = vals[o.a * 32 + lane];
-            R0[o.d * 32 + lane] *= l;
-            R1[o.d * 32 + lane] *= l;
-            R2[o.d * 32 + lane] *= l;
-            break;
+        const int code = c0.w & 255;
+        if (code == (REC_FMS | REC_FMS << 4)) {
+            const T a0 = va[c0.y], b0 = v0[c0.z], a1 = va[c1.y], b1 = v0[c1.z];
+            T d0 = v0[c0.x], d1 = v0[c1.x];
+            d0 -= a0 * b0;
+            d1 -= a1 * b1;
+            v0[c0.x] = d0;
+            v0[c1.x] = d1;
+        } else if (code == REC_FMS) {
+            v0[c0.x] -= va[c0.y] * v0[c0.z];
+        } else if (code == REC_MUL) {
+            v0[c0.x] *= va[c0.y];
+        } else if (code == (REC_MUL | REC_MUL << 4)) {
+            const T a0 = va[c0.y], a1 = va[c1.y];
+            const T d0 = v0[c0.x], d1 = v0[c1.x];
+            v0[c0.x] = d0 * a0;
+            v0[c1.x] = d1 * a1;
+        } else if (code == REC_RCP) {
+            v0[c0.x] = recip(va[c0.y]);
         }
-        default:
-            break;
-        }
+        if (c0.w & REC_SYNC) __syncthreads();
     }
 }
+
+__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+
+// Warp maximum of ordered norm bits.
+__device__ __forceinline__ unsigned long long warp_max(unsigned long long v) {
+    const unsigned hi = (unsigned)(v >> 32), lo = (unsigned)v;
+    const unsigned mh = __reduce_max_sync(FULL_MASK, hi);
+    const unsigned ml = __reduce_max_sync(FULL_MASK, hi == mh ? lo : 0u);
+    return (unsigned long long)mh << 32 | ml;
+}
+
+constexpr int kCluThreads = 32 * kCluWarps;
 
 // Modes per scenario: 0 exact Newton (Jacobian block, FP64 LU, three solves;
 // also the mixed solver's MX_EXACT); 1 the same, and the LU values and
 // coupling rows are kept in FP32 for the following iterations (MX_FP32).
 // The mixed solver's MX_KEEP scenarios (residual only, solved with the kept
 // FP32 LU) run cluster_keep_kernel instead.
-__global__ void __launch_bounds__(32) cluster_kernel(DevProblem P, DevWork W, DevClu Cl, DevMixed Mx, int want_f) {
-    extern __shared__ double vals[];
-    const int task = blockIdx.x, m = blockIdx.y, lane = threadIdx.x;
+__global__ void __launch_bounds__(kCluThreads, 4) cluster_kernel(DevProblem P, DevWork W, DevClu Cl, DevMixed Mx) {
+    extern __shared__ __align__(16) double vals[];
+    __shared__ unsigned long long s_nb[kCluWarps];
+    const int task = blockIdx.x, m = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (!W.active[m]) return;
     const int r = Mx.on ? Mx.refac[m] : MX_EXACT;
     if (r == MX_KEEP) return;
@@ -173,98 +286,86 @@ __global__ void __launch_bounds__(32) cluster_kernel(DevProblem P, DevWork W, De
     const int cls = Cl.task_class[task];
     const int cnt = Cl.task_count[task];
     const bool act = lane < cnt;
-    const int c = act ? Cl.order[Cl.task_first[task] + lane] : Cl.order[Cl.task_first[task]];
+    const int c = Cl.order[Cl.task_first[task] + (act ? lane : 0)];
     const int ws = P.cl_w_start[c], Wn = P.cl_w_size[c];
-    const int nslot = Cl.nslot[cls];
-    for (int s = 0; s < nslot; s++) vals[s * 32 + lane] = 0.0;
-    const double *z = W.z + (size_t)m * P.n_sys;
-    const double *zold = W.zold + (size_t)m * P.n_sys;
-    const double *u0 = W.u0 + (size_t)m * P.n_ctrl;
-    const double *p = W.p + (size_t)m * P.n_par;
-    double Cc[6] = {0, 0, 0, 0, 0, 0}, Ic[2] = {0, 0};
-    const CluOp *ops = Cl.ops;
-    const int q0 = Cl.prog_ptr[cls], qm = Cl.prog_mid[cls], q1 = Cl.prog_ptr[cls + 1];
-    if (act) {
-        LaneSink sink{vals, Cl.slot_of + (size_t)cls * 1024, ws, lane};
-        eval_cluster(P, c, z, u0, p, sink, Cc, Ic, ComputeK(), !P.exc_off || !P.exc_off[(size_t)m * P.n_cl + c]);
-    } else {
-        // idle lanes factor an identity so that no lane divides by zero
-        for (int q = qm; q < q1; q++)
-            if (ops[q].code == OP_RCP) vals[ops[q].a * 32 + lane] = 1.0;
-    }
+    const int rb = Cl.rhs_base[cls], n_img = Cl.n_img[cls];
     const double dt = *W.dt;
-    const int rb = Cl.rhs_base[cls];
+    // the constant slots arrive while the devices are evaluated
+    {
+        const double *img = Cl.img + ((((size_t)(dt == 0.0) * P.M + m) * Cl.n_tasks + task) * Cl.max_img) * 32;
+        for (int e = tid; e < n_img * 16; e += kCluThreads) cp_async16(vals + 2 * e, img + 2 * e);
+    }
     double *R0 = vals + (size_t)rb * 32, *R1 = R0 + (size_t)Wn * 32, *R2 = R1 + (size_t)Wn * 32;
-    // backward-Euler scaling, eight ops and their state loads in flight
-    for (int q = q0; q < qm; q += 8) {
-        CluOp o[8];
-        double zn[8], zo[8];
-#pragma unroll
-        for (int u = 0; u < 8; u++) o[u] = ops[min(q + u, qm - 1)];
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const bool ld = act && q + u < qm && o[u].code == OP_BEF;
-            zn[u] = ld ? z[ws + o[u].a] : 0.0;
-            zo[u] = ld ? zold[ws + o[u].a] : 0.0;
-        }
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-            if (q + u >= qm) break;
-            double *vd = vals + o[u].d * 32 + lane;
-            if (o[u].code == OP_SCL) *vd *= -dt;
-            else if (o[u].code == OP_DIAG) *vd += 1.0;
-            else if (o[u].code == OP_BEF) *vd = act ? zn[u] - zo[u] - dt * *vd : 0.0;
-        }
+    for (int e = tid; e < 2 * Wn * 32; e += kCluThreads) R0[e] = 0.0;
+    if (!act) {
+        // idle lanes factor an identity so that none divides by zero
+        const unsigned char *base = Cl.base + (size_t)cls * Cl.base_stride;
+        for (int s = n_img + warp; s < rb; s += kCluWarps) vals[s * 32 + lane] = base[s] & 2 ? 1.0 : 0.0;
+        for (int j = warp; j < Wn; j += kCluWarps) R2[j * 32 + lane] = 0.0;
     }
-    // residual norm (and the residual itself for the parity probe)
-    const int *pc = Cl.perm_col + cls * 32;
+    __syncthreads();
+    double Cc[6] = {0, 0, 0, 0, 0, 0}, Ic[2] = {0, 0};   // warp 1
     unsigned long long nb = 0ull;
-    for (int j = 0; j < Wn; j++) {
-        const unsigned long long t = norm_bits(R2[j * 32 + lane]);
-        nb = t > nb ? t : nb;
+    if (act) {
+        const double *z = W.z + (size_t)m * P.n_sys, *zold = W.zold + (size_t)m * P.n_sys;
+        const short *so = Cl.slot_of + (size_t)cls * 1024;
+        const unsigned diff = Cl.diff_mask[cls];
+        LaneSink<true> on{vals, so, z, zold, ws, lane, diff, dt, &nb};
+        LaneSink<false> off{vals, so, z, zold, ws, lane, diff, dt, &nb};
+        const LoadK lk{Cl.kc + (((size_t)m * Cl.n_tasks + task) * kConstSlots) * 32 + lane, 32};
+        eval_share(P, c, warp, z, W.u0 + (size_t)m * P.n_ctrl, W.p + (size_t)m * P.n_par, on, off, Cc, Ic, lk,
+                   exciter_on(P, m, c));
     }
-    if (!act) nb = 0ull;
-    if (want_f && act) {
-        // R2 is indexed by pivot position; OP_BEF / OP_ROW name the local row
-        // whose residual each position holds
-        for (int q = q0; q < qm; q++)
-            if (ops[q].code == OP_BEF || ops[q].code == OP_ROW)
-                W.f[(size_t)m * P.n_sys + ws + ops[q].a] = vals[ops[q].d * 32 + lane];
-    }
+    nb = warp_max(nb);
+    if (lane == 0) s_nb[warp] = nb;
+    cp_async_wait();
+    __syncthreads();
+    if (tid == 0) {
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        const unsigned long long o = __shfl_xor_sync(FULL_MASK, nb, off);
-        nb = o > nb ? o : nb;
+        for (int w = 1; w < kCluWarps; w++) nb = s_nb[w] > nb ? s_nb[w] : nb;
+        atomicMax(W.norm + m, nb);
     }
-    if (lane == 0) atomicMax(W.norm + m, nb);
-    float *keep = Mx.on ? Mx.lu + (((size_t)m * Cl.n_tasks + task) * Mx.n_lu) * 32 + lane : nullptr;
+    const int4 *stream = reinterpret_cast<const int4 *>(Cl.full) + 2 * (size_t)Cl.full_ptr[cls * kCluWarps + warp];
+    const int n_pairs = Cl.full_ptr[cls * kCluWarps + warp + 1] - Cl.full_ptr[cls * kCluWarps + warp];
     const int n_da = P.n_diff + P.n_alg;
     double *yx = W.yx + (size_t)m * 3 * n_da + ws;
-    const int *p3 = Cl.pos3 + cls * 3;
-    double X0[3], X1[3], X2[3];
+    const int *pc = Cl.perm_col + cls * 32, *p3 = Cl.pos3 + cls * 3;
+    double X0[3], X1[3], X2[3];   // warp 1
     if (mode == 1) {
         // MX_FP32: the factors are kept in FP32, so the factorisation and
-        // the three solves run in FP32 too.  The slots are converted in place:
-        // float slot s lies in the first half of double slot s / 2, which was
-        // read before (each slot is read into registers before the warp
-        // writes over it).
+        // the three solves run in FP32 too.  The slots are converted in
+        // place, eight a warp at a time: float slot s lies in the first half
+        // of double slot s / 2, which an earlier round or this one has read
         float *fv = reinterpret_cast<float *>(vals);
-        for (int s = 0; s < nslot; s++) {
-            const float x = (float)vals[s * 32 + lane];
-            __syncwarp();
-            fv[s * 32 + lane] = x;
-            __syncwarp();
+        const int nslot = rb + 3 * Wn;
+        for (int s0 = 0; s0 < nslot; s0 += 8 * kCluWarps) {
+            float x[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const int s = s0 + u * kCluWarps + warp;
+                x[u] = s < nslot ? (float)vals[s * 32 + lane] : 0.0f;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const int s = s0 + u * kCluWarps + warp;
+                if (s < nslot) fv[s * 32 + lane] = x[u];
+            }
+            __syncthreads();
         }
-        float *F0 = fv + (size_t)rb * 32, *F1 = F0 + (size_t)Wn * 32, *F2 = F1 + (size_t)Wn * 32;
-        clu_program<float>(fv, F0, F1, F2, ops, qm, q1, lane);
-        for (int s = 0; s < rb; s++) keep[s * 32] = fv[s * 32 + lane];
+        run_stages<float>(stream, n_pairs, fv, fv, lane);
+        __syncthreads();
+        float *keep = Mx.lu + (((size_t)m * Cl.n_tasks + task) * Mx.n_lu) * 32 + lane;
+        for (int s = warp; s < rb; s += kCluWarps) keep[(size_t)s * 32] = fv[s * 32 + lane];
         if (!act) return;
-        for (int j = 0; j < Wn; j++) {
+        const float *F0 = fv + (size_t)rb * 32, *F1 = F0 + (size_t)Wn * 32, *F2 = F1 + (size_t)Wn * 32;
+        for (int j = warp; j < Wn; j += kCluWarps) {
             const int st = pc[j];
             yx[st] = (double)F2[j * 32 + lane];
             yx[n_da + st] = (double)F0[j * 32 + lane];
             yx[2 * n_da + st] = (double)F1[j * 32 + lane];
         }
+        if (warp != 1) return;
 #pragma unroll
         for (int t = 0; t < 3; t++) {
             X0[t] = (double)F2[p3[t] * 32 + lane];
@@ -273,18 +374,20 @@ __global__ void __launch_bounds__(32) cluster_kernel(DevProblem P, DevWork W, De
         }
     } else {
         // factorisation and solves in FP64
-        clu_program<double>(vals, R0, R1, R2, ops, qm, q1, lane);
+        run_stages<double>(stream, n_pairs, vals, vals, lane);
+        __syncthreads();
         if (Cl.save_lu) {
             double *sv = Cl.save_lu + (((size_t)m * Cl.n_tasks + task) * Cl.n_save) * 32 + lane;
-            for (int s = 0; s < rb; s++) sv[s * 32] = vals[s * 32 + lane];
+            for (int s = warp; s < rb; s += kCluWarps) sv[(size_t)s * 32] = vals[s * 32 + lane];
         }
         if (!act) return;
-        for (int j = 0; j < Wn; j++) {
+        for (int j = warp; j < Wn; j += kCluWarps) {
             const int st = pc[j];
             yx[st] = R2[j * 32 + lane];
             yx[n_da + st] = R0[j * 32 + lane];
             yx[2 * n_da + st] = R1[j * 32 + lane];
         }
+        if (warp != 1) return;
 #pragma unroll
         for (int t = 0; t < 3; t++) {
             X0[t] = R2[p3[t] * 32 + lane];
@@ -311,116 +414,90 @@ __global__ void __launch_bounds__(32) cluster_kernel(DevProblem P, DevWork W, De
     }
 }
 
-// Sink of a residual-only evaluation: Jacobian entries are dropped (the
-// compiler removes their arithmetic), residuals go to their positions in the
-// staged residual column.
+// Residual-only evaluations: Jacobian entries are dropped (the compiler
+// removes their arithmetic); the backward-Euler residual goes to its
+// position in the solve's column (FP32), its norm to nb, and to f if set.
+template <bool ON>
 struct KeepSink {
-    double *v;
+    float *v;              // null: no column
     const short *slot_of;
+    const double *z, *zold;
+    double *f;
     int ws, lane, base;
+    unsigned diff;
+    double dt;
+    unsigned long long *nb;
     __device__ __forceinline__ void put(int, int, double) {}
+    __device__ __forceinline__ void putc(int, int, double) {}
     __device__ __forceinline__ void putv(int, int, double) {}
     __device__ __forceinline__ void putf(int r, double x) {
-        v[((int)slot_of[(r - ws) * 32 + 31] - base) * 32 + lane] = x;
+        const int lr = r - ws;
+        double y = ON ? x : 0.0;
+        if (diff >> lr & 1) y = z[r] - zold[r] - dt * y;
+        if (v) v[((int)__ldg(slot_of + lr * 32 + 31) - base) * 32 + lane] = (float)y;
+        if (f) f[r] = y;
+        const unsigned long long t = norm_bits(y);
+        *nb = t > *nb ? t : *nb;
     }
 };
 
 // MX_KEEP scenarios of the mixed solver: the FP64 residual and its solve
-// with the kept FP32 LU, nothing else.  Only the residual column is staged in
-// shared memory (W values per lane instead of the whole program's slots), the
-// LU values are read straight from the kept copy, and the op list is the
-// solve part of the program alone, so many more warps fit on an SM.  The
-// solve runs in FP32, like the kept LU it applies: FP64 arithmetic and
-// FP32<->FP64 conversions are scarce on this GPU, and the correction of an
-// iteration on kept factors is inexact at the FP32 level anyway (the residual
-// that drives it stays FP64).
-__global__ void __launch_bounds__(32, 16) cluster_keep_kernel(DevProblem P, DevWork W, DevClu Cl, DevMixed Mx,
-                                                             int want_f) {
-    extern __shared__ double R2[];   // [max_w][32] FP64 residual by pivot position, then [max_w][32] FP32
-    float *Rf = reinterpret_cast<float *>(R2 + (size_t)Cl.max_w * 32);
-    const int task = blockIdx.x, m = blockIdx.y, lane = threadIdx.x;
+// with the kept FP32 LU, nothing else: the kept LU values are copied to
+// shared memory while the devices are evaluated, and the staged solve of one
+// column follows.  The solve runs in FP32, like the kept LU it applies: FP64
+// arithmetic and FP32<->FP64 conversions are scarce on this GPU, and the
+// correction of an iteration on kept factors is inexact at the FP32 level
+// anyway (the residual that drives it stays FP64).
+__global__ void __launch_bounds__(kCluThreads, 6) cluster_keep_kernel(DevProblem P, DevWork W, DevClu Cl,
+                                                                      DevMixed Mx) {
+    extern __shared__ __align__(16) double vals[];   // kept LU [rhs_base][32] FP32, then the column [W][32] FP32
+    __shared__ unsigned long long s_nb[kCluWarps];
+    const int task = blockIdx.x, m = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (!W.active[m] || Mx.refac[m] != MX_KEEP) return;
     const int cls = Cl.task_class[task];
     const int cnt = Cl.task_count[task];
     const bool act = lane < cnt;
-    const int c = act ? Cl.order[Cl.task_first[task] + lane] : Cl.order[Cl.task_first[task]];
+    const int c = Cl.order[Cl.task_first[task] + (act ? lane : 0)];
     const int ws = P.cl_w_start[c], Wn = P.cl_w_size[c];
     const int rb = Cl.rhs_base[cls], base = rb + 2 * Wn;
-    for (int j = 0; j < Wn; j++) R2[j * 32 + lane] = 0.0;
-    const double *z = W.z + (size_t)m * P.n_sys;
-    const double *zold = W.zold + (size_t)m * P.n_sys;
-    double Cc[6] = {0, 0, 0, 0, 0, 0}, Ic[2] = {0, 0};
-    if (act) {
-        KeepSink sink{R2, Cl.slot_of + (size_t)cls * 1024, ws, lane, base};
-        LoadK lk{Mx.kc + (((size_t)m * Cl.n_tasks + task) * kConstSlots) * 32 + lane, 32};
-        eval_cluster(P, c, z, W.u0 + (size_t)m * P.n_ctrl, W.p + (size_t)m * P.n_par, sink, Cc, Ic, lk,
-                     !P.exc_off || !P.exc_off[(size_t)m * P.n_cl + c]);
+    float *lu = reinterpret_cast<float *>(vals), *Rf = lu + (size_t)rb * 32;
+    {
+        const float *kl = Mx.lu + (((size_t)m * Cl.n_tasks + task) * Mx.n_lu) * 32;
+        for (int e = tid; e < rb * 8; e += kCluThreads) cp_async16(lu + 4 * e, kl + 4 * e);
     }
     const double dt = *W.dt;
-    const CluOp *ops = Cl.ops;
-    const int q0 = Cl.prog_ptr[cls], qm = Cl.prog_mid[cls], qs = Cl.prog_sol[cls], q1 = Cl.prog_ptr[cls + 1];
-    // backward-Euler rows, eight ops and their state loads in flight
-    for (int q = q0; q < qm; q += 8) {
-        CluOp o[8];
-        double zn[8], zo[8];
-#pragma unroll
-        for (int u = 0; u < 8; u++) o[u] = ops[min(q + u, qm - 1)];
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const bool ld = act && q + u < qm && o[u].code == OP_BEF;
-            zn[u] = ld ? z[ws + o[u].a] : 0.0;
-            zo[u] = ld ? zold[ws + o[u].a] : 0.0;
-        }
-#pragma unroll
-        for (int u = 0; u < 8; u++)
-            if (q + u < qm && o[u].code == OP_BEF) {
-                double *vd = R2 + (o[u].d - base) * 32 + lane;
-                *vd = act ? zn[u] - zo[u] - dt * *vd : 0.0;
-            }
-    }
+    double Cc[6], Ic[2] = {0, 0};
     unsigned long long nb = 0ull;
-    for (int j = 0; j < Wn; j++) {
-        const unsigned long long t = norm_bits(R2[j * 32 + lane]);
-        nb = t > nb ? t : nb;
+    if (act) {
+        const double *z = W.z + (size_t)m * P.n_sys, *zold = W.zold + (size_t)m * P.n_sys;
+        const short *so = Cl.slot_of + (size_t)cls * 1024;
+        const unsigned diff = Cl.diff_mask[cls];
+        KeepSink<true> on{Rf, so, z, zold, nullptr, ws, lane, base, diff, dt, &nb};
+        KeepSink<false> off{Rf, so, z, zold, nullptr, ws, lane, base, diff, dt, &nb};
+        const LoadK lk{Cl.kc + (((size_t)m * Cl.n_tasks + task) * kConstSlots) * 32 + lane, 32};
+        eval_share(P, c, warp, z, W.u0 + (size_t)m * P.n_ctrl, W.p + (size_t)m * P.n_par, on, off, Cc, Ic, lk,
+                   exciter_on(P, m, c));
+    } else {
+        for (int j = warp; j < Wn; j += kCluWarps) Rf[j * 32 + lane] = 0.0f;
     }
-    if (!act) nb = 0ull;
-    if (want_f && act) {
-        for (int q = q0; q < qm; q++)
-            if (ops[q].code == OP_BEF || ops[q].code == OP_ROW)
-                W.f[(size_t)m * P.n_sys + ws + ops[q].a] = R2[(ops[q].d - base) * 32 + lane];
-    }
+    nb = warp_max(nb);
+    if (lane == 0) s_nb[warp] = nb;
+    cp_async_wait();
+    __syncthreads();
+    if (tid == 0) {
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        const unsigned long long o = __shfl_xor_sync(FULL_MASK, nb, off);
-        nb = o > nb ? o : nb;
+        for (int w = 1; w < kCluWarps; w++) nb = s_nb[w] > nb ? s_nb[w] : nb;
+        atomicMax(W.norm + m, nb);
     }
-    if (lane == 0) atomicMax(W.norm + m, nb);
-    for (int j = 0; j < Wn; j++) Rf[j * 32 + lane] = (float)R2[j * 32 + lane];
-    // the solves (OP_FMS3 / OP_MUL3 on the residual column), eight ops and
-    // their LU values loaded ahead of the arithmetic
-    const float *kl = Mx.lu + (((size_t)m * Cl.n_tasks + task) * Mx.n_lu) * 32 + lane;
-    constexpr int kAhead = 8;
-    for (int q = qs; q < q1; q += kAhead) {
-        CluOp o[kAhead];
-        float l[kAhead];
-#pragma unroll
-        for (int u = 0; u < kAhead; u++) {
-            o[u] = ops[min(q + u, q1 - 1)];
-            l[u] = kl[o[u].a * 32];
-        }
-#pragma unroll
-        for (int u = 0; u < kAhead; u++) {
-            if (q + u >= q1) break;
-            if (o[u].code == OP_FMS3) Rf[o[u].d * 32 + lane] = fmaf(-l[u], Rf[o[u].b * 32 + lane], Rf[o[u].d * 32 + lane]);
-            else Rf[o[u].d * 32 + lane] *= l[u];
-        }
-    }
+    run_stages<float>(reinterpret_cast<const int4 *>(Cl.sol) + 2 * (size_t)Cl.sol_ptr[cls * kCluWarps + warp],
+                      Cl.sol_ptr[cls * kCluWarps + warp + 1] - Cl.sol_ptr[cls * kCluWarps + warp], Rf, lu, lane);
+    __syncthreads();
     if (!act) return;
     const int n_da = P.n_diff + P.n_alg;
     double *yx = W.yx + (size_t)m * 3 * n_da + ws;
-    const int *pc = Cl.perm_col + cls * 32;
-    const int *p3 = Cl.pos3 + cls * 3;
-    for (int j = 0; j < Wn; j++) yx[pc[j]] = (double)Rf[j * 32 + lane];
+    const int *pc = Cl.perm_col + cls * 32, *p3 = Cl.pos3 + cls * 3;
+    for (int j = warp; j < Wn; j += kCluWarps) yx[pc[j]] = (double)Rf[j * 32 + lane];
+    if (warp != 1) return;
     const float Y0 = Rf[p3[0] * 32 + lane], Y1 = Rf[p3[1] * 32 + lane], Y2 = Rf[p3[2] * 32 + lane];
     const float *cc = Mx.cc + ((size_t)m * P.n_cl + c) * 6;
     double *o = W.clout + ((size_t)m * P.n_cl + c) * 8;
@@ -430,15 +507,50 @@ __global__ void __launch_bounds__(32, 16) cluster_keep_kernel(DevProblem P, DevW
     o[7] = Ic[1];
 }
 
-int launch_cluster(const DevProblem &P, const DevWork &W, const DevClu &C, const DevMixed &Mx, int want_f,
-                   cudaStream_t st) {
+// Parity probes: the residual rows of the clusters (W.f), their norm and the
+// injections, nothing else (no parameter constants or images needed).
+__global__ void __launch_bounds__(kCluThreads) cluster_residual_kernel(DevProblem P, DevWork W, DevClu Cl) {
+    const int task = blockIdx.x, m = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (!W.active[m]) return;
+    const bool act = lane < Cl.task_count[task];
+    unsigned long long nb = 0ull;
+    if (act) {
+        const int cls = Cl.task_class[task], c = Cl.order[Cl.task_first[task] + lane];
+        const double *z = W.z + (size_t)m * P.n_sys, *zold = W.zold + (size_t)m * P.n_sys;
+        double *f = W.f + (size_t)m * P.n_sys;
+        double Cc[6], Ic[2];
+        KeepSink<true> on{nullptr, nullptr, z, zold, f, P.cl_w_start[c], lane, 0, Cl.diff_mask[cls], *W.dt, &nb};
+        KeepSink<false> off{nullptr, nullptr, z, zold, f, P.cl_w_start[c], lane, 0, Cl.diff_mask[cls], *W.dt, &nb};
+        eval_share(P, c, warp, z, W.u0 + (size_t)m * P.n_ctrl, W.p + (size_t)m * P.n_par, on, off, Cc, Ic, ComputeK(),
+                   exciter_on(P, m, c));
+        if (warp == 1) {
+            double *o = W.clout + ((size_t)m * P.n_cl + c) * 8;
+            for (int t = 0; t < 6; t++) o[t] = 0.0;
+            o[6] = Ic[0];
+            o[7] = Ic[1];
+        }
+    }
+    nb = warp_max(nb);
+    if (lane == 0) atomicMax(W.norm + m, nb);
+}
+
+int launch_cluster(const DevProblem &P, const DevWork &W, const DevClu &C, const DevMixed &Mx, cudaStream_t st) {
     if (C.n_tasks == 0) return 0;
     dim3 grid(C.n_tasks, P.M);
-    cluster_kernel<<<grid, 32, (size_t)C.max_slots * 32 * sizeof(double), st>>>(P, W, C, Mx, want_f);
+    cluster_kernel<<<grid, kCluThreads, (size_t)C.max_slots * 32 * sizeof(double), st>>>(P, W, C, Mx);
     if (!Mx.on) return 1;
-    cluster_keep_kernel<<<grid, 32, (size_t)C.max_w * 32 * (sizeof(double) + sizeof(float)), st>>>(P, W, C, Mx,
-                                                                                                  want_f);
+    cluster_keep_kernel<<<grid, kCluThreads, (size_t)(C.max_rb + C.max_w) * 32 * sizeof(float), st>>>(P, W, C, Mx);
     return 2;
+}
+
+void launch_cluster_residual(const DevProblem &P, const DevWork &W, const DevClu &C, cudaStream_t st) {
+    if (C.n_tasks > 0) cluster_residual_kernel<<<dim3(C.n_tasks, P.M), kCluThreads, 0, st>>>(P, W, C);
+}
+
+void launch_cluster_image(const DevProblem &P, const DevWork &W, const DevClu &C, double dt, cudaStream_t st) {
+    if (C.n_tasks > 0)
+        cluster_image_kernel<<<dim3(C.n_tasks, P.M), 32, (size_t)C.max_rb * 32 * sizeof(double), st>>>(
+            P, W, C, dt, dt == 0.0 ? 1 : 0);
 }
 
 // Parameter products of every ZIP load per scenario for network_kernel:
@@ -462,14 +574,12 @@ void launch_zip_const(const DevProblem &P, const DevWork &W, double *out, cudaSt
     if (n > 0) zip_const_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(P, W, out);
 }
 
-void launch_cluster_const(const DevProblem &P, const DevWork &W, const DevClu &C, const DevMixed &Mx,
-                          cudaStream_t st) {
-    if (C.n_tasks == 0) return;
-    cluster_const_kernel<<<dim3(C.n_tasks, P.M), 32, 0, st>>>(P, W, C, Mx);
-}
-
 int cluster_smem_optin(int bytes) {
-    if (cudaFuncSetAttribute(cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) {
+    if (cudaFuncSetAttribute(cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess ||
+        cudaFuncSetAttribute(cluster_image_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) !=
+            cudaSuccess ||
+        cudaFuncSetAttribute(cluster_keep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) !=
+            cudaSuccess) {
         cudaGetLastError();
         return -1;
     }
