@@ -55,7 +55,8 @@ struct ND {
     int next_id = 1;
     static constexpr int LEAF = 48;
 
-    explicit ND(const Graph &g) : G(g), set_id(g.n, 0), lev(g.n, -1), pos_in(g.n, -1) {}
+    explicit ND(const Graph &g)
+        : G(g), set_id(g.n, 0), lev(g.n, -1), pos_in(g.n, -1), part(g.n, 0), stamp(g.n, 0) {}
 
     // BFS inside the set `sid` from r; fills lev for visited nodes and
     // returns the visited nodes in BFS order.
@@ -78,6 +79,151 @@ struct ND {
     void clear_lev(const std::vector<int> &V) {
         for (int v : V) lev[v] = -1;
     }
+
+    // Splits the connected set V into A, B and a separator S: the smallest
+    // of the breadth-first level sets near the middle, seen from r and from
+    // the far end, each then refined (part: 0 A, 1 B, 2 S).  Against the
+    // median level alone, unrefined, on the 70,000-bus grid: largest front
+    // 132 -> 40 rows, factorisation flops 33.7 -> 19.4 M a scenario, levels
+    // 30 -> 16; FP64 run of 8 scenarios x 18 steps 104 -> 58 ms (its
+    // factorisations 78 -> 36 ms), mixed (36 steps) 70 -> 56 ms; the analysis
+    // itself 0.39 -> 0.6 s.
+    std::vector<signed char> part;
+    void split(const std::vector<int> &V, int r, int sid, std::vector<int> &A, std::vector<int> &B,
+               std::vector<int> &S) {
+        std::vector<int> visit, best;
+        std::vector<signed char> best_part;
+        double best_cost = 1e300;
+        for (int side = 0; side < 2; side++) {
+            clear_lev(V);
+            bfs(r, sid, visit);
+            const int nlev = lev[visit.back()] + 1, n = (int)V.size(), far = visit.back();
+            std::vector<int> cnt(nlev, 0);
+            for (int v : V) cnt[lev[v]]++;
+            // the smallest levels with at least a third of the nodes on
+            // either side, and the median one
+            std::vector<std::pair<int, int>> cand;
+            int acc = 0, median = -1;
+            for (int l = 0; l < nlev; l++) {
+                if (l > 0 && l < nlev - 1 && acc >= n / 3 && n - acc - cnt[l] >= n / 3) cand.push_back({cnt[l], l});
+                acc += cnt[l];
+                if (median < 0 && 2 * acc >= n) median = std::max(0, std::min(l, nlev - 2));
+            }
+            std::sort(cand.begin(), cand.end());
+            if (cand.size() > 3) cand.resize(3);
+            cand.push_back({0, median});
+            for (auto &c : cand) {
+                const int l = c.second;
+                for (int v : V) {
+                    if (lev[v] != l) {
+                        part[v] = lev[v] < l ? 0 : 1;
+                        continue;
+                    }
+                    bool touches = false;
+                    for (int q = G.ptr[v]; q < G.ptr[v + 1] && !touches; q++) {
+                        const int u = G.adj[q];
+                        touches = set_id[u] == sid && lev[u] == l + 1;
+                    }
+                    part[v] = touches ? 2 : 0;
+                }
+                const double cost = refine(V, sid);
+                if (cost < best_cost) {
+                    best_cost = cost;
+                    best_part.resize(V.size());
+                    for (size_t i = 0; i < V.size(); i++) best_part[i] = part[V[i]];
+                }
+            }
+            r = far;
+        }
+        clear_lev(V);
+        for (size_t i = 0; i < V.size(); i++)
+            (best_part[i] == 0 ? A : (best_part[i] == 1 ? B : S)).push_back(V[i]);
+    }
+
+    // Vertex-separator refinement (C. Fiduccia, R. Mattheyses, "A linear-time
+    // heuristic for improving network partitions", DAC 1982, in its form for
+    // vertex separators): a separator node moves to one side and pulls its
+    // neighbours on the other side into the separator; the moves of a pass
+    // are taken back to its best point.  Returns the separator's cost.
+    std::vector<int> stamp;
+    double refine(const std::vector<int> &V, int sid) {
+        const int n = (int)V.size();
+        int w[3] = {0, 0, 0};
+        for (int v : V) w[(int)part[v]]++;
+        const int lo = std::max(1, (int)(0.3 * n));
+        auto cost = [&] {
+            const double bal = std::max(w[0], w[1]) / (double)std::max(1, std::min(w[0], w[1]));
+            return w[2] * (1.0 + 0.1 * std::max(0.0, bal - 1.2)) + (w[0] == 0 || w[1] == 0 ? 1e9 : 0.0);
+        };
+        auto pulls = [&](int v, int to) {
+            int k = 0;
+            for (int q = G.ptr[v]; q < G.ptr[v + 1]; q++) k += set_id[G.adj[q]] == sid && part[G.adj[q]] == 1 - to;
+            return k;
+        };
+        double best = cost();
+        for (int pass = 0; pass < 6; pass++) {
+            using Item = std::pair<int, std::pair<int, int>>;   // gain, node, side
+            std::priority_queue<Item> heap;
+            auto push = [&](int v) {
+                for (int to = 0; to < 2; to++) heap.push({1 - pulls(v, to), {v, to}});
+            };
+            pass_id++;
+            for (int v : V)
+                if (part[v] == 2) push(v);
+            std::vector<std::pair<int, signed char>> undo;
+            size_t keep = 0;
+            const double start = best;
+            int since = 0;
+            while (!heap.empty() && since < 60) {
+                const Item it = heap.top();
+                heap.pop();
+                const int v = it.second.first, to = it.second.second;
+                if (part[v] != 2 || stamp[v] == pass_id) continue;
+                const int k = pulls(v, to);
+                if (1 - k != it.first) {
+                    heap.push({1 - k, {v, to}});
+                    continue;
+                }
+                if (w[1 - to] - k < lo) continue;
+                stamp[v] = pass_id;   // (a node leaves the separator once a pass)
+                undo.push_back({v, 2});
+                part[v] = (signed char)to;
+                w[2]--;
+                w[to]++;
+                for (int q = G.ptr[v]; q < G.ptr[v + 1]; q++) {
+                    const int u = G.adj[q];
+                    if (set_id[u] != sid || part[u] != 1 - to) continue;
+                    undo.push_back({u, (signed char)(1 - to)});
+                    part[u] = 2;
+                    w[1 - to]--;
+                    w[2]++;
+                    push(u);
+                }
+                // separator nodes beside v gained or lost a neighbour
+                for (int q = G.ptr[v]; q < G.ptr[v + 1]; q++) {
+                    const int u = G.adj[q];
+                    if (set_id[u] == sid && part[u] == 2 && stamp[u] != pass_id) push(u);
+                }
+                const double c = cost();
+                since++;
+                if (c < best) {
+                    best = c;
+                    keep = undo.size();
+                    since = 0;
+                }
+            }
+            while (undo.size() > keep) {
+                const auto u = undo.back();
+                undo.pop_back();
+                w[(int)part[u.first]]--;
+                part[u.first] = u.second;
+                w[(int)u.second]++;
+            }
+            if (best >= start) break;
+        }
+        return best;
+    }
+    int pass_id = 0;
 
     void run(std::vector<int> V, int sid) {
         if ((int)V.size() <= LEAF) {
@@ -122,31 +268,8 @@ struct ND {
             }
             r = best;
         }
-        clear_lev(V);
-        bfs(r, sid, visit);
-        int nlev = lev[visit.back()] + 1;
-        std::vector<int> cnt(nlev + 1, 0);
-        for (int v : V) cnt[lev[v]]++;
-        int half = (int)V.size() / 2, acc = 0, l = 0;
-        for (l = 0; l < nlev; l++) {
-            acc += cnt[l];
-            if (acc >= half) break;
-        }
-        if (l >= nlev - 1) l = std::max(0, nlev - 2);
         std::vector<int> A, B, S;
-        for (int v : V) {
-            if (lev[v] < l) A.push_back(v);
-            else if (lev[v] > l) B.push_back(v);
-            else {
-                bool touches = false;
-                for (int q = G.ptr[v]; q < G.ptr[v + 1] && !touches; q++) {
-                    int u = G.adj[q];
-                    touches = set_id[u] == sid && lev[u] == l + 1;
-                }
-                (touches ? S : A).push_back(v);
-            }
-        }
-        clear_lev(V);
+        split(V, r, sid, A, B, S);
         if (A.empty() || B.empty()) {
             // no useful split: order the whole set by minimum degree on its
             // own adjacency (ties in BFS order)
@@ -229,47 +352,91 @@ void analyse(int n, const std::vector<int> &rowptr, const std::vector<int> &coli
     for (int a : nd.order)
         for (int i : members[a]) S.perm.push_back(i);
     if ((int)S.perm.size() != n) throw std::runtime_error("unknowns without a node");
-    S.iperm.assign(n, 0);
-    for (int k = 0; k < n; k++) S.iperm[S.perm[k]] = k;
-    // ---- permuted symmetric pattern: lower part per column ----
-    std::vector<std::vector<int>> low(n), upp(n);
-    for (int i = 0; i < n; i++)
-        for (int q = rowptr[i]; q < rowptr[i + 1]; q++) {
-            int a = S.iperm[i], b = S.iperm[colidx[q]];
-            if (a == b) continue;
-            int lo = std::min(a, b), hi = std::max(a, b);
-            low[lo].push_back(hi);
-            upp[hi].push_back(lo);
-        }
-    for (int j = 0; j < n; j++) {
-        std::sort(low[j].begin(), low[j].end());
-        low[j].erase(std::unique(low[j].begin(), low[j].end()), low[j].end());
-        std::sort(upp[j].begin(), upp[j].end());
-        upp[j].erase(std::unique(upp[j].begin(), upp[j].end()), upp[j].end());
-    }
-    // ---- elimination tree (Liu, path compression) ----
-    std::vector<int> par(n, -1), anc(n, -1);
-    for (int j = 0; j < n; j++)
-        for (int i : upp[j]) {
-            int r = i;
-            while (anc[r] != -1 && anc[r] != j) {
-                int nx = anc[r];
-                anc[r] = j;
-                r = nx;
+    // ---- elimination tree of the dissection's order, then of its postorder
+    // with the column structures ----
+    std::vector<int> par, nchild;
+    std::vector<std::vector<int>> cs;
+    for (int round = 0; round < 2; round++) {
+        S.iperm.assign(n, 0);
+        for (int k = 0; k < n; k++) S.iperm[S.perm[k]] = k;
+        // lower part per column (sorted), and by row for the tree
+        std::vector<int> up_ptr(n + 1, 0);
+        for (int i = 0; i < n; i++)
+            for (int q = rowptr[i]; q < rowptr[i + 1]; q++) {
+                const int a = S.iperm[i], b = S.iperm[colidx[q]];
+                if (a != b) up_ptr[std::max(a, b) + 1]++;
             }
-            if (anc[r] == -1) { anc[r] = j; par[r] = j; }
+        for (int j = 0; j < n; j++) up_ptr[j + 1] += up_ptr[j];
+        std::vector<int> upp(up_ptr[n]), at(up_ptr.begin(), up_ptr.end() - 1);
+        for (int i = 0; i < n; i++)
+            for (int q = rowptr[i]; q < rowptr[i + 1]; q++) {
+                const int a = S.iperm[i], b = S.iperm[colidx[q]];
+                if (a != b) upp[at[std::max(a, b)]++] = std::min(a, b);
+            }
+        // elimination tree (Liu, path compression)
+        par.assign(n, -1);
+        std::vector<int> anc(n, -1);
+        for (int j = 0; j < n; j++)
+            for (int q = up_ptr[j]; q < up_ptr[j + 1]; q++) {
+                int r = upp[q];
+                while (anc[r] != -1 && anc[r] != j) {
+                    int nx = anc[r];
+                    anc[r] = j;
+                    r = nx;
+                }
+                if (anc[r] == -1) { anc[r] = j; par[r] = j; }
+            }
+        nchild.assign(n, 0);
+        std::vector<std::vector<int>> kids(n);
+        for (int j = 0; j < n; j++)
+            if (par[j] >= 0) {
+                nchild[par[j]]++;
+                kids[par[j]].push_back(j);
+            }
+        if (round == 1) {
+            // column structures: the rows below a column's diagonal and
+            // those its children pass on (the rows come in increasing order)
+            cs.assign(n, {});
+            for (int i = 0; i < n; i++)
+                for (int q = up_ptr[i]; q < up_ptr[i + 1]; q++)
+                    if (cs[upp[q]].empty() || cs[upp[q]].back() != i) cs[upp[q]].push_back(i);
+            for (int j = 0; j < n; j++)
+                for (int c : kids[j]) merge_into(cs[j], cs[c], j);
+            break;
         }
-    // ---- column structures ----
-    std::vector<int> nchild(n, 0);
-    for (int j = 0; j < n; j++)
-        if (par[j] >= 0) nchild[par[j]]++;
-    std::vector<std::vector<int>> cs(n);
-    std::vector<std::vector<int>> kids(n);
-    for (int j = 0; j < n; j++)
-        if (par[j] >= 0) kids[par[j]].push_back(j);
-    for (int j = 0; j < n; j++) {
-        cs[j] = low[j];
-        for (int c : kids[j]) merge_into(cs[j], cs[c], j);
+        // postorder, each column's child with the tallest subtree last: the
+        // supernode that a merge can join to its parent's columns (they
+        // must follow it directly) is then the one on the longest path.
+        // (The unknowns of a node stay adjacent: each has the one before it
+        // as its only child, since whatever reaches a node reaches its
+        // first unknown.)
+        std::vector<int> height(n, 0), post;
+        for (int j = 0; j < n; j++)
+            if (par[j] >= 0) height[par[j]] = std::max(height[par[j]], height[j] + 1);
+        post.reserve(n);
+        std::vector<std::pair<int, size_t>> walk;
+        for (int j = 0; j < n; j++) {
+            std::stable_sort(kids[j].begin(), kids[j].end(), [&](int a, int b) {
+                return height[a] < height[b];
+            });
+        }
+        for (int root = 0; root < n; root++) {
+            if (par[root] >= 0) continue;
+            walk.push_back({root, 0});
+            while (!walk.empty()) {
+                auto &w = walk.back();
+                if (w.second < kids[w.first].size()) {
+                    const int c = kids[w.first][w.second++];
+                    walk.push_back({c, 0});
+                } else {
+                    post.push_back(w.first);
+                    walk.pop_back();
+                }
+            }
+        }
+        std::vector<int> perm(n);
+        for (int k = 0; k < n; k++) perm[k] = S.perm[post[k]];
+        S.perm.swap(perm);
     }
     // ---- fundamental supernodes ----
     std::vector<int> fstart;
@@ -279,15 +446,22 @@ void analyse(int n, const std::vector<int> &rowptr, const std::vector<int> &coli
     }
     int nf = (int)fstart.size();
     fstart.push_back(n);
-    // ---- amalgamation: merge a supernode into its parent when the
-    // parent's columns follow it directly and the merge adds at most
-    // `relax_zeros` explicit zeros (0 = only exact nesting) ----
+    // ---- amalgamation: merge a supernode into its parent when the parent's
+    // columns follow it directly and the merge adds no explicit zero, or when
+    // the merged supernode has at most 24 columns and less than a fifth of
+    // its entries are zeros.  Every level costs the factorisation and the
+    // solves a hand-off (3 to 10 us), every zero FP64 work: this rule against
+    // at most two zeros a column (widths to 48), and against a share of 0.35
+    // (widths to 12) or 0.2 (to 32), FP64 runs: 70,000 buses x 8 (18 steps)
+    // 58.0, 59.1, 59.6 ms, 9,001 x 3 29.2, 28.0, 30.7, 39 x 64 53.0, 61, 54.6
+    // ----
     {
         std::vector<int> fsup_of(n);
         for (int f = 0; f < nf; f++)
             for (int j = fstart[f]; j < fstart[f + 1]; j++) fsup_of[j] = f;
         std::vector<int> st(fstart.begin(), fstart.end() - 1), ncol(nf), fpar(nf, -1);
         std::vector<char> gone(nf, 0);
+        std::vector<int64_t> zeros(nf, 0);   // explicit zeros of the merged supernode, one triangle
         for (int f = 0; f < nf; f++) {
             ncol[f] = fstart[f + 1] - fstart[f];
             int last = fstart[f + 1] - 1;
@@ -300,8 +474,13 @@ void analyse(int n, const std::vector<int> &rowptr, const std::vector<int> &coli
             int64_t rp = (int64_t)cs[fstart[p + 1] - 1].size();
             int64_t extra = (int64_t)ncol[f] * (ncol[p] + rp - rs);
             int64_t width = ncol[f] + ncol[p];
-            bool ok = extra == 0 || (width <= 48 && extra <= width * 2);
-            if (!ok) continue;
+            zeros[p] += zeros[f] + extra;
+            const double share = (double)zeros[p] / (double)(width * (width + 2 * rp));
+            const bool ok = extra == 0 || (width <= 24 && share < 0.2);
+            if (!ok) {
+                zeros[p] -= zeros[f] + extra;
+                continue;
+            }
             st[p] = st[f];
             ncol[p] += ncol[f];
             gone[f] = 1;

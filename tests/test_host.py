@@ -101,6 +101,29 @@ def test_reduced_factorisation_matches_scipy(lib, name):
     assert np.max(np.abs(x - xr)) <= 1e-12 * np.max(np.abs(xr))
 
 
+@pytest.mark.parametrize("n_bus,n_gen", [(49, 8), (97, 12), (301, 40), (1999, 150), (5001, 900)])
+def test_reduced_factorisation_on_other_grids(lib, n_bus, n_gen):
+    """The same on planar grids around and above the dissection's leaf size:
+    the analysis keeps every unknown, its tree is valid (relative maps found,
+    factors against scipy's), and the separators stay small."""
+    w = synthetic._planar("planar", 11, n_bus, n_gen, 0.55, 1, 1.0, "random")
+    PA = LY.ProblemArrays(w.ps)
+    P = PA.as_ctypes()
+    rng = np.random.default_rng(n_bus)
+    S = _reduced_S(w.ps, rng)
+    rhs = rng.normal(size=S.shape[0])
+    x = np.zeros_like(rhs)
+    out = np.zeros(12)
+    rp, ci, sv = S.indptr.astype(np.int32), S.indices.astype(np.int32), S.data.astype(np.float64)
+    lib.gp_reduced_selftest.argtypes = [C.c_void_p] * 7
+    assert lib.gp_reduced_selftest(C.addressof(P), rp.ctypes.data, ci.ctypes.data, sv.ctypes.data,
+                                   rhs.ctypes.data, x.ctypes.data, out.ctypes.data) == 0, lib_error(lib)
+    assert out[0] == 0.0 and out[1] == 0 and out[4] <= 1e-13 and out[8] <= 1e-10 and out[11] == 0.0
+    assert out[9] <= 64
+    xr = spla.spsolve(S.tocsc(), rhs)
+    assert np.max(np.abs(x - xr)) <= 1e-12 * np.max(np.abs(xr))
+
+
 def test_reduced_factorisation_with_static_generators(lib, golden_cases, orc):
     """IEEE 9-bus with the slack machine (bus 1) and one PV machine (bus 2)
     left without a dynamic model: StaticGenerator stand-ins add algebraic
