@@ -1082,14 +1082,10 @@ void host_block_solve(const gp::Symbolic &S, const HostBlk &B, const std::vector
     }
 }
 
-// Task order of the dataflow kernels: supernodes whose whole subtree has
-// fronts of at most dag_small_front() rows first (by level), then the rest
-// (by level).  Both parts list children before parents.
 // The dataflow schedule (host side): the topological order of the
-// factorisation tasks (the tiny region, subtrees whose fronts have at most
-// dag_tiny_front() rows, by level; the rest of the small region, at most
-// dag_small_front() rows; then the rest by level) and the split of the
-// tail's large FP64 fronts into parts.
+// factorisation tasks (by region: subtrees whose fronts have at most
+// dag_tiny_front() and 32 rows, and the rest; by level within a region)
+// and the split of the tail's large FP64 fronts into parts.
 struct DagPlan {
     std::vector<int> order, rank, submax;
     int n_tiny = 0, n_small = 0, max_big = 0, max_big_whole = 0;
@@ -1111,10 +1107,13 @@ void make_dag_plan(const gp::Symbolic &sym, DagPlan &dp) {
             for (int c = sym.child_ptr[s]; c < sym.child_ptr[s + 1]; c++) mx = std::max(mx, dp.submax[sym.children[c]]);
             dp.submax[s] = mx;
         }
-    const int lim = gp::dag_small_front(), tiny = gp::dag_tiny_front();
+    const int tiny = gp::dag_tiny_front();
     dp.order.clear();
     dp.rank.assign(ns, 0);
-    auto region = [&](int s) { return dp.submax[s] <= tiny ? 0 : (dp.submax[s] <= lim ? 1 : 2); };
+    auto region = [&](int s) {
+        const int m = dp.submax[s];
+        return m <= tiny ? 0 : (m <= 32 ? 1 : 2);
+    };
     for (int pass = 0; pass < 3; pass++)
         for (int l = 0; l < sym.nlevels; l++)
             for (int q = sym.level_ptr[l]; q < sym.level_ptr[l + 1]; q++) {
@@ -1163,12 +1162,11 @@ void build_dag(gp_layout *L, const gp::Symbolic &sym) {
     DagPlan dp;
     make_dag_plan(sym, dp);
     const std::vector<int> &order = dp.order, &rank = dp.rank, &submax = dp.submax;
-    const int lim = gp::dag_small_front();
-    const int n_small = dp.n_small;
+    const int lim = gp::dag_tiny_front();
     gp::DevDag &D = L->D;
     D.nsup = ns;
-    D.n_small = n_small;
     D.n_tiny = dp.n_tiny;
+    D.n_small = dp.n_small;
     D.max_front = sym.max_front;
     D.order = A.upload(order);
     D.rank = A.upload(rank);
@@ -1177,7 +1175,7 @@ void build_dag(gp_layout *L, const gp::Symbolic &sym) {
         const size_t M = L->M;
         D.tail0 = dp.tail0;
         D.n_tail = ns - dp.tail0;
-        D.big_units = (D.tail0 - n_small) + dp.tail_units.back();
+        D.big_units = (D.tail0 - D.n_small) + dp.tail_units.back();
         D.max_panels = dp.max_panels;
         D.max_split_ns = dp.max_split_ns;
         D.max_part_entries = dp.max_part_entries;
@@ -1482,7 +1480,7 @@ void build_work(gp_layout *L, const double *z0, const double *u0, const double *
         to_device(L, S.ipiv, ident.data(), ident.size() * sizeof(int), "ipiv");
     }
     gp::DevDag &D = L->D;
-    D.ctr = A.alloc<int>(8);
+    D.ctr = A.alloc<int>(16);
     D.epoch = A.alloc<int>(1);
     D.err = A.alloc<int>(1);
     D.fdone = A.alloc<int>(M * D.nsup);
@@ -1492,7 +1490,7 @@ void build_work(gp_layout *L, const double *z0, const double *u0, const double *
     D.xtag = A.alloc<unsigned long long>(M * std::max(1, P.n_red));
     fill(L, D.utag, 0, M * std::max<int64_t>(1, S.uvec_total) * sizeof(unsigned long long));
     fill(L, D.xtag, 0, M * std::max(1, P.n_red) * sizeof(unsigned long long));
-    fill(L, D.ctr, 0, 8 * sizeof(int));
+    fill(L, D.ctr, 0, 16 * sizeof(int));
     fill(L, D.epoch, 0, sizeof(int));
     fill(L, D.err, 0, sizeof(int));
     fill(L, D.fdone, 0, M * D.nsup * sizeof(int));
@@ -1661,10 +1659,7 @@ void mark(gp_layout *L, int i) {
 // own factors), and the update.
 int enqueue_solve(gp_layout *L, int variant, int *nfac_out) {
     const gp::DevDag &D = L->D;
-    // factorisation launches: FP32 the warp and CTA kernels; FP64 also the
-    // tiny region's warp launch
-    const int nfac = (D.n_small > 0) + (D.nsup > D.n_small);
-    const int nfac64 = (D.n_tiny > 0) + (D.n_small > D.n_tiny) + (D.nsup > D.n_small);
+    const int nfac = gp::dag_factor_launches(D, 1), nfac64 = gp::dag_factor_launches(D, 0);
     const gp::DevBlk &B = L->B;
     const int nsolve = (B.nblk + B.n_top) > 0;   // one fused kernel per direction
     int launches = 2, facs = 0;   // dag_begin, update
@@ -1923,10 +1918,9 @@ void wb_prepare(gp_layout *L, double dt) {
     }
     gp::launch_wb_setup(L->P, L->wb_W1, L->wb_W2, L->wb_Hinv, L->st);
     {
-        const gp::DevDag &D = L->D;
-        const int nfac64 = (D.n_tiny > 0) + (D.n_small > D.n_tiny) + (D.nsup > D.n_small);
-        L->launches += 14 + nfac64;
-        L->factor_launches += nfac64;
+        const int nfac = gp::dag_factor_launches(L->D, 0);
+        L->launches += 14 + nfac;
+        L->factor_launches += nfac;
     }
 }
 

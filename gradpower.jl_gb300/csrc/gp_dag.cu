@@ -50,7 +50,6 @@ namespace {
 constexpr unsigned FULL = kFullMask;
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
-constexpr int kSmallFront = 32;
 // FP64 factorisations run the subtrees whose fronts have at most
 // kTinyFront rows first, in a launch of their own with a smaller front
 // buffer: more fronts in flight, where the 32-row buffers hold an SM to 24
@@ -58,6 +57,7 @@ constexpr int kSmallFront = 32;
 // (factor_group_kernel).  FP32 ones keep one launch: their 32-row buffers
 // already allow 48 warps, and the launch boundary would cost the overlap of
 // the two regions (74 -> 81 ms per mixed run).
+constexpr int kSmallFront = 32;
 constexpr int kTinyFront = 20;
 // lanes a tiny front gets in factor_group_kernel (32 / kTinyLanes fronts a
 // warp).  16: two fronts a warp.  8 (four fronts a warp, a quarter fewer
@@ -142,8 +142,15 @@ struct KeyOf<float> {
     using type = unsigned;
 };
 
+__device__ __forceinline__ unsigned key_hi(double v) { return (unsigned)__double2hiint(v) & 0x7fffffffu; }
+__device__ __forceinline__ unsigned key_lo(double v) { return (unsigned)__double2loint(v); }
+__device__ __forceinline__ unsigned key_hi(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+
 // LW < 32: the warp is LW-lane segments, each searching its own front (the
-// whole warp calls it).
+// whole warp calls it).  A whole warp takes the maximum by integer
+// reductions of the key's words (25 cycles each on GB300, a 64-bit shuffle
+// 38); segments by shuffles (reductions over half a warp run one half after
+// the other: factor_group_kernel 403 -> 420 us on 70,000 buses x 8).
 template <class T, int LW = 32>
 __device__ __forceinline__ int warp_pivot(const T *F, int mm, int k, int ns, bool &zero) {
     using K = typename KeyOf<T>::type;
@@ -154,14 +161,30 @@ __device__ __forceinline__ int warp_pivot(const T *F, int mm, int k, int ns, boo
         const K v = (K)mag_key(F[i + k * mm]);
         if (v > bk) { bk = v; bi = i; }
     }
+    if constexpr (LW == 32) {
+        unsigned mh, ml = 0;
+        bool mine;
+        if constexpr (sizeof(T) == 8) {
+            const unsigned hi = (unsigned)((unsigned long long)bk >> 32), lo = (unsigned)bk;
+            mh = __reduce_max_sync(FULL, hi);
+            ml = __reduce_max_sync(FULL, hi == mh ? lo : 0u);
+            mine = hi == mh && lo == ml;
+        } else {
+            mh = __reduce_max_sync(FULL, (unsigned)bk);
+            mine = (unsigned)bk == mh;
+        }
+        zero = (mh | ml) == 0u;
+        return (int)__reduce_min_sync(FULL, mine ? (unsigned)bi : 0xffffffffu);
+    } else {
 #pragma unroll
-    for (int off = LW / 2; off > 0; off >>= 1) {
-        const K ok = __shfl_xor_sync(FULL, bk, off, LW);
-        const int oi = __shfl_xor_sync(FULL, bi, off, LW);
-        if (ok > bk || (ok == bk && oi < bi)) { bk = ok; bi = oi; }
+        for (int off = LW / 2; off > 0; off >>= 1) {
+            const K ok = __shfl_xor_sync(FULL, bk, off, LW);
+            const int oi = __shfl_xor_sync(FULL, bi, off, LW);
+            if (ok > bk || (ok == bk && oi < bi)) { bk = ok; bi = oi; }
+        }
+        zero = bk == 0;
+        return bi;
     }
-    zero = bk == 0;
-    return bi;
 }
 
 // Thread groups that factor one front: a warp, the whole CTA, or a W-lane
@@ -1039,6 +1062,239 @@ __host__ __device__ inline int big_front_bytes(int max_front) {
     return (max_front * (max_front + 1) * (int)sizeof(T) + 15) & ~15;
 }
 
+// ---- middle fronts: registers --------------------------------------------
+// Fronts above the tiny region's, up to 32 rows, four warps a front: the
+// warps take the columns in turn (column warp + 4 c), the lanes the rows,
+// every entry in a register of its thread.  These fronts lie near
+// the root, where few tasks are ready at a time, so the time of one front
+// counts: waiting for the children, the column steps one after the other,
+// and handing on.  A column step has one barrier: the column's owner put it
+// into shared memory before the barrier; then every warp finds the pivot
+// (three integer reductions), while each lane takes the reciprocal of its
+// own row's entry (the FP64 pipe charges a warp instruction the same
+// whatever its active lanes, so this costs one reciprocal), the multipliers,
+// and updates its columns, the next pivot column first, which its owner puts
+// into the other half of the buffer.  The four warps sit on the four
+// sub-partitions, whose FP64 pipes take 64 cycles per instruction each.
+// Rows are not exchanged: a row that was pivot at step k drops out of the
+// updates and is stored as pivot row k.  Every entry receives the operations
+// of the right-looking elimination in factor_front.
+// Measured, one warp a front (factor_small_kernel) -> this: 9,001 buses x 3
+// (261 tasks) 145 -> 81 us, 2,000 x 64 (1,344) 144 -> 108 us.
+constexpr int kMidThreads = 128, kMidWarps = 4;
+// FP64 tasks of the region of 21 to 32 rows above which factor_small_kernel
+// (a warp a front, a quarter of the FP64 instructions for reciprocals and
+// multipliers, 24 fronts a SM) takes it: 70,000 buses x 8 (5,240 tasks) 294
+// us against 395, 2,000 x 64 (1,344) 144 against 108, 9,001 x 3 (261) 145
+// against 81.
+constexpr long long kMidTasks = 3000;
+
+template <class T>
+struct MidShape {
+    static constexpr int rows = 32;
+    static constexpr int cw = (rows + 1 + kMidWarps - 1) / kMidWarps;   // columns a warp holds (with the RHS)
+    static constexpr int front_bytes = (rows * (rows + 1) * (int)sizeof(T) + 15) & ~15;
+    static constexpr int bytes = front_bytes + 2 * rows * (int)sizeof(T);
+};
+
+template <class T, bool RHS, class Wait, class Done>
+__device__ void factor_mid(const DevProblem &P, const DevWork &W, const DevSym &S, T *fronts, T *lfac, T *ufac, int s,
+                           int m, T *F, T *colbuf, Wait wait, Done done) {
+    constexpr int CW = MidShape<T>::cw;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int start = S.sup_start[s];
+    const int ns = S.sup_start[s + 1] - start;
+    const int mm = ns + S.row_ptr[s + 1] - S.row_ptr[s];
+    const int nc = mm + (RHS ? 1 : 0);
+    T *fr = fronts + (size_t)m * S.front_total;
+    double *x = W.xperm + (size_t)m * P.n_red;
+    double *uv = S.uvec + (size_t)m * S.uvec_total;
+    // ---- what needs nothing from the children: the entries of S and the
+    // right-hand side, and where the children's entries come from ----
+    for (int i = tid; i < mm * nc; i += kMidThreads) F[i] = T(0);
+    __syncthreads();
+    for (int e = S.asmc_ptr[s] + tid; e < S.asmc_ptr[s + 1]; e += kMidThreads) F[S.asmc_pos[e]] += (T)S.asmc_val[e];
+    if (RHS)
+        for (int i = tid; i < ns; i += kMidThreads) F[mm * mm + i] = (T)x[start + i];
+    __syncthreads();
+    const double *sv = W.svar + (size_t)m * P.n_var;
+    for (int e = S.asmv_ptr[s] + tid; e < S.asmv_ptr[s + 1]; e += kMidThreads)
+        F[S.asmv_pos[e]] += (T)sv[S.asmv_idx[e]];
+    if (S.asmt_ptr)
+        for (int e = S.asmt_ptr[s] + tid; e < S.asmt_ptr[s + 1]; e += kMidThreads) {
+            const int t = S.asmt_tr[e];
+            if (P.tr_on[t] && t >= P.tr_ptr[m] && t < P.tr_ptr[m + 1]) F[S.asmt_pos[e]] += (T)S.asmt_val[e];
+        }
+    // sources of each entry: where its list starts, its length, the offsets
+    // of the next kSrc of them
+    constexpr int kSrc = 2;
+    int e0[CW], ne[CW], src[CW][kSrc], kmax = 0;
+    const int *pp = S.pa_ptr + S.pa_base[s], *rp = S.pr_ptr + S.pr_base[s];
+    auto is_rhs = [&](int c) { return RHS && warp + kMidWarps * c == mm; };
+#pragma unroll
+    for (int c = 0; c < CW; c++) {
+        const int j = warp + kMidWarps * c;
+        e0[c] = ne[c] = 0;
+        if (lane < mm && j < nc) {
+            const int *p = is_rhs(c) ? rp + lane : pp + lane + j * mm;
+            e0[c] = p[0];
+            ne[c] = p[1] - p[0];
+        }
+        kmax = max(kmax, ne[c]);
+    }
+    auto next_src = [&](int k) {
+#pragma unroll
+        for (int c = 0; c < CW; c++) {
+            const int *l = (is_rhs(c) ? S.pr_src : S.pa_src) + e0[c];
+#pragma unroll
+            for (int u = 0; u < kSrc; u++) src[c][u] = k + u < ne[c] ? l[k + u] : 0;
+        }
+    };
+    next_src(0);
+    __syncthreads();
+    T A[CW];
+#pragma unroll
+    for (int c = 0; c < CW; c++) {
+        const int j = warp + kMidWarps * c;
+        A[c] = lane < mm && j < nc ? F[lane + j * mm] : T(0);
+    }
+    wait();   // for the children (bounded); ends with a barrier
+    // ---- the children's entries, in child order, the loads of a round
+    // together ----
+    for (int k = 0; k < kmax; k += kSrc) {
+        T v[CW][kSrc];
+#pragma unroll
+        for (int c = 0; c < CW; c++)
+#pragma unroll
+            for (int u = 0; u < kSrc; u++) {
+                v[c][u] = T(0);
+                if (k + u < ne[c]) v[c][u] = is_rhs(c) ? (T)ldcg(uv + src[c][u]) : ldcg(fr + src[c][u]);
+            }
+        next_src(k + kSrc);
+#pragma unroll
+        for (int c = 0; c < CW; c++)
+#pragma unroll
+            for (int u = 0; u < kSrc; u++)
+                if (k + u < ne[c]) A[c] += v[c][u];
+    }
+    // ---- elimination ----
+    if (warp == 0) colbuf[lane] = A[0];
+    int rpos = lane < ns ? -1 : lane;   // row of the factored front, once known
+    for (int k = 0; k < ns; k++) {
+        __syncthreads();
+        const T v = colbuf[(k & 1) * 32 + lane];
+        // the pivot: the largest magnitude among the rows not yet taken, the
+        // smallest row on ties; beside the reductions each lane takes the
+        // reciprocal of its own candidate (a value that takes a division, a
+        // zero above all, waits for the choice)
+        const bool cand = rpos < 0;
+        const T own = cand ? v : T(1);
+        bool special = false;
+        T rown;
+        if constexpr (sizeof(T) == 8) {
+            special = recip_special(own);
+            rown = recip_normal(special ? 1.0 : own);
+        } else {
+            rown = recip(own);
+        }
+        const unsigned kh = cand ? key_hi(v) : 0u;
+        unsigned kl = 0, ml = 0;
+        const unsigned mh = __reduce_max_sync(FULL, kh);
+        if constexpr (sizeof(T) == 8) {
+            kl = cand && kh == mh ? key_lo(v) : 0u;
+            ml = __reduce_max_sync(FULL, kl);
+        }
+        const int pv = (int)__reduce_min_sync(FULL, cand && kh == mh && kl == ml ? (unsigned)lane : 32u);
+        if (tid == 0 && (mh | ml) == 0u) atomicOr(W.status + m, 4);
+        // the pivot row's entries of this warp's columns
+        T u[CW];
+#pragma unroll
+        for (int c = 0; c < CW; c++) u[c] = __shfl_sync(FULL, A[c], pv);
+        T inv = __shfl_sync(FULL, rown, pv);
+        if constexpr (sizeof(T) == 8)
+            if (__shfl_sync(FULL, (int)special, pv)) inv = T(1) / __shfl_sync(FULL, own, pv);
+        if (lane == pv) rpos = k;
+        const bool upd = (lane >= ns || rpos < 0) && lane < mm;
+        const T l = v * inv;
+#pragma unroll
+        for (int c = 0; c < CW; c++) {
+            const int j = warp + kMidWarps * c;
+            if (j > k && j < nc) {
+                const T t = A[c] - l * u[c];
+                if (upd) A[c] = t;
+                if (j == k + 1) colbuf[((k + 1) & 1) * 32 + lane] = A[c];
+            } else if (j == k) {
+                // the factored column: multipliers and the reciprocal
+                if (upd) A[c] = l;
+                if (lane == pv) A[c] = inv;
+            }
+        }
+    }
+    // ---- store: first what the parent reads (the update matrix and, with
+    // RHS, the update vector and the forward-solved entries), then done(),
+    // then the solve-ordered copies and the composed pivots ----
+    T *out = fr + S.front_off[s];
+    double *us = uv + S.uvec_off[s];
+#pragma unroll
+    for (int c = 0; c < CW; c++) {
+        const int j = warp + kMidWarps * c;
+        if (j >= ns && j < mm && lane >= ns && lane < mm) out[lane + j * mm] = A[c];
+        if (is_rhs(c) && lane < mm) {
+            if (lane < ns) x[start + rpos] = (double)A[c];
+            else us[lane - ns] = (double)A[c];
+        }
+    }
+    __syncthreads();
+    done();
+    T *lo = lfac ? lfac + (size_t)m * S.lu_total + S.lu_off[s] : nullptr;
+    T *uo = ufac + (size_t)m * S.lu_total + S.lu_off[s];
+#pragma unroll
+    for (int c = 0; c < CW; c++) {
+        const int j = warp + kMidWarps * c;
+        if (lane >= mm || j >= mm) continue;
+        if (j < ns && lo) lo[rpos + j * mm] = A[c];
+        if (lane < ns) uo[rpos + j * ns] = A[c];
+    }
+    if (warp == 0 && lane < ns) S.ipiv[(size_t)m * S.n + start + rpos] = lane;
+}
+
+// Ranks [r0, r1) of the order, one CTA per front; tasks claimed from counter
+// ctr.  The ranks below `from` were factored by earlier launches.
+template <class T, bool RHS>
+__global__ void __launch_bounds__(kMidThreads, 6) factor_mid_kernel(
+    DevProblem P, DevWork W, DevSym S, DevDag D, T *fronts, T *lfac, T *ufac, const uint8_t *mask, int want, int r0,
+    int r1, int ctr) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T *F = reinterpret_cast<T *>(smem_raw);
+    T *colbuf = reinterpret_cast<T *>(smem_raw + MidShape<T>::front_bytes);
+    __shared__ int s_task, s_ok;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int M = P.M;
+    const int epoch = *D.epoch;
+    const int n_tasks = (r1 - r0) * M;
+    for (;;) {
+        __syncthreads();
+        if (tid == 0) s_task = atomicAdd(D.ctr + ctr, 1);
+        __syncthreads();
+        const int t = s_task;
+        if (t >= n_tasks) break;
+        const int s = D.order[r0 + t / M], m = t % M;
+        if (mask[m] != want) continue;
+        auto wait = [&] {
+            if (tid < 32) {
+                const bool ok = warp_wait_children(S, D, D.fdone, s, m, M, epoch, r0);
+                if (lane == 0) s_ok = ok;
+            }
+            __syncthreads();
+            if (!s_ok && tid == 0) atomicOr(W.status + m, 8);
+        };
+        auto done = [&] {
+            if (tid == 0) signal_done(D.fdone + (size_t)s * M + m, epoch);
+        };
+        factor_mid<T, RHS>(P, W, S, fronts, lfac, ufac, s, m, F, colbuf, wait, done);
+    }
+}
+
 // Ranks [r0, r1) of the order, one warp per task, fronts of at most cap
 // rows; tasks claimed from counter ctr.
 template <class T, bool RHS>
@@ -1138,8 +1394,9 @@ __global__ void __launch_bounds__(kThreads, 3) factor_big_kernel(DevProblem P, D
     const int tid = threadIdx.x, lane = tid & 31;
     const int M = P.M;
     const int epoch = *D.epoch;
-    const int n_tasks = kSplit ? D.big_units * M : (D.nsup - D.n_small) * M;
-    const int t_tail = kSplit ? (D.tail0 - D.n_small) * M : n_tasks;   // first task of the tail
+    const int from = D.n_small;   // first rank
+    const int n_tasks = kSplit ? D.big_units * M : (D.nsup - from) * M;
+    const int t_tail = kSplit ? (D.tail0 - from) * M : n_tasks;   // first task of the tail
     // the tail's cumulative part counts, for the task decoding
     __shared__ int s_units[kSplitTailMax + 1];
     if (kSplit)
@@ -1155,7 +1412,7 @@ __global__ void __launch_bounds__(kThreads, 3) factor_big_kernel(DevProblem P, D
         // are consecutive tasks
         int rank, m, part = 0, np = 1;
         if (!kSplit || t < t_tail) {
-            rank = D.n_small + t / M;
+            rank = from + t / M;
             m = t % M;
         } else {
             const int u = t - t_tail;
@@ -1177,7 +1434,7 @@ __global__ void __launch_bounds__(kThreads, 3) factor_big_kernel(DevProblem P, D
         // entries that need nothing from them are in place
         auto wait = [&] {
             if (tid < 32) {
-                const bool ok = warp_wait_children(S, D, D.fdone, s, m, M, epoch, D.n_small, kSplit);
+                const bool ok = warp_wait_children(S, D, D.fdone, s, m, M, epoch, from, kSplit);
                 if (lane == 0) s_ok = ok;
             }
             __syncthreads();
@@ -1200,7 +1457,7 @@ __global__ void __launch_bounds__(kThreads, 3) factor_big_kernel(DevProblem P, D
 // previous solve no longer match.  The error flag stays raised until the
 // host clears it.
 __global__ void dag_begin_kernel(DevDag D) {
-    if (threadIdx.x < 8) D.ctr[threadIdx.x] = 0;
+    if (threadIdx.x < 16) D.ctr[threadIdx.x] = 0;
     if (threadIdx.x == 0) *D.epoch += 1;
 }
 
@@ -1226,7 +1483,7 @@ int configure_one(DagGrid &g, int nsm, int tiny_bytes, int small_bytes, int big_
         return -1;
     g.small = nsm * occ;
     if constexpr (sizeof(T) == 8) {
-        // the tiny fronts of FP64 factorisations: two scenarios a warp
+        // the tiny fronts: two scenarios a warp
         if (cudaFuncSetAttribute(factor_group_kernel<T, R, kTinyLanes>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  tiny_bytes) != cudaSuccess ||
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, factor_group_kernel<T, R, kTinyLanes>, kThreads,
@@ -1234,8 +1491,12 @@ int configure_one(DagGrid &g, int nsm, int tiny_bytes, int small_bytes, int big_
                 cudaSuccess || occ < 1)
             return -1;
         g.tiny = nsm * occ;
-    } else {
-        g.tiny = 0;
+        if (cudaFuncSetAttribute(factor_mid_kernel<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 MidShape<T>::bytes) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, factor_mid_kernel<T, R>, kMidThreads,
+                                                          MidShape<T>::bytes) != cudaSuccess || occ < 1)
+            return -1;
+        g.mid = nsm * occ;
     }
     if (cudaFuncSetAttribute(factor_big_kernel<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, big_bytes) !=
             cudaSuccess ||
@@ -1277,7 +1538,10 @@ int dag_configure(const DevDag &D, int fp32, DagGrid &g) {
     return 0;
 }
 
-int dag_small_front() { return kSmallFront; }
+int dag_factor_launches(const DevDag &D, int fp32) {
+    if (fp32) return (D.n_small > 0) + (D.nsup > D.n_small);
+    return (D.n_tiny > 0) + (D.n_small > D.n_tiny) + (D.nsup > D.n_small);
+}
 int dag_tiny_front() { return kTinyFront; }
 
 void launch_dag_begin(const DevDag &D, cudaStream_t st) { dag_begin_kernel<<<1, 32, 0, st>>>(D); }
@@ -1297,21 +1561,31 @@ template <class T>
 void launch_dag_factor(const DevProblem &P, const DevWork &W, const DevSym &S, const DevDag &D, const DagGrid &g,
                        T *fronts, T *lfac, T *ufac, const uint8_t *mask, int want, cudaStream_t st) {
     constexpr bool R = FusedRhs<T>::value;
-    const int n_tiny = sizeof(T) == 8 ? D.n_tiny : 0;
-    constexpr int G = 32 / kTinyLanes;
-    const long long tt = (long long)n_tiny * ((P.M + G - 1) / G), ts = (long long)(D.n_small - n_tiny) * P.M,
-                    tb = (long long)(sizeof(T) == 8 ? D.big_units : D.nsup - D.n_small) * P.M;
     if constexpr (sizeof(T) == 8) {
+        constexpr int G = 32 / kTinyLanes;
+        const long long tt = (long long)D.n_tiny * ((P.M + G - 1) / G), ts = (long long)(D.n_small - D.n_tiny) * P.M,
+                        tb = (long long)D.big_units * P.M;
         if (tt > 0)
             factor_group_kernel<T, R, kTinyLanes><<<blocks_for(g.tiny, tt, kWarps), kThreads, g.tiny_bytes, st>>>(
-                P, W, S, D, fronts, lfac, ufac, mask, want, 0, n_tiny, kTinyFront, 7);
+                P, W, S, D, fronts, lfac, ufac, mask, want, 0, D.n_tiny, kTinyFront, 7);
+        if (ts > kMidTasks)
+            factor_small_kernel<T, R><<<blocks_for(g.small, ts, kWarps), kThreads, g.small_bytes, st>>>(
+                P, W, S, D, fronts, lfac, ufac, mask, want, D.n_tiny, D.n_small, kSmallFront, 0);
+        else if (ts > 0)
+            factor_mid_kernel<T, R><<<blocks_for(g.mid, ts, 1), kMidThreads, MidShape<T>::bytes, st>>>(
+                P, W, S, D, fronts, lfac, ufac, mask, want, D.n_tiny, D.n_small, 0);
+        if (tb > 0)
+            factor_big_kernel<T, R><<<blocks_for(g.big, tb, 1), kThreads, g.big_bytes, st>>>(
+                P, W, S, D, fronts, lfac, ufac, mask, want);
+    } else {
+        const long long ts = (long long)D.n_small * P.M, tb = (long long)(D.nsup - D.n_small) * P.M;
+        if (ts > 0)
+            factor_small_kernel<T, R><<<blocks_for(g.small, ts, kWarps), kThreads, g.small_bytes, st>>>(
+                P, W, S, D, fronts, lfac, ufac, mask, want, 0, D.n_small, kSmallFront, 0);
+        if (tb > 0)
+            factor_big_kernel<T, R><<<blocks_for(g.big, tb, 1), kThreads, g.big_bytes, st>>>(
+                P, W, S, D, fronts, lfac, ufac, mask, want);
     }
-    if (ts > 0)
-        factor_small_kernel<T, R><<<blocks_for(g.small, ts, kWarps), kThreads, g.small_bytes, st>>>(
-            P, W, S, D, fronts, lfac, ufac, mask, want, n_tiny, D.n_small, kSmallFront, 0);
-    if (tb > 0)
-        factor_big_kernel<T, R><<<blocks_for(g.big, tb, 1), kThreads, g.big_bytes, st>>>(P, W, S, D, fronts, lfac,
-                                                                                          ufac, mask, want);
 }
 
 template void launch_dag_factor<double>(const DevProblem &, const DevWork &, const DevSym &, const DevDag &,

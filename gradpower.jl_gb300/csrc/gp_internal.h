@@ -178,18 +178,20 @@ struct DevMixed {
 };
 
 // Dataflow schedule of the multifrontal factorisation and solves
-// (gp_dag.cu).  order: supernodes of the small region (every front of the
-// subtree at most 32 rows) by level, then the others by level; a topological
-// order of the assembly tree.
+// (gp_dag.cu).  order: the supernodes by region (largest front of the
+// subtree: tiny, at most 32 rows, the rest) and by level within
+// a region; a topological order of the assembly tree.
 struct DevDag {
-    int nsup, n_small;
-    int n_tiny;                   // the first n_tiny ranks: subtrees with fronts of at most dag_tiny_front() rows
+    int nsup;
+    // ranks below n_tiny: subtrees with fronts of at most dag_tiny_front()
+    // rows; below n_small: at most 32
+    int n_tiny, n_small;
     int max_front, max_big_front;
     int max_big_whole;            // largest front of the CTA kernel that is not split (FP64)
     const int *order;       // [nsup]
     const int *rank;        // [nsup] position in order
     const int *parent;      // [nsup] parent supernode or -1
-    int *ctr;               // [8] claim counters: small factor, big factor, forward top, backward top,
+    int *ctr;               // [16] claim counters: factor up to 32 rows, big factor, forward top, backward top,
                             //     forward blocks, backward blocks, forward lower top, tiny factor
     int *epoch;             // [1] current solve
     int *err;               // [1] a wait gave up (sticky until the host clears it)
@@ -247,15 +249,15 @@ __host__ __device__ inline int split_cols_cap(int nc, int np) {
 }
 
 struct DagGrid {
-    int tiny = 0, small = 0, big = 0;                    // resident blocks
-    int tiny_bytes = 0, small_bytes = 0, big_bytes = 0;  // dynamic shared memory
+    int tiny = 0, small = 0, mid = 0, big = 0;            // resident blocks
+    int tiny_bytes = 0, small_bytes = 0, big_bytes = 0;     // dynamic shared memory
 };
 
 int dag_configure(const DevDag &D, int fp32, DagGrid &g);
 // launch_dag_factor<double> also does the forward solve (the right-hand side
 // rides along as an extra front column); launch_dag_factor<float> does not.
-int dag_small_front();
 int dag_tiny_front();
+int dag_factor_launches(const DevDag &D, int fp32);   // launches of one factorisation (one per region present)
 void launch_dag_begin(const DevDag &D, cudaStream_t st);
 // r[i] = the factorisations' reciprocal of x[i] (device arrays), i < n.
 void launch_recip_check(const double *x, double *r, int n, cudaStream_t st);
