@@ -53,7 +53,14 @@ struct ND {
     std::vector<int> set_id, lev, pos_in;
     std::vector<int> order;
     int next_id = 1;
-    static constexpr int LEAF = 48;
+    // sets of at most LEAF nodes are ordered by minimum degree as a whole;
+    // separators and sets that do not split, in chunks of CHUNK.  LEAF 6
+    // against 48: the tree of the 39-bus ring has 4 levels instead of 6, the
+    // one of 70,000 buses 23,567 supernodes instead of 26,477 and 14 levels
+    // instead of 16; FP64 runs of 70,000 buses x 8 57.0 -> 50.6 ms, 2,000 x
+    // 64 39.2 -> 34.6.  (8: 4 and 23,775; 4 and 3 have fewer flops but more
+    // supernodes.)
+    static constexpr int LEAF = 6, CHUNK = 48;
 
     explicit ND(const Graph &g)
         : G(g), set_id(g.n, 0), lev(g.n, -1), pos_in(g.n, -1), part(g.n, 0), stamp(g.n, 0) {}
@@ -83,9 +90,9 @@ struct ND {
     // Splits the connected set V into A, B and a separator S: the smallest
     // of the breadth-first level sets near the middle, seen from r and from
     // the far end, each then refined (part: 0 A, 1 B, 2 S).  Against the
-    // median level alone, unrefined, on the 70,000-bus grid: largest front
-    // 132 -> 40 rows, factorisation flops 33.7 -> 19.4 M a scenario, levels
-    // 30 -> 16; FP64 run of 8 scenarios x 18 steps 104 -> 58 ms (its
+    // median level alone, unrefined (and leaves of 48), on the 70,000-bus
+    // grid: largest front 132 -> 40 rows, factorisation flops 33.7 -> 19.4 M
+    // a scenario, levels 30 -> 16; FP64 run of 8 scenarios x 18 steps 104 -> 58 ms (its
     // factorisations 78 -> 36 ms), mixed (36 steps) 70 -> 56 ms; the analysis
     // itself 0.39 -> 0.6 s.
     std::vector<signed char> part;
@@ -275,7 +282,7 @@ struct ND {
             // own adjacency (ties in BFS order)
             std::vector<int> tmp = V;
             while (!tmp.empty()) {
-                size_t take = std::min<size_t>(LEAF, tmp.size());
+                size_t take = std::min<size_t>(CHUNK, tmp.size());
                 std::vector<int> chunk(tmp.begin(), tmp.begin() + take);
                 leaf_min_degree(G, chunk, pos_in, order);
                 tmp.erase(tmp.begin(), tmp.begin() + take);
@@ -289,8 +296,8 @@ struct ND {
         run(A, ida);
         run(B, idb);
         // separator nodes: order them by minimum degree in chunks
-        for (size_t a = 0; a < S.size(); a += LEAF) {
-            std::vector<int> chunk(S.begin() + a, S.begin() + std::min(S.size(), a + LEAF));
+        for (size_t a = 0; a < S.size(); a += CHUNK) {
+            std::vector<int> chunk(S.begin() + a, S.begin() + std::min(S.size(), a + CHUNK));
             leaf_min_degree(G, chunk, pos_in, order);
         }
     }
