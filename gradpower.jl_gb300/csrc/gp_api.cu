@@ -56,15 +56,31 @@ void ck(cudaError_t e, const char *what) {
 // legacy default stream (cudaStreamNonBlocking), so a plain cudaMemcpy would
 // not be ordered before the kernels launched on it.
 struct DeviceArena {
+    // Small arrays share blocks of kBlock bytes (a layout holds about 150 of
+    // them, and each cudaMalloc costs microseconds), at 256-byte boundaries
+    // as cudaMalloc's own; the others get an allocation each.
+    static constexpr size_t kBlock = 1 << 20, kShared = 1 << 17;
     std::vector<void *> ptrs;
+    unsigned char *block = nullptr;
+    size_t used = 0;
     cudaStream_t st = nullptr;
+    void *raw(size_t bytes) {
+        void *p = nullptr;
+        const cudaError_t e = cudaMalloc(&p, bytes);
+        if (e != cudaSuccess) fail(GP_E_NOMEM, "cudaMalloc of %zu bytes: %s", bytes, cudaGetErrorString(e));
+        ptrs.push_back(p);
+        return p;
+    }
     template <class T>
     T *alloc(size_t n) {
-        void *p = nullptr;
-        if (n == 0) n = 1;
-        cudaError_t e = cudaMalloc(&p, n * sizeof(T));
-        if (e != cudaSuccess) fail(GP_E_NOMEM, "cudaMalloc of %zu bytes: %s", n * sizeof(T), cudaGetErrorString(e));
-        ptrs.push_back(p);
+        const size_t bytes = (std::max<size_t>(n, 1) * sizeof(T) + 255) & ~size_t(255);
+        if (bytes > kShared) return (T *)raw(bytes);
+        if (!block || used + bytes > kBlock) {
+            block = (unsigned char *)raw(kBlock);
+            used = 0;
+        }
+        unsigned char *p = block + used;
+        used += bytes;
         return (T *)p;
     }
     template <class T>
@@ -83,6 +99,7 @@ struct DeviceArena {
     void release() {
         for (void *p : ptrs) cudaFree(p);
         ptrs.clear();
+        block = nullptr;
     }
 };
 
@@ -133,6 +150,7 @@ struct gp_layout {
     cudaGraphExec_t g_loop = nullptr;
     cudaGraphConditionalHandle h_loop = 0, h_var = 0;
     int *d_cnt = nullptr;
+    bool one_cta = false;        // this call runs on the small-system kernel
     bool profiling = false;      // host-driven loop with phase events (gp_set_profiling)
     // line trips (gp_set_line_trips): expanded per scenario, with their
     // off-diagonal assembly entries; statuses reset at every call
@@ -190,6 +208,7 @@ struct gp_layout {
     gp::DagGrid G64, G32;
     gp::DevBlk B{};
     gp::SolveGrid SG;
+    gp::DevSmall small{};   // small systems: one CTA a scenario
     int n_top_levels = 0;
     // mixed-precision solver: kept FP32 factors (allocated on first use)
     gp::DevMixed Mx{};
@@ -1285,6 +1304,56 @@ void build_blocks(gp_layout *L, const gp::Symbolic &sym) {
     if (sc != 0) fail(GP_E_CUDA, "could not configure the solve kernels");
 }
 
+// Lists of the one-CTA path (build_small) from the plan: the fronts' places in
+// shared memory, their constant entries, where the scenario's entries and the
+// right-hand sides go, and every child's extend-add.
+void small_lists(gp_layout *L, const Plan &pl) {
+    constexpr int kSmallRed = 512;
+    const gp::Symbolic &sym = pl.sym;
+    if (sym.max_front > gp::kSmallMaxFront || L->n_red > kSmallRed) return;
+    gp::DevSmall &D = L->small;
+    std::vector<int4> desc(sym.nsup);
+    int64_t total = 0;
+    for (int s = 0; s < sym.nsup; s++) {
+        const int mm = sym.front_m(s);
+        desc[s] = make_int4(sym.sup_start[s], sym.front_n(s), mm, (int)total);
+        total += (int64_t)mm * (mm + 1);
+    }
+    if (total > 20000) return;
+    D.front_total = (int)total;
+    D.n_levels = sym.nlevels;
+    DeviceArena &A = L->arena;
+    D.desc = A.upload(desc);
+    std::vector<double> fc(total, 0.0);
+    std::vector<int> vp, vi, rhs(L->n_red), ea_ptr(1, 0);
+    std::vector<int2> ea;
+    for (int s = 0; s < sym.nsup; s++) {
+        const int4 d = desc[s];
+        for (int e = pl.acp[s]; e < pl.acp[s + 1]; e++) fc[d.w + pl.acpos[e]] += pl.acval[e];
+        for (int e = pl.avp[s]; e < pl.avp[s + 1]; e++) {
+            vp.push_back(d.w + pl.avpos[e]);
+            vi.push_back(pl.avidx[e]);
+        }
+        for (int i = 0; i < d.y; i++) rhs[d.x + i] = d.w + d.z * d.z + i;
+        // update matrix and update vector into the parent's front
+        const int r = sym.front_r(s), p = sym.parent[s];
+        const int *rel = sym.relmap.data() + sym.relmap_ptr[s];
+        if (p >= 0)
+            for (int b = 0; b <= r; b++)
+                for (int a = 0; a < r; a++)
+                    ea.push_back(make_int2(desc[p].w + rel[a] + (b < r ? rel[b] : desc[p].z) * desc[p].z,
+                                           d.w + (d.y + a) + (d.y + b) * d.z));
+        ea_ptr.push_back((int)ea.size());
+    }
+    D.front_const = A.upload(fc);
+    D.n_var_ent = (int)vp.size();
+    D.var_pos = A.upload(vp);
+    D.var_idx = A.upload(vi);
+    D.rhs_pos = A.upload(rhs);
+    D.ea_ptr = A.upload(ea_ptr);
+    D.ea = A.upload(ea);
+}
+
 void build_problem(gp_layout *L, const gp_problem *pr) {
     using namespace gp;
     Plan &pl = *new Plan();
@@ -1430,6 +1499,7 @@ void build_problem(gp_layout *L, const gp_problem *pr) {
     L->sym = pl.sym;
     build_dag(L, sym);
     build_blocks(L, sym);
+    small_lists(L, pl);
 }
 
 void build_work(gp_layout *L, const double *z0, const double *u0, const double *p) {
@@ -1571,6 +1641,28 @@ void build_clusters(gp_layout *L, const gp_problem *pr, const double *z0, const 
     const int bytes = cp.max_slots * 32 * (int)sizeof(double);
     if (bytes > 48 * 1024 && (gp::cluster_smem_optin(bytes) < 0 || gp::adj_smem_optin(bytes) < 0))
         fail(GP_E_CUDA, "cluster kernel needs %d bytes of shared memory", bytes);
+}
+
+// The one-CTA path for small systems: systems of at most kSmallTasks cluster
+// tasks whose fronts a warp holds and whose scenario fits a SM's shared
+// memory.  (FP64 integrations and the adjoint's forward run; the host-driven
+// profiling loop keeps the batch kernels.)
+void build_small(gp_layout *L) {
+    constexpr int kSmallTasks = 4;
+    const gp::Symbolic &sym = L->sym;
+    gp::DevSmall &D = L->small;
+    if (D.front_total == 0 || L->C.n_tasks > kSmallTasks) return;
+    D.bytes = gp::small_shared_bytes(L->P, L->C, D);
+    int dev = 0, limit = 0;
+    ck(cudaGetDevice(&dev), "cudaGetDevice");
+    ck(cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "device attribute");
+    if (D.bytes + 1024 > limit) return;
+    if (gp::small_configure(D.bytes) != 0) fail(GP_E_CUDA, "could not configure the small-system kernel");
+    D.lev_ptr = L->arena.upload(sym.level_ptr);
+    D.lev_sup = L->arena.upload(sym.level_sups);
+    D.state_bus = L->d_state_maps;
+    D.red_of = L->d_state_maps + L->n_da;
+    D.on = 1;
 }
 
 void drop_graphs(gp_layout *L) {
@@ -1929,11 +2021,13 @@ void ensure_graphs(gp_layout *L, double tol, int itermax, int solver) {
     const bool mixed = solver == GP_SOLVER_SCHUR_MIXED;
     if (mixed) ensure_mixed(L);
     L->Mx.on = mixed ? 1 : 0;
+    L->one_cta = L->small.on && solver == GP_SOLVER_SCHUR_FP64 && !L->profiling;
     L->graph_tol = tol;
     L->graph_itermax = itermax;
     L->solver = solver;
     const int plain = solver == GP_SOLVER_SHARED_WOODBURY ? -2 : -1;
     if (solver == GP_SOLVER_SHARED_WOODBURY) ensure_woodbury(L);
+    if (L->one_cta) return;
     if (!L->profiling) {
         if (!L->g_loop) L->g_loop = build_loop(L, tol, itermax, mixed, plain);
         return;
@@ -2035,6 +2129,15 @@ void cluster_images(gp_layout *L, double dt, bool resolves) {
     gp::launch_cluster_image(L->P, L->W, L->C, dt, L->st);
     if (resolves) gp::launch_cluster_image(L->P, L->W, L->C, 0.0, L->st);
     if (L->C.n_tasks > 0) L->launches += resolves ? 2 : 1;
+}
+
+// Steps k0 + 1 .. k1 on the small-system kernel (slot 1: the dt = 0
+// re-solve of the active scenarios after step k0 + 1).
+void small_steps(gp_layout *L, const gp_options *opt, double dt, int k0, int k1, int slot, int *iters, double *traj,
+                 long long stride) {
+    const gp::SmallRun R{dt, opt->newton_tol, opt->itermax, k0, k1, slot, slot, iters, traj, stride};
+    gp::launch_small(L->P, L->W, L->S, L->C, L->small, R, L->st);
+    L->launches += 1;
 }
 
 // Event steps of the current fault table, and per step the scenarios whose
@@ -2147,6 +2250,7 @@ int32_t gp_layout_create(const gp_problem *prob, int32_t M, const double *z0, co
     build_problem(L, prob);
     build_work(L, z0, u0, p);
     build_clusters(L, prob, z0, u0, p);
+    build_small(L);
     L->h_adj_ptr.assign(prob->adj_rowptr, prob->adj_rowptr + prob->n_bus + 1);
     L->h_adj.assign(prob->adj_colidx, prob->adj_colidx + prob->adj_rowptr[prob->n_bus]);
     if (gp_set_line_trips(L, 0, nullptr) != GP_OK) fail(GP_E_CUDA, "%s", g_last_error.c_str());
@@ -2373,6 +2477,16 @@ int32_t gp_integrate(gp_layout *L, const gp_options *opt, int32_t n_faults, cons
     const int predict = opt->solver == GP_SOLVER_SCHUR_MIXED ? L->mx_predict : 0;
     int smooth = 0;   // earlier states on the current smooth stretch
     for (int k = 1; k <= ns; k++) {
+        if (L->one_cta) {
+            // the steps up to the next event in one launch (64 at most: a
+            // launch stays within milliseconds, and a pinned trajectory
+            // is copied out while the next one runs)
+            int ke = k;
+            while (ke < ns && ke < k + 63 && !ev_steps.count(ke)) ke++;
+            small_steps(L, opt, opt->dt, k - 1, ke, 0, d_iters, d_traj, (long long)(ns + 1) * nsys);
+            for (; k < ke; k++) send_slice(k);
+            if (d_traj) send_slice(k);
+        } else {
         ck(cudaMemcpyAsync(L->W.zold, L->W.z, (size_t)M * nsys * sizeof(double), cudaMemcpyDeviceToDevice, L->st),
            "zold");
         if (predict) {
@@ -2392,6 +2506,7 @@ int32_t gp_integrate(gp_layout *L, const gp_options *opt, int32_t n_faults, cons
                "snapshot");
             send_slice(k);
         }
+        }
         if (ev_steps.count(k)) {
             ck(cudaMemsetAsync(L->W.active, 0, M, L->st), "memset");
             gp::launch_events(L->P, L->W, L->d_fl_on_step, L->d_fl_off_step, L->d_fl_scen, L->d_fl_on, L->n_fl, k,
@@ -2402,6 +2517,10 @@ int32_t gp_integrate(gp_layout *L, const gp_options *opt, int32_t n_faults, cons
                                    k, L->st);
             // an exciter that went offline changes its cluster's constants
             if (dc_steps.count(k)) cluster_images(L, opt->dt, true);
+            if (L->one_cta) {
+                small_steps(L, opt, 0.0, k - 1, k, 1, d_iters, nullptr, 0);
+                continue;
+            }
             ck(cudaMemcpyAsync(L->W.zold, L->W.z, (size_t)M * nsys * sizeof(double), cudaMemcpyDeviceToDevice,
                                L->st),
                "zold");
@@ -2442,6 +2561,8 @@ int32_t gp_integrate(gp_layout *L, const gp_options *opt, int32_t n_faults, cons
         to_host(L, traj, d_traj, (size_t)M * (ns + 1) * nsys * sizeof(double), "trajectory copy");
     std::vector<int> hi((size_t)2 * std::max(ns, 1) * M);
     to_host(L, hi.data(), d_iters, hi.size() * sizeof(int), "iters copy");
+    if (L->one_cta)
+        for (int q = 0; q < 2 * ns; q++) L->solves += *std::max_element(hi.begin() + (size_t)q * M, hi.begin() + (size_t)(q + 1) * M);
     double tot = 0.0;
     for (int m = 0; m < M; m++) {
         double s = 0.0;
@@ -2649,6 +2770,18 @@ int32_t gp_adjoint(gp_layout *L, const gp_options *opt, int32_t n_faults, const 
     // one forward step k; after(0) runs after the regular solve, after(1)
     // after the re-solve of the scenarios whose faults toggle at k
     auto step = [&](int k, auto after) {
+        if (L->one_cta) {
+            small_steps(L, opt, opt->dt, k - 1, k, 0, nullptr, nullptr, 0);
+            after(0);
+            if (ev.count(k)) {
+                ck(cudaMemsetAsync(L->W.active, 0, M, L->st), "memset");
+                launch_events(L->P, L->W, L->d_fl_on_step, L->d_fl_off_step, L->d_fl_scen, L->d_fl_on, L->n_fl, k,
+                              L->st);
+                small_steps(L, opt, 0.0, k - 1, k, 1, nullptr, nullptr, 0);
+                after(1);
+            }
+            return;
+        }
         ck(cudaMemcpyAsync(L->W.zold, L->W.z, blk * sizeof(double), cudaMemcpyDeviceToDevice, L->st), "zold");
         ck(cudaMemsetAsync(L->W.active, 1, M, L->st), "memset");
         solve_step(L, opt->dt, opt->newton_tol, opt->itermax, false);

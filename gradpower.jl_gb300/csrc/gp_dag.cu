@@ -144,7 +144,6 @@ struct KeyOf<float> {
 
 __device__ __forceinline__ unsigned key_hi(double v) { return (unsigned)__double2hiint(v) & 0x7fffffffu; }
 __device__ __forceinline__ unsigned key_lo(double v) { return (unsigned)__double2loint(v); }
-__device__ __forceinline__ unsigned key_hi(float v) { return __float_as_uint(v) & 0x7fffffffu; }
 
 // LW < 32: the warp is LW-lane segments, each searching its own front (the
 // whole warp calls it).  A whole warp takes the maximum by integer
@@ -1189,21 +1188,12 @@ __device__ void factor_mid(const DevProblem &P, const DevWork &W, const DevSym &
         // zero above all, waits for the choice)
         const bool cand = rpos < 0;
         const T own = cand ? v : T(1);
-        bool special = false;
-        T rown;
-        if constexpr (sizeof(T) == 8) {
-            special = recip_special(own);
-            rown = recip_normal(special ? 1.0 : own);
-        } else {
-            rown = recip(own);
-        }
+        const bool special = recip_special(own);
+        const T rown = recip_normal(special ? 1.0 : own);
         const unsigned kh = cand ? key_hi(v) : 0u;
-        unsigned kl = 0, ml = 0;
         const unsigned mh = __reduce_max_sync(FULL, kh);
-        if constexpr (sizeof(T) == 8) {
-            kl = cand && kh == mh ? key_lo(v) : 0u;
-            ml = __reduce_max_sync(FULL, kl);
-        }
+        const unsigned kl = cand && kh == mh ? key_lo(v) : 0u;
+        const unsigned ml = __reduce_max_sync(FULL, kl);
         const int pv = (int)__reduce_min_sync(FULL, cand && kh == mh && kl == ml ? (unsigned)lane : 32u);
         if (tid == 0 && (mh | ml) == 0u) atomicOr(W.status + m, 4);
         // the pivot row's entries of this warp's columns
@@ -1211,8 +1201,7 @@ __device__ void factor_mid(const DevProblem &P, const DevWork &W, const DevSym &
 #pragma unroll
         for (int c = 0; c < CW; c++) u[c] = __shfl_sync(FULL, A[c], pv);
         T inv = __shfl_sync(FULL, rown, pv);
-        if constexpr (sizeof(T) == 8)
-            if (__shfl_sync(FULL, (int)special, pv)) inv = T(1) / __shfl_sync(FULL, own, pv);
+        if (__shfl_sync(FULL, (int)special, pv)) inv = T(1) / __shfl_sync(FULL, own, pv);
         if (lane == pv) rpos = k;
         const bool upd = (lane >= ns || rpos < 0) && lane < mm;
         const T l = v * inv;

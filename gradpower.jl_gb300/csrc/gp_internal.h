@@ -8,6 +8,19 @@
 
 namespace gp {
 
+// Raises a kernel's dynamic shared-memory limit to `bytes`; never lowers it
+// (the limit belongs to the kernel, and layouts of other sizes may be alive).
+template <class K>
+bool raise_shared_limit(K *kernel, int bytes) {
+    cudaFuncAttributes a;
+    if (cudaFuncGetAttributes(&a, kernel) == cudaSuccess &&
+        (a.maxDynamicSharedSizeBytes >= bytes ||
+         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess))
+        return true;
+    cudaGetLastError();
+    return false;
+}
+
 // Struct-of-arrays device table on the GPU (see gp_device_table).
 struct DTab {
     int n;
@@ -392,6 +405,39 @@ void launch_events(const DevProblem &P, const DevWork &W, const int *fl_on_step,
                    const int *fl_scen, uint8_t *fl_on, int n_fl, int step, cudaStream_t st);
 void launch_snapshot(const double *z, double *traj, int M, int n_sys, int n_steps, int k, cudaStream_t st);
 int cluster_smem_optin(int bytes);
+
+// Small systems, one CTA a scenario (gp_small.cu).
+constexpr int kSmallMaxFront = 32;   // a lane a row
+struct DevSmall {
+    int on = 0;            // the layout's FP64 integrations take this path
+    int bytes = 0;         // dynamic shared memory
+    int n_levels = 0;
+    int front_total = 0;   // entries of all fronts with their right-hand-side columns
+    const int *lev_ptr, *lev_sup;   // supernodes by level
+    const int4 *desc;               // [nsup] first unknown, pivots, rows, offset of the front
+    const double *front_const;      // [front_total] constant entries of S
+    int n_var_ent = 0;
+    const int *var_pos, *var_idx;   // scenario entries: place in the fronts, svar index
+    const int *rhs_pos;             // [n_red] place of each unknown's right-hand side
+    const int *ea_ptr;              // [nsup+1] a child's extend-add entries:
+    const int2 *ea;                 //     place in the parent's front, place in its own
+    const int *state_bus, *red_of;  // as update_kernel
+};
+// Steps k0 + 1 .. k1 of every scenario (masked: of the active ones) from W.z
+// with time step dt: Newton counts to iters[(2 k + slot) * M + m], the state
+// after step k to traj[m * traj_stride + k * n_sys].  The cluster images of
+// dt must be current.
+struct SmallRun {
+    double dt, tol;
+    int itermax, k0, k1, slot, masked;
+    int *iters;            // may be null
+    double *traj;          // may be null
+    long long traj_stride;
+};
+int small_shared_bytes(const DevProblem &P, const DevClu &C, const DevSmall &D);
+int small_configure(int bytes);
+void launch_small(const DevProblem &P, const DevWork &W, const DevSym &S, const DevClu &C, const DevSmall &D,
+                  const SmallRun &R, cudaStream_t st);
 
 // Discrete adjoint of the backward-Euler step (gp_adjoint.cu).
 struct DevAdj {

@@ -25,8 +25,10 @@
 
 #include <algorithm>
 
+#include "gp_cluster.cuh"
 #include "gp_devices.cuh"
 #include "gp_internal.h"
+#include "gp_network.cuh"
 #include "gp_warp.cuh"
 
 namespace gp {
@@ -36,14 +38,6 @@ namespace gp {
 // ---------------------------------------------------------------------------
 // helpers
 // ---------------------------------------------------------------------------
-
-__device__ __forceinline__ unsigned long long norm_bits(double v) {
-    // the bit pattern of |v| (non-negative doubles order like their bit
-    // patterns); NaN counts as +inf.  Integer operations only: the FP64
-    // pipe is the scarce one on this GPU.
-    const unsigned long long a = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
-    return a > 0x7ff0000000000000ull ? 0x7ff0000000000000ull : a;
-}
 
 // ---------------------------------------------------------------------------
 // cluster kernels: one lane per (cluster, scenario), 32 clusters of one
@@ -71,54 +65,6 @@ __device__ __forceinline__ unsigned long long norm_bits(double v) {
 // mixed solver's (mostly kept factors) 70,000 x 8 85 -> 58 us.
 // ---------------------------------------------------------------------------
 
-__device__ __forceinline__ DevRef devref(const DTab &T, int k) {
-    DevRef d;
-    d.dp = T.diff_ptr[k];
-    d.ap = T.alg_ptr[k];
-    d.cp = T.ctrl_ptr[k];
-    d.pp = T.par_ptr[k];
-    d.bus = T.bus[k];
-    d.link0 = T.link0[k];
-    d.link1 = T.link1[k];
-    return d;
-}
-
-// The warps' shares of a cluster's evaluation: 0 the machine's flux rows, 1
-// its network-frame rows (C, I) and the exciter, 2 the governor, 3 the
-// stabiliser.  `off` receives the entries of an offline exciter.
-template <class Sink, class Off, class KP>
-__device__ __forceinline__ void eval_share(const DevProblem &P, int c, int share, const double *z, const double *u0,
-                                           const double *p, Sink &sink, Off &off, double Cc[6], double Ic[2],
-                                           const KP &kc, bool exc_on) {
-    if (share == 0) {
-        genrou_flux(devref(P.dev[0], P.cl_gen[c]), z, u0, p, sink, kc);
-    } else if (share == 1) {
-        const int et = P.cl_exc_type[c], iex = P.cl_exc[c];
-        const DevRef dg = devref(P.dev[0], P.cl_gen[c]);
-        DevRef dex{};
-        if (et == 3 || et == 4) dex = devref(P.dev[et], iex);
-        genrou_stator(dg, P.net, z, sink, Cc, Ic);
-        if (exc_on) {
-            if (et == 3) sexs_eval(dex, P.net, z, p, sink, kc);
-            else if (et == 4) esdc1a_eval(dex, P.net, z, p, sink, kc);
-        } else {
-            if (et == 3) sexs_eval(dex, P.net, z, p, off, kc);
-            else if (et == 4) esdc1a_eval(dex, P.net, z, p, off, kc);
-        }
-    } else if (share == 2) {
-        const int gt = P.cl_gov_type[c], igv = P.cl_gov[c];
-        if (gt == 1) ieesgo_eval(devref(P.dev[1], igv), z, p, sink, kc);
-        else if (gt == 2) tgov1_eval(devref(P.dev[2], igv), z, p, sink, kc);
-    } else {
-        const int ip = P.cl_pss[c];
-        if (ip >= 0) ieeest_eval(devref(P.dev[5], ip), z, p, sink, kc);
-    }
-}
-
-__device__ __forceinline__ bool exciter_on(const DevProblem &P, int m, int c) {
-    return !P.exc_off || !P.exc_off[(size_t)m * P.n_cl + c];
-}
-
 // Image of the constant entries: the slot keeps the entry with the
 // backward-Euler scaling (rows of the class's differential mask) and the
 // diagonal's one.  ON false: an offline exciter, whose rows hold (the
@@ -141,42 +87,6 @@ struct ImageSink {
     }
     __device__ __forceinline__ void putv(int, int, double) {}
     __device__ __forceinline__ void putf(int, double) {}
-};
-
-// State-dependent entries, the B columns and the backward-Euler residual
-// (its norm in nb).  Same scaling as ImageSink.
-template <bool ON>
-struct LaneSink {
-    double *v;
-    const short *slot_of;
-    const double *z, *zold;
-    int ws, lane;
-    unsigned diff;
-    double dt;
-    unsigned long long *nb;
-    __device__ __forceinline__ void put(int r, int c, double x) {
-        const int lr = r - ws;
-        const bool d = diff >> lr & 1;
-        double y = ON ? x : 0.0;
-        if (d) y = __dmul_rn(y, -dt);
-        if (d && r == c) y = __dadd_rn(y, 1.0);
-        v[(int)__ldg(slot_of + lr * 32 + (c - ws)) * 32 + lane] = y;
-    }
-    __device__ __forceinline__ void putc(int, int, double) {}
-    __device__ __forceinline__ void putv(int r, int k, double x) {
-        const int lr = r - ws;
-        double y = ON ? x : 0.0;
-        if (diff >> lr & 1) y = __dmul_rn(y, -dt);
-        v[(int)__ldg(slot_of + lr * 32 + 29 + k) * 32 + lane] = y;
-    }
-    __device__ __forceinline__ void putf(int r, double x) {
-        const int lr = r - ws;
-        double y = ON ? x : 0.0;
-        if (diff >> lr & 1) y = z[r] - zold[r] - dt * y;
-        v[(int)__ldg(slot_of + lr * 32 + 31) * 32 + lane] = y;
-        const unsigned long long t = norm_bits(y);
-        *nb = t > *nb ? t : *nb;
-    }
 };
 
 // Once per integration, one warp per (task, scenario): the parameter
@@ -217,64 +127,15 @@ __global__ void __launch_bounds__(32) cluster_image_kernel(DevProblem P, DevWork
     for (int s = 0; s < n_img; s++) img[(size_t)s * 32] = vals[s * 32 + lane];
 }
 
-// A staged stream of record pairs (CluRec) by one of the task's warps: v0 +
-// offsets for d and b, va + offsets for a.  The next pair is read ahead.
-template <class T>
-__device__ __forceinline__ void run_stages(const int4 *q, int n, T *v0, const T *va, int lane) {
-    v0 += lane;
-    va += lane;
-    int4 r0 = __ldg(q), r1 = __ldg(q + 1);
-    for (int i = 0; i < n; i++) {
-        const int4 c0 = r0, c1 = r1;
-        if (i + 1 < n) {
-            r0 = __ldg(q + 2 * i + 2);
-            r1 = __ldg(q + 2 * i + 3);
-        }
-        const int code = c0.w & 255;
-        if (code == (REC_FMS | REC_FMS << 4)) {
-            const T a0 = va[c0.y], b0 = v0[c0.z], a1 = va[c1.y], b1 = v0[c1.z];
-            T d0 = v0[c0.x], d1 = v0[c1.x];
-            d0 -= a0 * b0;
-            d1 -= a1 * b1;
-            v0[c0.x] = d0;
-            v0[c1.x] = d1;
-        } else if (code == REC_FMS) {
-            v0[c0.x] -= va[c0.y] * v0[c0.z];
-        } else if (code == REC_MUL) {
-            v0[c0.x] *= va[c0.y];
-        } else if (code == (REC_MUL | REC_MUL << 4)) {
-            const T a0 = va[c0.y], a1 = va[c1.y];
-            const T d0 = v0[c0.x], d1 = v0[c1.x];
-            v0[c0.x] = d0 * a0;
-            v0[c1.x] = d1 * a1;
-        } else if (code == REC_RCP) {
-            v0[c0.x] = recip(va[c0.y]);
-        }
-        if (c0.w & REC_SYNC) __syncthreads();
-    }
-}
-
-__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-
-// Warp maximum of ordered norm bits.
-__device__ __forceinline__ unsigned long long warp_max(unsigned long long v) {
-    const unsigned hi = (unsigned)(v >> 32), lo = (unsigned)v;
-    const unsigned mh = __reduce_max_sync(FULL_MASK, hi);
-    const unsigned ml = __reduce_max_sync(FULL_MASK, hi == mh ? lo : 0u);
-    return (unsigned long long)mh << 32 | ml;
-}
-
-constexpr int kCluThreads = 32 * kCluWarps;
-
 // Modes per scenario: 0 exact Newton (Jacobian block, FP64 LU, three solves;
 // also the mixed solver's MX_EXACT); 1 the same, and the LU values and
 // coupling rows are kept in FP32 for the following iterations (MX_FP32).
 // The mixed solver's MX_KEEP scenarios (residual only, solved with the kept
 // FP32 LU) run cluster_keep_kernel instead.
+struct CtaSync {
+    __device__ __forceinline__ void operator()() const { __syncthreads(); }
+};
+
 __global__ void __launch_bounds__(kCluThreads, 4) cluster_kernel(DevProblem P, DevWork W, DevClu Cl, DevMixed Mx) {
     extern __shared__ __align__(16) double vals[];
     __shared__ unsigned long long s_nb[kCluWarps];
@@ -284,60 +145,29 @@ __global__ void __launch_bounds__(kCluThreads, 4) cluster_kernel(DevProblem P, D
     if (r == MX_KEEP) return;
     const int mode = r == MX_FP32 ? 1 : 0;
     const int cls = Cl.task_class[task];
-    const int cnt = Cl.task_count[task];
-    const bool act = lane < cnt;
+    const bool act = lane < Cl.task_count[task];
     const int c = Cl.order[Cl.task_first[task] + (act ? lane : 0)];
-    const int ws = P.cl_w_start[c], Wn = P.cl_w_size[c];
-    const int rb = Cl.rhs_base[cls], n_img = Cl.n_img[cls];
+    const int rb = Cl.rhs_base[cls];
     const double dt = *W.dt;
     // the constant slots arrive while the devices are evaluated
-    {
-        const double *img = Cl.img + ((((size_t)(dt == 0.0) * P.M + m) * Cl.n_tasks + task) * Cl.max_img) * 32;
-        for (int e = tid; e < n_img * 16; e += kCluThreads) cp_async16(vals + 2 * e, img + 2 * e);
-    }
-    double *R0 = vals + (size_t)rb * 32, *R1 = R0 + (size_t)Wn * 32, *R2 = R1 + (size_t)Wn * 32;
-    for (int e = tid; e < 2 * Wn * 32; e += kCluThreads) R0[e] = 0.0;
-    if (!act) {
-        // idle lanes factor an identity so that none divides by zero
-        const unsigned char *base = Cl.base + (size_t)cls * Cl.base_stride;
-        for (int s = n_img + warp; s < rb; s += kCluWarps) vals[s * 32 + lane] = base[s] & 2 ? 1.0 : 0.0;
-        for (int j = warp; j < Wn; j += kCluWarps) R2[j * 32 + lane] = 0.0;
-    }
-    __syncthreads();
+    load_image(P, Cl, task, m, dt, vals, tid);
     double Cc[6] = {0, 0, 0, 0, 0, 0}, Ic[2] = {0, 0};   // warp 1
-    unsigned long long nb = 0ull;
-    if (act) {
-        const double *z = W.z + (size_t)m * P.n_sys, *zold = W.zold + (size_t)m * P.n_sys;
-        const short *so = Cl.slot_of + (size_t)cls * 1024;
-        const unsigned diff = Cl.diff_mask[cls];
-        LaneSink<true> on{vals, so, z, zold, ws, lane, diff, dt, &nb};
-        LaneSink<false> off{vals, so, z, zold, ws, lane, diff, dt, &nb};
-        const LoadK lk{Cl.kc + (((size_t)m * Cl.n_tasks + task) * kConstSlots) * 32 + lane, 32};
-        eval_share(P, c, warp, z, W.u0 + (size_t)m * P.n_ctrl, W.p + (size_t)m * P.n_par, on, off, Cc, Ic, lk,
-                   exciter_on(P, m, c));
-    }
-    nb = warp_max(nb);
-    if (lane == 0) s_nb[warp] = nb;
-    cp_async_wait();
-    __syncthreads();
+    cluster_fill(P, Cl, task, m, W.z + (size_t)m * P.n_sys, W.zold + (size_t)m * P.n_sys,
+                 W.u0 + (size_t)m * P.n_ctrl, W.p + (size_t)m * P.n_par, dt, vals, tid, s_nb, Cc, Ic, CtaSync());
     if (tid == 0) {
+        unsigned long long nb = s_nb[0];
 #pragma unroll
         for (int w = 1; w < kCluWarps; w++) nb = s_nb[w] > nb ? s_nb[w] : nb;
         atomicMax(W.norm + m, nb);
     }
-    const int4 *stream = reinterpret_cast<const int4 *>(Cl.full) + 2 * (size_t)Cl.full_ptr[cls * kCluWarps + warp];
-    const int n_pairs = Cl.full_ptr[cls * kCluWarps + warp + 1] - Cl.full_ptr[cls * kCluWarps + warp];
-    const int n_da = P.n_diff + P.n_alg;
-    double *yx = W.yx + (size_t)m * 3 * n_da + ws;
-    const int *pc = Cl.perm_col + cls * 32, *p3 = Cl.pos3 + cls * 3;
-    double X0[3], X1[3], X2[3];   // warp 1
+    double *yx = W.yx + (size_t)m * 3 * (P.n_diff + P.n_alg), *o = W.clout + ((size_t)m * P.n_cl + c) * 8;
     if (mode == 1) {
         // MX_FP32: the factors are kept in FP32, so the factorisation and
         // the three solves run in FP32 too.  The slots are converted in
         // place, eight a warp at a time: float slot s lies in the first half
         // of double slot s / 2, which an earlier round or this one has read
         float *fv = reinterpret_cast<float *>(vals);
-        const int nslot = rb + 3 * Wn;
+        const int nslot = rb + 3 * P.cl_w_size[c];
         for (int s0 = 0; s0 < nslot; s0 += 8 * kCluWarps) {
             float x[8];
 #pragma unroll
@@ -353,57 +183,22 @@ __global__ void __launch_bounds__(kCluThreads, 4) cluster_kernel(DevProblem P, D
             }
             __syncthreads();
         }
-        run_stages<float>(stream, n_pairs, fv, fv, lane);
-        __syncthreads();
+        cluster_solve<float>(Cl, cls, fv, tid, CtaSync());
         float *keep = Mx.lu + (((size_t)m * Cl.n_tasks + task) * Mx.n_lu) * 32 + lane;
         for (int s = warp; s < rb; s += kCluWarps) keep[(size_t)s * 32] = fv[s * 32 + lane];
         if (!act) return;
-        const float *F0 = fv + (size_t)rb * 32, *F1 = F0 + (size_t)Wn * 32, *F2 = F1 + (size_t)Wn * 32;
-        for (int j = warp; j < Wn; j += kCluWarps) {
-            const int st = pc[j];
-            yx[st] = (double)F2[j * 32 + lane];
-            yx[n_da + st] = (double)F0[j * 32 + lane];
-            yx[2 * n_da + st] = (double)F1[j * 32 + lane];
-        }
-        if (warp != 1) return;
-#pragma unroll
-        for (int t = 0; t < 3; t++) {
-            X0[t] = (double)F2[p3[t] * 32 + lane];
-            X1[t] = (double)F0[p3[t] * 32 + lane];
-            X2[t] = (double)F1[p3[t] * 32 + lane];
-        }
+        cluster_out<float>(P, Cl, cls, c, fv, tid, Cc, Ic, yx, o);
     } else {
         // factorisation and solves in FP64
-        run_stages<double>(stream, n_pairs, vals, vals, lane);
-        __syncthreads();
+        cluster_solve<double>(Cl, cls, vals, tid, CtaSync());
         if (Cl.save_lu) {
             double *sv = Cl.save_lu + (((size_t)m * Cl.n_tasks + task) * Cl.n_save) * 32 + lane;
             for (int s = warp; s < rb; s += kCluWarps) sv[(size_t)s * 32] = vals[s * 32 + lane];
         }
         if (!act) return;
-        for (int j = warp; j < Wn; j += kCluWarps) {
-            const int st = pc[j];
-            yx[st] = R2[j * 32 + lane];
-            yx[n_da + st] = R0[j * 32 + lane];
-            yx[2 * n_da + st] = R1[j * 32 + lane];
-        }
-        if (warp != 1) return;
-#pragma unroll
-        for (int t = 0; t < 3; t++) {
-            X0[t] = R2[p3[t] * 32 + lane];
-            X1[t] = R0[p3[t] * 32 + lane];
-            X2[t] = R1[p3[t] * 32 + lane];
-        }
+        cluster_out<double>(P, Cl, cls, c, vals, tid, Cc, Ic, yx, o);
     }
-    double *o = W.clout + ((size_t)m * P.n_cl + c) * 8;
-    o[0] = Cc[0] * X1[0] + Cc[1] * X1[1] + Cc[2] * X1[2];
-    o[1] = Cc[0] * X2[0] + Cc[1] * X2[1] + Cc[2] * X2[2];
-    o[2] = Cc[3] * X1[0] + Cc[4] * X1[1] + Cc[5] * X1[2];
-    o[3] = Cc[3] * X2[0] + Cc[4] * X2[1] + Cc[5] * X2[2];
-    o[4] = Cc[0] * X0[0] + Cc[1] * X0[1] + Cc[2] * X0[2];
-    o[5] = Cc[3] * X0[0] + Cc[4] * X0[1] + Cc[5] * X0[2];
-    o[6] = Ic[0];
-    o[7] = Ic[1];
+    if (warp != 1) return;
     if (mode == 1) {
         float *cc = Mx.cc + ((size_t)m * P.n_cl + c) * 6;
         for (int t = 0; t < 6; t++) cc[t] = (float)Cc[t];
@@ -490,7 +285,7 @@ __global__ void __launch_bounds__(kCluThreads, 6) cluster_keep_kernel(DevProblem
         atomicMax(W.norm + m, nb);
     }
     run_stages<float>(reinterpret_cast<const int4 *>(Cl.sol) + 2 * (size_t)Cl.sol_ptr[cls * kCluWarps + warp],
-                      Cl.sol_ptr[cls * kCluWarps + warp + 1] - Cl.sol_ptr[cls * kCluWarps + warp], Rf, lu, lane);
+                      Cl.sol_ptr[cls * kCluWarps + warp + 1] - Cl.sol_ptr[cls * kCluWarps + warp], Rf, lu, lane, CtaSync());
     __syncthreads();
     if (!act) return;
     const int n_da = P.n_diff + P.n_alg;
@@ -575,24 +370,16 @@ void launch_zip_const(const DevProblem &P, const DevWork &W, double *out, cudaSt
 }
 
 int cluster_smem_optin(int bytes) {
-    if (cudaFuncSetAttribute(cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess ||
-        cudaFuncSetAttribute(cluster_image_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(cluster_keep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) !=
-            cudaSuccess) {
-        cudaGetLastError();
-        return -1;
-    }
-    return bytes;
+    return raise_shared_limit(cluster_kernel, bytes) && raise_shared_limit(cluster_image_kernel, bytes) &&
+                   raise_shared_limit(cluster_keep_kernel, bytes)
+               ? bytes
+               : -1;
 }
 
 // ---------------------------------------------------------------------------
 // network kernel
 // ---------------------------------------------------------------------------
 
-// With the mixed solver, a scenario iterating on kept factors needs only the
-// residual and the right-hand side: the entries of S (diagonal blocks,
-// static-generator couplings) are skipped for it.
 __global__ void __launch_bounds__(64) network_kernel(DevProblem P, DevWork W, DevMixed Mx, int want_f,
                                                       int skip_s) {
     const long long task = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -603,187 +390,11 @@ __global__ void __launch_bounds__(64) network_kernel(DevProblem P, DevWork W, De
     const int b = valid ? P.bus_order[(int)(task % P.n_bus)] : 0;
     const bool act = valid && W.active[m];
     unsigned long long nb = 0ull;
-    if (act) {
-        const bool need_s = !skip_s && !(Mx.on && Mx.refac[m] == MX_KEEP);
-        const double *z = W.z + (size_t)m * P.n_sys;
-        const double *p = W.p + (size_t)m * P.n_par;
-        const int net = P.net;
-        const double vr = z[net + 2 * b], vi = z[net + 2 * b + 1];
-        double fr = 0.0, fi = 0.0, d00 = 0.0, d01 = 0.0, d10 = 0.0, d11 = 0.0, rr = 0.0, ri = 0.0;
-        for (int q = P.y_rowptr[b]; q < P.y_rowptr[b + 1]; q++) {
-            const int j = P.y_colidx[q];
-            const double2 y = P.y_val[q];   // one 16-byte load
-            const double g = y.x, bb = y.y;
-            const double vrj = z[net + 2 * j], vij = z[net + 2 * j + 1];
-            // -(g + j bb)(vrj + j vij), two FMAs per part
-            fr = fma(-g, vrj, fma(bb, vij, fr));
-            fi = fma(-bb, vrj, fma(-g, vij, fi));
-            if (need_s && j == b) { d00 -= g; d01 += bb; d10 -= bb; d11 -= g; }
-        }
-        for (int q = P.bus_cl_ptr[b]; q < P.bus_cl_ptr[b + 1]; q++) {
-            const double *o = W.clout + ((size_t)m * P.n_cl + P.bus_cl[q]) * 8;
-            if (need_s) { d00 -= o[0]; d01 -= o[1]; d10 -= o[2]; d11 -= o[3]; }
-            rr += o[4]; ri += o[5];
-            fr += o[6]; fi += o[7];
-        }
-        const DTab &ZL = P.dev[6];
-        for (int q = P.bus_zl_ptr[b]; q < P.bus_zl_ptr[b + 1]; q++) {
-            const int k = P.bus_zl[q];
-            if (P.zl_off && P.zl_off[(size_t)m * ZL.n + k]) continue;
-            // the load's parameter products ((1 - al) P, (1 - al) Q, al y0),
-            // from the table zip_const_kernel fills once per call
-            const double *kz = P.zl_k + ((size_t)m * ZL.n + k) * 4;
-            const double A1 = kz[0], A2 = kz[1], B1 = kz[2], B2 = kz[3];
-            const double vm2 = vr * vr + vi * vi, vm2_tld = 0.2;
-            const bool above = vm2 > vm2_tld;
-            // one division per load (FP64 division is dear here)
-            const double inv = 1.0 / (above ? vm2 : vm2_tld);
-            // the constant-impedance part al*y0 and the constant-power part
-            // (1 - al)(P - jQ)/max(|V|^2, 0.2) multiply the same V: one
-            // complex admittance a + jc; f -= (a + jc) V in FMA form
-            const double a = fma(inv, A1, B1), c = fma(inv, A2, B2);
-            fr = fma(vi, c, fma(-vr, a, fr));
-            fi = fma(-vi, a, fma(-vr, c, fi));
-            if (!need_s) continue;
-            double p11, p12, p21, p22;
-            if (above) {
-                const double iv4 = inv * inv;
-                p11 = ((A1 * vr - A2 * vi) * 2.0 * vr - A1 * vm2) * iv4;
-                p12 = ((A1 * vr - A2 * vi) * 2.0 * vi + A2 * vm2) * iv4;
-                p21 = ((A2 * vr + A1 * vi) * 2.0 * vr - A2 * vm2) * iv4;
-                p22 = ((A2 * vr + A1 * vi) * 2.0 * vi - A1 * vm2) * iv4;
-            } else {
-                p11 = -A1 * inv;
-                p12 = A2 * inv;
-                p21 = -A2 * inv;
-                p22 = -A1 * inv;
-            }
-            d00 += -B1 + p11;
-            d01 += B2 + p12;
-            d10 += -B2 + p21;
-            d11 += -B1 + p22;
-        }
-        const DTab &SG = P.dev[7];
-        for (int q = P.bus_sg_ptr[b]; q < P.bus_sg_ptr[b + 1]; q++) {
-            const int k = P.bus_sg[q];
-            if (P.sg_off && P.sg_off[(size_t)m * SG.n + k]) continue;   // constant-power ones only
-            const int pp = SG.par_ptr[k], ap = SG.alg_ptr[k], bt = SG.link0[k];
-            const double vm2r = vr * vr + vi * vi, vm2 = vm2r > 0.2 ? vm2r : 0.2;
-            double Pg, Qg;
-            if (bt == 2) { Pg = p[pp]; Qg = z[ap]; }
-            else if (bt == 3) { Pg = z[ap]; Qg = z[ap + 1]; }
-            else { Pg = p[pp]; Qg = p[pp + 1]; }
-            const double irn = Pg * vr + Qg * vi, iin = Pg * vi - Qg * vr;
-            const double inv = 1.0 / vm2;
-            fr += irn * inv;
-            fi += iin * inv;
-            if (!need_s) {
-                double *xp = W.xperm + (size_t)m * P.n_red;
-                const int r0 = P.sg_red[k];
-                if (bt == 2) {
-                    const double vset = p[pp + 2];
-                    const double fa = vr * vr + vi * vi - vset * vset;
-                    xp[P.iperm[r0]] = -fa;
-                    if (want_f) W.f[(size_t)m * P.n_sys + ap] = fa;
-                    const unsigned long long t = norm_bits(fa);
-                    nb = t > nb ? t : nb;
-                } else if (bt == 3) {
-                    const double vset = p[pp + 2], aset = p[pp + 3];
-                    const double fa0 = vr - vset * cos(aset), fa1 = vi - vset * sin(aset);
-                    xp[P.iperm[r0]] = -fa0;
-                    xp[P.iperm[r0 + 1]] = -fa1;
-                    if (want_f) {
-                        W.f[(size_t)m * P.n_sys + ap] = fa0;
-                        W.f[(size_t)m * P.n_sys + ap + 1] = fa1;
-                    }
-                    unsigned long long t = norm_bits(fa0);
-                    nb = t > nb ? t : nb;
-                    t = norm_bits(fa1);
-                    nb = t > nb ? t : nb;
-                }
-                continue;
-            }
-            if (vm2r > 0.2) {
-                const double iv4 = inv * inv;
-                d00 += Pg * inv - 2.0 * vr * irn * iv4;
-                d01 += Qg * inv - 2.0 * vi * irn * iv4;
-                d10 += -Qg * inv - 2.0 * vr * iin * iv4;
-                d11 += Pg * inv - 2.0 * vi * iin * iv4;
-            } else {
-                d00 += Pg * inv;
-                d01 += Qg * inv;
-                d10 += -Qg * inv;
-                d11 += Pg * inv;
-            }
-            double *sv = W.svar + (size_t)m * P.n_var + P.sg_var[k];
-            double *xp = W.xperm + (size_t)m * P.n_red;
-            const int r0 = P.sg_red[k];
-            if (bt == 2) {
-                const double vset = p[pp + 2];
-                const double fa = vr * vr + vi * vi - vset * vset;
-                // (ap,vr) (ap,vi) (vr,ap) (vi,ap)
-                sv[0] = 2.0 * vr; sv[1] = 2.0 * vi; sv[2] = vi * inv; sv[3] = -vr * inv;
-                xp[P.iperm[r0]] = -fa;
-                if (want_f) W.f[(size_t)m * P.n_sys + ap] = fa;
-                const unsigned long long t = norm_bits(fa);
-                nb = t > nb ? t : nb;
-            } else if (bt == 3) {
-                const double vset = p[pp + 2], aset = p[pp + 3];
-                const double fa0 = vr - vset * cos(aset), fa1 = vi - vset * sin(aset);
-                // (ap,vr) (ap+1,vi) (vr,ap) (vi,ap) (vr,ap+1) (vi,ap+1)
-                sv[0] = 1.0; sv[1] = 1.0; sv[2] = vr * inv; sv[3] = vi * inv; sv[4] = vi * inv; sv[5] = -vr * inv;
-                xp[P.iperm[r0]] = -fa0;
-                xp[P.iperm[r0 + 1]] = -fa1;
-                if (want_f) {
-                    W.f[(size_t)m * P.n_sys + ap] = fa0;
-                    W.f[(size_t)m * P.n_sys + ap + 1] = fa1;
-                }
-                unsigned long long t = norm_bits(fa0);
-                nb = t > nb ? t : nb;
-                t = norm_bits(fa1);
-                nb = t > nb ? t : nb;
-            }
-        }
-        // tripped lines: their Ybus terms removed (f = -Y V gains
-        // +y_line V; the S diagonal block gains the realified y_line)
-        for (int e = P.tr_ptr[m]; e < P.tr_ptr[m + 1]; e++) {
-            if (!P.tr_on[e]) continue;
-            const int fb = P.tr_from[e], tb = P.tr_to[e];
-            if (fb != b && tb != b) continue;
-            const double *y = P.tr_y + 8 * (size_t)e + (fb == b ? 0 : 4);   // (yff, yft) or (ytf, ytt)
-            const double ybr = fb == b ? y[0] : y[2], ybi = fb == b ? y[1] : y[3];
-            const double yor = fb == b ? y[2] : y[0], yoi = fb == b ? y[3] : y[1];
-            const int o = fb == b ? tb : fb;
-            const double vro = z[net + 2 * o], vio = z[net + 2 * o + 1];
-            fr += ybr * vr - ybi * vi + yor * vro - yoi * vio;
-            fi += ybi * vr + ybr * vi + yoi * vro + yor * vio;
-            if (need_s) { d00 += ybr; d01 -= ybi; d10 += ybi; d11 += ybr; }
-        }
-        for (int e = P.fl_ptr[m]; e < P.fl_ptr[m + 1]; e++) {
-            if (P.fl_on[e] && P.fl_bus[e] == b) {
-                const double yf = P.fl_yf[e];
-                fr -= yf * vr;
-                fi -= yf * vi;
-                d00 -= yf;
-                d11 -= yf;
-            }
-        }
-        if (want_f) {
-            W.f[(size_t)m * P.n_sys + net + 2 * b] = fr;
-            W.f[(size_t)m * P.n_sys + net + 2 * b + 1] = fi;
-        }
-        if (need_s) {
-            double *sv = W.svar + (size_t)m * P.n_var + 4 * b;
-            sv[0] = d00; sv[1] = d01; sv[2] = d10; sv[3] = d11;
-        }
-        double *xp = W.xperm + (size_t)m * P.n_red;
-        xp[P.iperm[2 * b]] = -(fr - rr);
-        xp[P.iperm[2 * b + 1]] = -(fi - ri);
-        unsigned long long t = norm_bits(fr);
-        nb = t > nb ? t : nb;
-        t = norm_bits(fi);
-        nb = t > nb ? t : nb;
-    }
+    if (act)
+        nb = network_bus(P, m, b, W.z + (size_t)m * P.n_sys, W.p + (size_t)m * P.n_par,
+                         W.clout + (size_t)m * P.n_cl * 8, W.svar + (size_t)m * P.n_var,
+                         W.xperm + (size_t)m * P.n_red, want_f ? W.f + (size_t)m * P.n_sys : nullptr,
+                         !skip_s && !(Mx.on && Mx.refac[m] == MX_KEEP));
     // segmented max over lanes of the same scenario, one atomic per segment
     const int lane = threadIdx.x & 31;
 #pragma unroll

@@ -32,7 +32,7 @@
 // words, and the tasks that consume them poll those words directly, so that
 // a hand-off costs one store and the polls that see it, with no fence.
 //
-// Within a front, one warp holds up to kMaxJ rows per lane in registers
+// Within a front, one warp holds up to eight rows per lane in registers
 // (row i in lane i % 32, register i / 32).  The unit-lower and upper
 // triangular parts are swept column by column, the pivot value broadcast by
 // a shuffle; the factor columns are read chunk by chunk ahead of the
@@ -56,6 +56,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "gp_front.cuh"
 #include "gp_internal.h"
 #include "gp_warp.cuh"
 
@@ -67,7 +68,6 @@ constexpr unsigned FULL = kFullMask;
 constexpr int kBlkWarps = 4;   // block tasks per CTA
 constexpr int kTopThreads = 128;             // threads of a top-region task
 constexpr int kTopStage = 20 * 1024;         // shared memory for a task's factor columns
-constexpr int kMaxJ = 8;       // register rows per lane: fronts up to 256 rows
 constexpr int kBlkFront = 64;  // largest front inside a block (two rows per lane)
 
 __host__ __device__ constexpr int align16(int b) { return (b + 15) & ~15; }
@@ -146,28 +146,6 @@ template <class T>
 __device__ __forceinline__ const T *ufac(const FrontSel &fs, const DevSym &S, int m) {
     return Fac<T>::u(fs) + (size_t)(fs.shared ? 0 : m) * S.lu_total;
 }
-
-template <class T, int J>
-__device__ __forceinline__ T pick(const T (&r)[J], int j) {
-    T v = r[0];
-#pragma unroll
-    for (int q = 1; q < J; q++)
-        if (j == q) v = r[q];
-    return v;
-}
-
-template <class T, int J>
-__device__ __forceinline__ void place(T (&r)[J], int j, T v) {
-#pragma unroll
-    for (int q = 0; q < J; q++)
-        if (j == q) r[q] = v;
-}
-
-// Columns read per chunk of a sweep.
-template <int J>
-struct Chunk {
-    static constexpr int value = J <= 2 ? 8 : (J <= 4 ? 4 : 2);
-};
 
 // ---- forward elimination -------------------------------------------------
 // Sweeps columns k in [k0, k1) of the unit-lower factor over rows (k, mm):
@@ -268,58 +246,7 @@ __device__ void fwd_cols(const T *F, int ld, int kbase, int k0, int k1, int ns, 
     }
 }
 
-// ---- backward substitution -----------------------------------------------
-// U12 columns c in [c0, c1) (front columns, ns <= c < mm):
-// v[i] -= U(i, c) v[c] for i < ns, U(i, c) = F[i + (c - cbase) * ld].
-template <class T, int LW = 32>
-__device__ __forceinline__ void bwd_u12(const T *__restrict__ F, int ld, int cbase, int c0, int c1, int ns, T *v) {
-    warp_row_dots<T, LW>(F + (c0 - cbase) * ld, 1, ld, ns, c1 - c0, [&](int a) { return v[c0 + a]; },
-                         [&](int i, T acc) { v[i] -= acc; });
-    __syncwarp();
-}
-
-// U11 columns k from k1 - 1 down to k0: v[k] *= U(k, k) (the stored
-// reciprocal pivot), then v[i] -= U(i, k) v[k] for i < k.
-template <class T, int J, int CH = Chunk<J>::value, int LW = 32>
-__device__ void bwd_cols_j(const T *__restrict__ F, int ld, int kbase, int k0, int k1, int ns, T *v) {
-    const int lane = threadIdx.x & (LW - 1);
-    T r[J];
-#pragma unroll
-    for (int j = 0; j < J; j++) {
-        const int i = lane + LW * j;
-        r[j] = i < ns ? v[i] : T(0);
-    }
-    for (int kc = k1 - 1; kc >= k0; kc -= CH) {
-        T c[CH][J], d[CH];
-#pragma unroll
-        for (int kk = 0; kk < CH; kk++) {
-            const int k = kc - kk;
-            d[kk] = k >= k0 ? F[k + (k - kbase) * ld] : T(0);
-#pragma unroll
-            for (int j = 0; j < J; j++) {
-                const int i = lane + LW * j;
-                c[kk][j] = (k >= k0 && i < k) ? F[i + (k - kbase) * ld] : T(0);
-            }
-        }
-#pragma unroll
-        for (int kk = 0; kk < CH; kk++) {
-            const int k = kc - kk;
-            if (k >= k0) {
-                const T tk = __shfl_sync(FULL, pick(r, k / LW), k % LW, LW) * d[kk];
-                if (lane == k % LW) place(r, k / LW, tk);
-#pragma unroll
-                for (int j = 0; j < J; j++) r[j] -= c[kk][j] * tk;
-            }
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < J; j++) {
-        const int i = lane + LW * j;
-        if (i < ns) v[i] = r[j];
-    }
-    __syncwarp();
-}
-
+// ---- backward substitution: gp_front.cuh (register path) -------------------
 template <class T>
 __device__ void bwd_cols_smem(const T *__restrict__ F, int ld, int kbase, int k0, int k1, T *v) {
     const int lane = threadIdx.x & 31;
