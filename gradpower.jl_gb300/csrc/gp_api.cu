@@ -1643,10 +1643,15 @@ void build_clusters(gp_layout *L, const gp_problem *pr, const double *z0, const 
         fail(GP_E_CUDA, "cluster kernel needs %d bytes of shared memory", bytes);
 }
 
-// The one-CTA path for small systems: systems of at most kSmallTasks cluster
-// tasks whose fronts a warp holds and whose scenario fits a SM's shared
-// memory.  (FP64 integrations and the adjoint's forward run; the host-driven
-// profiling loop keeps the batch kernels.)
+// The one-CTA path for small systems (FP64 integrations and the adjoint's
+// forward run; the host-driven profiling loop keeps the batch kernels):
+// systems of at most kSmallTasks cluster tasks, fronts that a warp holds and a
+// scenario that fits a SM's shared memory, with a SM for every scenario, or
+// up to three scenarios a SM for the smallest.  24 steps through a fault, ms,
+// batch kernels against this (buses, machines; scenarios 1, 152, 400):
+// 12, 4: 4.8 / 2.1, 5.1 / 2.1, 5.3 / 4.2; 39, 10: 6.8 / 3.1, 7.4 / 3.1, 8.3 /
+// 6.6; 80, 20: 6.4 / 4.3, 7.2 / 4.4, 8.1 / 9.7; 120, 40: 7.9 / 5.5, 8.7 / 5.5,
+// 12.8 / 16.2.
 void build_small(gp_layout *L) {
     constexpr int kSmallTasks = 4;
     const gp::Symbolic &sym = L->sym;
@@ -1657,6 +1662,9 @@ void build_small(gp_layout *L) {
     ck(cudaGetDevice(&dev), "cudaGetDevice");
     ck(cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "device attribute");
     if (D.bytes + 1024 > limit) return;
+    int nsm = 0;
+    ck(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev), "device attribute");
+    if (L->M > nsm && !(L->C.n_tasks <= 1 && L->n_red <= 128 && L->M <= 3 * nsm)) return;
     if (gp::small_configure(D.bytes) != 0) fail(GP_E_CUDA, "could not configure the small-system kernel");
     D.lev_ptr = L->arena.upload(sym.level_ptr);
     D.lev_sup = L->arena.upload(sym.level_sups);
