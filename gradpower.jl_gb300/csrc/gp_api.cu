@@ -131,6 +131,10 @@ struct gp_layout {
     size_t traj_cap = 0;
     cudaStream_t st_copy = nullptr;
     cudaEvent_t ev_snap = nullptr;
+    // workspace of gp_adjoint (kept between calls, grown on demand)
+    DeviceArena adj_arena;
+    double *adj_buf = nullptr;
+    size_t adj_bytes = 0;
     double *d_zl_k = nullptr;   // DevProblem::zl_k
     int *d_state_maps = nullptr;   // state_bus then red_of
     int *d_gen_w = nullptr;        // z index of every machine's speed deviation
@@ -2162,24 +2166,24 @@ std::map<int, std::vector<uint8_t>> event_masks(const gp_layout *L) {
 }
 
 // One transposed Newton-Jacobian solve of the adjoint for the active
-// scenarios at the current state W.z (time step dt, current fault status):
+// scenarios at the state z (time step dt, current fault status):
 // g holds the right-hand side on entry and E lambda on exit; lambda and the
 // parameter partials go to A.
-void adj_solve(gp_layout *L, const gp::DevAdj &A, const gp::DevClu &Csave, double dt) {
+void adj_solve(gp_layout *L, double *z, const gp::DevAdj &A, const gp::DevClu &Csave, double dt) {
     using namespace gp;
-    const size_t M = L->M, nsys = L->n_sys;
     launch_set_double(L->W.dt, dt, L->st);
-    ck(cudaMemcpyAsync(L->W.zold, L->W.z, M * nsys * sizeof(double), cudaMemcpyDeviceToDevice, L->st), "zold");
+    // (the residual is not used: zold = z)
+    DevWork W = L->W;
+    W.z = W.zold = z;
     const DevMixed exact{};
-    launch_cluster(L->P, L->W, Csave, exact, L->st);
-    launch_network(L->P, L->W, exact, 0, L->st);
-    launch_adj_rhs(L->P, L->W, Csave, A, L->st);
+    launch_cluster(L->P, W, Csave, exact, L->st);
+    launch_network(L->P, W, exact, 0, L->st);
+    launch_adj_rhs(L->P, W, Csave, A, L->st);
     launch_dag_begin(L->D, L->st);
-    launch_dag_factor<double>(L->P, L->W, L->ST, L->D, L->G64, L->ST.fronts, nullptr, L->ST.ufac, L->W.active, 1,
-                              L->st);
-    launch_solve_bwd(L->P, L->W, L->ST, L->B, L->D, L->SG, FrontSel{nullptr, nullptr, L->ST.lfac, L->ST.ufac, nullptr, 1},
+    launch_dag_factor<double>(L->P, W, L->ST, L->D, L->G64, L->ST.fronts, nullptr, L->ST.ufac, W.active, 1, L->st);
+    launch_solve_bwd(L->P, W, L->ST, L->B, L->D, L->SG, FrontSel{nullptr, nullptr, L->ST.lfac, L->ST.ufac, nullptr, 1},
                      L->st);
-    launch_adj_back(L->P, L->W, Csave, A, L->d_state_maps, L->st);
+    launch_adj_back(L->P, W, Csave, A, L->d_state_maps, L->st);
     ck(cudaGetLastError(), "adjoint launch");
 }
 
@@ -2199,6 +2203,7 @@ void free_layout(gp_layout *L) {
     if (L->st_copy) cudaStreamSynchronize(L->st_copy);
     L->call.release();
     L->traj_arena.release();
+    L->adj_arena.release();
     L->fault_arena.release();
     L->iters_arena.release();
     L->dc_arena.release();
@@ -2253,7 +2258,7 @@ int32_t gp_layout_create(const gp_problem *prob, int32_t M, const double *z0, co
     ck(cudaStreamCreateWithFlags(&L->st, cudaStreamNonBlocking), "stream");
     ck(cudaStreamCreateWithFlags(&L->st_copy, cudaStreamNonBlocking), "stream");
     for (DeviceArena *a : {&L->arena, &L->call, &L->traj_arena, &L->trip_arena, &L->fault_arena, &L->iters_arena,
-                           &L->dc_arena})
+                           &L->dc_arena, &L->adj_arena})
         a->st = L->st;
     build_problem(L, prob);
     build_work(L, z0, u0, p);
@@ -2762,11 +2767,50 @@ int32_t gp_adjoint(gp_layout *L, const gp_options *opt, int32_t n_faults, const 
     // device copies of the re-solve masks
     std::map<int, uint8_t *> d_mask;
     for (const auto &kv : ev) d_mask[kv.first] = L->call.upload(kv.second);
-    DeviceArena &CA = L->call;
-    const int nck = (ns + K - 1) / K;                       // checkpoints at steps 0, K, 2K, ...
-    double *ckp = CA.alloc<double>(blk * nck);
-    double *seg = CA.alloc<double>(blk * 2 * K);           // per step: regular and re-solve states
-    double *zfin = CA.alloc<double>(blk);
+    // the states of every solve are kept when they fit a quarter of the free
+    // device memory; else the checkpoints (at steps 0, K, 2K, ...) and one
+    // segment's.  The workspace stays with the layout, up to kAdjKeep bytes
+    constexpr size_t kAdjKeep = size_t(4) << 30;
+    const int nck = (ns + K - 1) / K;
+    std::map<int, int> ev_slot;   // event step -> its re-solve state's slot
+    for (const auto &kv : ev) {
+        const int i = (int)ev_slot.size();
+        ev_slot[kv.first] = ns + i;
+    }
+    const size_t n_all = (size_t)ns + ev.size(), n_seg = nck + (size_t)2 * K;
+    size_t mem_free = 0, mem_total = 0;
+    ck(cudaMemGetInfo(&mem_free, &mem_total), "memory info");
+    const bool keep_all = n_all <= n_seg || n_all * blk * sizeof(double) <= (mem_free + L->adj_bytes) / 4;
+    DevClu Cs = L->C;
+    Cs.n_save = 1;
+    for (int v : L->cplan.rhs_base) Cs.n_save = std::max(Cs.n_save, v);
+    const size_t n_cl = std::max(1, L->P.n_cl), n_par = std::max(1, L->n_par);
+    const size_t n_lu = (size_t)M * std::max(1, Cs.n_tasks) * Cs.n_save * 32;
+    const size_t sizes[] = {(keep_all ? n_all : n_seg) * blk, blk, blk, blk, M * n_cl * 2, M * n_par, (size_t)M,
+                            n_lu, M * n_cl * 6};
+    size_t total = 0;
+    for (size_t n : sizes) total += (n + 31) & ~size_t(31);
+    if (total * sizeof(double) > L->adj_bytes) {
+        L->adj_arena.release();
+        L->adj_bytes = 0;
+        L->adj_buf = L->adj_arena.alloc<double>(total);
+        L->adj_bytes = total * sizeof(double);
+    }
+    double *next = L->adj_buf;
+    auto take = [&](size_t n) {
+        double *p = next;
+        next += (n + 31) & ~size_t(31);
+        return p;
+    };
+    double *states = take(sizes[0]), *zfin = take(blk);
+    double *ckp = states, *seg = states + nck * blk;   // (not keep_all)
+    auto state_at = [&](int k, int kind, int ka) {     // step k's solve (kind 0) or re-solve (1)
+        return keep_all ? states + blk * (kind ? (size_t)ev_slot.at(k) : (size_t)k - 1)
+                        : seg + blk * (2 * (size_t)(k - ka - 1) + kind);
+    };
+    auto put_state = [&](double *dst) {
+        ck(cudaMemcpyAsync(dst, L->W.z, blk * sizeof(double), cudaMemcpyDeviceToDevice, L->st), "state");
+    };
     L->launches = L->factor_launches = L->solves = 0;
     L->refreshes = L->exact_iters = L->retries = 0;
     for (int i = 0; i < 8; i++) L->ph_ms[i] = 0.0;
@@ -2803,13 +2847,13 @@ int32_t gp_adjoint(gp_layout *L, const gp_options *opt, int32_t n_faults, const 
             after(1);
         }
     };
-    // ---- forward, keeping the checkpoints ----
-    ck(cudaMemcpyAsync(ckp, L->W.z, blk * sizeof(double), cudaMemcpyDeviceToDevice, L->st), "checkpoint");
+    // ---- forward, keeping every state or the checkpoints ----
+    if (!keep_all) put_state(ckp);
     for (int k = 1; k <= ns; k++) {
-        step(k, [](int) {});
-        if (k % K == 0 && k / K < nck)
-            ck(cudaMemcpyAsync(ckp + blk * (k / K), L->W.z, blk * sizeof(double), cudaMemcpyDeviceToDevice, L->st),
-               "checkpoint");
+        step(k, [&](int kind) {
+            if (keep_all) put_state(state_at(k, kind, 0));
+        });
+        if (!keep_all && k % K == 0 && k / K < nck) put_state(ckp + blk * (k / K));
     }
     ck(cudaMemcpyAsync(zfin, L->W.z, blk * sizeof(double), cudaMemcpyDeviceToDevice, L->st), "final state");
     if (status) {
@@ -2818,11 +2862,11 @@ int32_t gp_adjoint(gp_layout *L, const gp_options *opt, int32_t n_faults, const 
     }
     // ---- backward sweep ----
     DevAdj A{};
-    A.g = CA.alloc<double>(blk);
-    A.lam = CA.alloc<double>(blk);
-    A.cadj = CA.alloc<double>((size_t)M * std::max(1, L->P.n_cl) * 2);
-    A.grad = CA.alloc<double>((size_t)M * std::max(1, L->n_par));
-    A.J = CA.alloc<double>(M);
+    A.g = take(blk);
+    A.lam = take(blk);
+    A.cadj = take(M * n_cl * 2);
+    A.grad = take(M * n_par);
+    A.J = take(M);
     A.gen_w = L->d_gen_w;
     A.n_gen = L->n_gen;
     A.w_speed = obj->w_speed;
@@ -2832,40 +2876,31 @@ int32_t gp_adjoint(gp_layout *L, const gp_options *opt, int32_t n_faults, const 
     ck(cudaMemsetAsync(A.lam, 0, blk * sizeof(double), L->st), "memset");
     ck(cudaMemsetAsync(A.grad, 0, (size_t)M * std::max(1, L->n_par) * sizeof(double), L->st), "memset");
     ck(cudaMemsetAsync(A.J, 0, M * sizeof(double), L->st), "memset");
-    DevClu Cs = L->C;
-    Cs.n_save = 1;
-    for (int v : L->cplan.rhs_base) Cs.n_save = std::max(Cs.n_save, v);
-    Cs.save_lu = CA.alloc<double>((size_t)M * std::max(1, Cs.n_tasks) * Cs.n_save * 32);
-    Cs.save_cc = CA.alloc<double>((size_t)M * std::max(1, L->P.n_cl) * 6);
+    Cs.save_lu = take(n_lu);
+    Cs.save_cc = take(M * n_cl * 6);
     for (int c = nck - 1; c >= 0; c--) {
         const int ka = c * K, kb = std::min(ns, ka + K);
-        // recompute the segment from its checkpoint, keeping every solve's state
-        ck(cudaMemcpyAsync(L->W.z, ckp + blk * c, blk * sizeof(double), cudaMemcpyDeviceToDevice, L->st), "restore");
-        launch_fault_status(L->P, L->d_fl_on_step, L->d_fl_off_step, L->d_fl_on, L->n_fl, ka, L->st);
-        for (int k = ka + 1; k <= kb; k++)
-            step(k, [&](int kind) {
-                ck(cudaMemcpyAsync(seg + blk * (2 * (k - ka - 1) + kind), L->W.z, blk * sizeof(double),
-                                   cudaMemcpyDeviceToDevice, L->st),
-                   "segment state");
-            });
+        if (!keep_all) {
+            // recompute the segment from its checkpoint, keeping every solve's state
+            ck(cudaMemcpyAsync(L->W.z, ckp + blk * c, blk * sizeof(double), cudaMemcpyDeviceToDevice, L->st),
+               "restore");
+            launch_fault_status(L->P, L->d_fl_on_step, L->d_fl_off_step, L->d_fl_on, L->n_fl, ka, L->st);
+            for (int k = ka + 1; k <= kb; k++) step(k, [&](int kind) { put_state(state_at(k, kind, ka)); });
+        }
         for (int k = kb; k > ka; k--) {
             if (ev.count(k)) {
                 // the dt = 0 re-solve after step k, for the scenarios that took it
-                ck(cudaMemcpyAsync(L->W.z, seg + blk * (2 * (k - ka - 1) + 1), blk * sizeof(double),
-                                   cudaMemcpyDeviceToDevice, L->st),
-                   "state");
                 ck(cudaMemcpyAsync(L->W.active, d_mask[k], M, cudaMemcpyDeviceToDevice, L->st), "mask");
                 launch_fault_status(L->P, L->d_fl_on_step, L->d_fl_off_step, L->d_fl_on, L->n_fl, k, L->st);
-                adj_solve(L, A, Cs, 0.0);
+                adj_solve(L, state_at(k, 1, ka), A, Cs, 0.0);
             }
             // the regular solve of step k: its state is trajectory point k
-            ck(cudaMemcpyAsync(L->W.z, seg + blk * (2 * (k - ka - 1)), blk * sizeof(double),
-                               cudaMemcpyDeviceToDevice, L->st),
-               "state");
             ck(cudaMemsetAsync(L->W.active, 1, M, L->st), "memset");
             launch_fault_status(L->P, L->d_fl_on_step, L->d_fl_off_step, L->d_fl_on, L->n_fl, k - 1, L->st);
-            launch_adj_objective(L->P, L->W, A, opt->dt, L->st);
-            adj_solve(L, A, Cs, opt->dt);
+            gp::DevWork Wk = L->W;
+            Wk.z = state_at(k, 0, ka);
+            launch_adj_objective(L->P, Wk, A, opt->dt, L->st);
+            adj_solve(L, Wk.z, A, Cs, opt->dt);
         }
     }
     ck(cudaMemcpyAsync(L->W.z, zfin, blk * sizeof(double), cudaMemcpyDeviceToDevice, L->st), "final state");
@@ -2891,6 +2926,10 @@ int32_t gp_adjoint(gp_layout *L, const gp_options *opt, int32_t n_faults, const 
     if (grad_p && L->n_par > 0)
         to_host(L, grad_p, A.grad, (size_t)M * L->n_par * sizeof(double), "grad copy");
     if (grad_z0) to_host(L, grad_z0, A.g, blk * sizeof(double), "grad z0 copy");
+    if (L->adj_bytes > kAdjKeep) {
+        L->adj_arena.release();
+        L->adj_bytes = 0;
+    }
     API_END
 }
 

@@ -334,11 +334,13 @@ typedef struct gp_objective {
 } gp_objective;
 
 /* Discrete adjoint of gp_integrate (FP64 Schur path), for every scenario:
- * integrates opt->n_steps steps forward from the current state, keeping the
- * state every checkpoint_every steps, then sweeps backwards, recomputing the
- * steps between checkpoints, with one transposed Newton-Jacobian solve per
- * forward solve (regular steps and dt = 0 event re-solves) at its converged
- * state and fault status.
+ * integrates opt->n_steps steps forward from the current state, then sweeps
+ * backwards with one transposed Newton-Jacobian solve per forward solve
+ * (regular steps and dt = 0 event re-solves) at its converged state and
+ * fault status.  The states of every solve are kept when they fit
+ * a quarter of the free device memory; else the state every
+ * checkpoint_every steps, and the sweep recomputes the steps between (the
+ * same values either way).
  *   J        [M] objective value
  *   grad_p   [M][n_par] dJ/dp at the fixed initial state: filled for the
  *            machine inertia H and damping D (GENROU/GENSAL), the exciter
