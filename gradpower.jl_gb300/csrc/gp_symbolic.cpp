@@ -4,8 +4,10 @@
 #include "gp_symbolic.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
 #include <cstring>
+#include <future>
 #include <queue>
 #include <stdexcept>
 
@@ -19,16 +21,17 @@ struct Graph {
 
 // Minimum-degree order of a small induced subgraph (|V| <= 64) using an
 // explicit elimination graph held in 64-bit masks.
-void leaf_min_degree(const Graph &G, const std::vector<int> &V, std::vector<int> &pos_in,
-                     std::vector<int> &order) {
+void leaf_min_degree(const Graph &G, const std::vector<int> &V, std::vector<int> &order) {
     const int k = (int)V.size();
-    for (int a = 0; a < k; a++) pos_in[V[a]] = a;
-    std::vector<uint64_t> m(k, 0);
+    std::vector<std::pair<int, int>> at(k);   // node -> place in V
+    for (int a = 0; a < k; a++) at[a] = {V[a], a};
+    std::sort(at.begin(), at.end());
+    uint64_t m[64] = {};
     for (int a = 0; a < k; a++) {
         int v = V[a];
         for (int q = G.ptr[v]; q < G.ptr[v + 1]; q++) {
-            int b = pos_in[G.adj[q]];
-            if (b >= 0 && b != a) m[a] |= (uint64_t)1 << b;
+            auto it = std::lower_bound(at.begin(), at.end(), std::make_pair(G.adj[q], 0));
+            if (it != at.end() && it->first == G.adj[q] && it->second != a) m[a] |= (uint64_t)1 << it->second;
         }
     }
     uint64_t alive = (k == 64) ? ~(uint64_t)0 : (((uint64_t)1 << k) - 1);
@@ -45,14 +48,25 @@ void leaf_min_degree(const Graph &G, const std::vector<int> &V, std::vector<int>
         alive &= ~((uint64_t)1 << best);
         order.push_back(V[best]);
     }
-    for (int a = 0; a < k; a++) pos_in[V[a]] = -1;
 }
 
+// Nested dissection.  The two halves of a large set are ordered by two
+// threads: a call touches its own set's entries of the arrays below and, of
+// set_id, reads its neighbours' (atomics: another call may be writing them;
+// no value but a node's own set's equals its id).  The order does not depend
+// on the threads.
 struct ND {
     const Graph &G;
-    std::vector<int> set_id, lev, pos_in;
-    std::vector<int> order;
-    int next_id = 1;
+    std::vector<std::atomic<int>> set_id;
+    std::vector<int> lev;
+    std::atomic<int> next_id{1};
+    // sets of at least PAR nodes give one half to another thread (analysis of
+    // 70,000 buses on eight cores 630 -> 295 ms, of 2,000 20 -> 10)
+    static constexpr int PAR = 200;
+    int set_of(int v) const { return set_id[v].load(std::memory_order_relaxed); }
+    void assign(const std::vector<int> &V, int id) {
+        for (int v : V) set_id[v].store(id, std::memory_order_relaxed);
+    }
     // sets of at most LEAF nodes are ordered by minimum degree as a whole;
     // separators and sets that do not split, in chunks of CHUNK.  LEAF 6
     // against 48: the tree of the 39-bus ring has 4 levels instead of 6, the
@@ -63,7 +77,9 @@ struct ND {
     static constexpr int LEAF = 6, CHUNK = 48;
 
     explicit ND(const Graph &g)
-        : G(g), set_id(g.n, 0), lev(g.n, -1), pos_in(g.n, -1), part(g.n, 0), stamp(g.n, 0) {}
+        : G(g), set_id(g.n), lev(g.n, -1), part(g.n, 0), stamp(g.n, 0) {
+        for (auto &s : set_id) s.store(0, std::memory_order_relaxed);
+    }
 
     // BFS inside the set `sid` from r; fills lev for visited nodes and
     // returns the visited nodes in BFS order.
@@ -75,7 +91,7 @@ struct ND {
             int u = visit[h];
             for (int q = G.ptr[u]; q < G.ptr[u + 1]; q++) {
                 int v = G.adj[q];
-                if (set_id[v] == sid && lev[v] < 0) {
+                if (set_of(v) == sid && lev[v] < 0) {
                     lev[v] = lev[u] + 1;
                     visit.push_back(v);
                 }
@@ -93,10 +109,9 @@ struct ND {
     // median level alone, unrefined (and leaves of 48), on the 70,000-bus
     // grid: largest front 132 -> 40 rows, factorisation flops 33.7 -> 19.4 M
     // a scenario, levels 30 -> 16; FP64 run of 8 scenarios x 18 steps 104 -> 58 ms (its
-    // factorisations 78 -> 36 ms), mixed (36 steps) 70 -> 56 ms; the analysis
-    // itself 0.39 -> 0.6 s.
+    // factorisations 78 -> 36 ms), mixed (36 steps) 70 -> 56 ms.
     std::vector<signed char> part;
-    void split(const std::vector<int> &V, int r, int sid, std::vector<int> &A, std::vector<int> &B,
+    void split(const std::vector<int> &V, int r, int sid, int &pass_id, std::vector<int> &A, std::vector<int> &B,
                std::vector<int> &S) {
         std::vector<int> visit, best;
         std::vector<signed char> best_part;
@@ -129,11 +144,11 @@ struct ND {
                     bool touches = false;
                     for (int q = G.ptr[v]; q < G.ptr[v + 1] && !touches; q++) {
                         const int u = G.adj[q];
-                        touches = set_id[u] == sid && lev[u] == l + 1;
+                        touches = set_of(u) == sid && lev[u] == l + 1;
                     }
                     part[v] = touches ? 2 : 0;
                 }
-                const double cost = refine(V, sid);
+                const double cost = refine(V, sid, pass_id);
                 if (cost < best_cost) {
                     best_cost = cost;
                     best_part.resize(V.size());
@@ -153,7 +168,7 @@ struct ND {
     // neighbours on the other side into the separator; the moves of a pass
     // are taken back to its best point.  Returns the separator's cost.
     std::vector<int> stamp;
-    double refine(const std::vector<int> &V, int sid) {
+    double refine(const std::vector<int> &V, int sid, int &pass_id) {
         const int n = (int)V.size();
         int w[3] = {0, 0, 0};
         for (int v : V) w[(int)part[v]]++;
@@ -164,7 +179,7 @@ struct ND {
         };
         auto pulls = [&](int v, int to) {
             int k = 0;
-            for (int q = G.ptr[v]; q < G.ptr[v + 1]; q++) k += set_id[G.adj[q]] == sid && part[G.adj[q]] == 1 - to;
+            for (int q = G.ptr[v]; q < G.ptr[v + 1]; q++) k += set_of(G.adj[q]) == sid && part[G.adj[q]] == 1 - to;
             return k;
         };
         double best = cost();
@@ -181,7 +196,7 @@ struct ND {
             size_t keep = 0;
             const double start = best;
             int since = 0;
-            while (!heap.empty() && since < 60) {
+            while (!heap.empty() && since < 20) {
                 const Item it = heap.top();
                 heap.pop();
                 const int v = it.second.first, to = it.second.second;
@@ -199,7 +214,7 @@ struct ND {
                 w[to]++;
                 for (int q = G.ptr[v]; q < G.ptr[v + 1]; q++) {
                     const int u = G.adj[q];
-                    if (set_id[u] != sid || part[u] != 1 - to) continue;
+                    if (set_of(u) != sid || part[u] != 1 - to) continue;
                     undo.push_back({u, (signed char)(1 - to)});
                     part[u] = 2;
                     w[1 - to]--;
@@ -209,7 +224,7 @@ struct ND {
                 // separator nodes beside v gained or lost a neighbour
                 for (int q = G.ptr[v]; q < G.ptr[v + 1]; q++) {
                     const int u = G.adj[q];
-                    if (set_id[u] == sid && part[u] == 2 && stamp[u] != pass_id) push(u);
+                    if (set_of(u) == sid && part[u] == 2 && stamp[u] != pass_id) push(u);
                 }
                 const double c = cost();
                 since++;
@@ -230,11 +245,11 @@ struct ND {
         }
         return best;
     }
-    int pass_id = 0;
-
-    void run(std::vector<int> V, int sid) {
+    // pass_id: refinement passes on the path to this set (a node's stamps
+    // are of earlier ones)
+    void run(std::vector<int> V, int sid, int pass_id, std::vector<int> &order) {
         if ((int)V.size() <= LEAF) {
-            leaf_min_degree(G, V, pos_in, order);
+            leaf_min_degree(G, V, order);
             return;
         }
         // connected components
@@ -252,8 +267,8 @@ struct ND {
             clear_lev(V);
             for (auto &c : comps) {
                 int id = next_id++;
-                for (int v : c) set_id[v] = id;
-                run(c, id);
+                assign(c, id);
+                run(c, id, pass_id, order);
             }
             return;
         }
@@ -270,13 +285,13 @@ struct ND {
             for (int i = (int)visit.size() - 1; i >= 0 && lev[visit[i]] == d; i--) {
                 int v = visit[i];
                 int dg = 0;
-                for (int q = G.ptr[v]; q < G.ptr[v + 1]; q++) dg += set_id[G.adj[q]] == sid;
+                for (int q = G.ptr[v]; q < G.ptr[v + 1]; q++) dg += set_of(G.adj[q]) == sid;
                 if (dg < bd) { bd = dg; best = v; }
             }
             r = best;
         }
         std::vector<int> A, B, S;
-        split(V, r, sid, A, B, S);
+        split(V, r, sid, pass_id, A, B, S);
         if (A.empty() || B.empty()) {
             // no useful split: order the whole set by minimum degree on its
             // own adjacency (ties in BFS order)
@@ -284,21 +299,29 @@ struct ND {
             while (!tmp.empty()) {
                 size_t take = std::min<size_t>(CHUNK, tmp.size());
                 std::vector<int> chunk(tmp.begin(), tmp.begin() + take);
-                leaf_min_degree(G, chunk, pos_in, order);
+                leaf_min_degree(G, chunk, order);
                 tmp.erase(tmp.begin(), tmp.begin() + take);
             }
             return;
         }
         int ida = next_id++, idb = next_id++, ids = next_id++;
-        for (int v : A) set_id[v] = ida;
-        for (int v : B) set_id[v] = idb;
-        for (int v : S) set_id[v] = ids;
-        run(A, ida);
-        run(B, idb);
+        assign(A, ida);
+        assign(B, idb);
+        assign(S, ids);
+        if ((int)V.size() >= PAR) {
+            std::vector<int> ob;
+            auto half = std::async(std::launch::async, [&] { run(B, idb, pass_id, ob); });
+            run(A, ida, pass_id, order);
+            half.get();
+            order.insert(order.end(), ob.begin(), ob.end());
+        } else {
+            run(A, ida, pass_id, order);
+            run(B, idb, pass_id, order);
+        }
         // separator nodes: order them by minimum degree in chunks
         for (size_t a = 0; a < S.size(); a += CHUNK) {
             std::vector<int> chunk(S.begin() + a, S.begin() + std::min(S.size(), a + CHUNK));
-            leaf_min_degree(G, chunk, pos_in, order);
+            leaf_min_degree(G, chunk, order);
         }
     }
 };
@@ -344,19 +367,20 @@ void analyse(int n, const std::vector<int> &rowptr, const std::vector<int> &coli
     }
     // ---- nested dissection on nodes ----
     ND nd(G);
+    std::vector<int> node_order;
     {
         std::vector<int> all(n_nodes);
         for (int a = 0; a < n_nodes; a++) all[a] = a;
-        nd.run(all, 0);
+        nd.run(all, 0, 0, node_order);
     }
-    if ((int)nd.order.size() != n_nodes) throw std::runtime_error("nested dissection lost nodes");
+    if ((int)node_order.size() != n_nodes) throw std::runtime_error("nested dissection lost nodes");
     // ---- expand to scalar unknowns ----
     std::vector<std::vector<int>> members(n_nodes);
     for (int i = 0; i < n; i++) members[group[i]].push_back(i);
     S.n = n;
     S.perm.clear();
     S.perm.reserve(n);
-    for (int a : nd.order)
+    for (int a : node_order)
         for (int i : members[a]) S.perm.push_back(i);
     if ((int)S.perm.size() != n) throw std::runtime_error("unknowns without a node");
     // ---- elimination tree of the dissection's order, then of its postorder
