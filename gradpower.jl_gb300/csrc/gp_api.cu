@@ -1107,11 +1107,12 @@ void host_block_solve(const gp::Symbolic &S, const HostBlk &B, const std::vector
 
 // The dataflow schedule (host side): the topological order of the
 // factorisation tasks (by region: subtrees whose fronts have at most
-// dag_tiny_front() and 32 rows, and the rest; by level within a region)
+// dag_mini_front(), dag_little_front(), dag_tiny_front() and 32 rows, and
+// the rest; by level within a region)
 // and the split of the tail's large FP64 fronts into parts.
 struct DagPlan {
     std::vector<int> order, rank, submax;
-    int n_tiny = 0, n_small = 0, max_big = 0, max_big_whole = 0;
+    int n_mini = 0, n_little = 0, n_tiny = 0, n_small = 0, max_big = 0, max_big_whole = 0;
     int tail0 = 0;
     std::vector<uint8_t> nparts;
     std::vector<int> tail_units{0};
@@ -1130,26 +1131,29 @@ void make_dag_plan(const gp::Symbolic &sym, DagPlan &dp) {
             for (int c = sym.child_ptr[s]; c < sym.child_ptr[s + 1]; c++) mx = std::max(mx, dp.submax[sym.children[c]]);
             dp.submax[s] = mx;
         }
-    const int tiny = gp::dag_tiny_front();
+    const int lim[] = {gp::dag_mini_front(), gp::dag_little_front(), gp::dag_tiny_front(), 32};
     dp.order.clear();
     dp.rank.assign(ns, 0);
     auto region = [&](int s) {
-        const int m = dp.submax[s];
-        return m <= tiny ? 0 : (m <= 32 ? 1 : 2);
+        int r = 0;
+        while (r < 4 && dp.submax[s] > lim[r]) r++;
+        return r;
     };
-    for (int pass = 0; pass < 3; pass++)
+    for (int pass = 0; pass < 5; pass++)
         for (int l = 0; l < sym.nlevels; l++)
             for (int q = sym.level_ptr[l]; q < sym.level_ptr[l + 1]; q++) {
                 const int s = sym.level_sups[q];
                 if (region(s) != pass) continue;
                 dp.rank[s] = (int)dp.order.size();
                 dp.order.push_back(s);
-                if (pass == 2) dp.max_big = std::max(dp.max_big, sym.front_m(s));
+                if (pass == 4) dp.max_big = std::max(dp.max_big, sym.front_m(s));
             }
-    dp.n_tiny = dp.n_small = 0;
+    dp.n_mini = dp.n_little = dp.n_tiny = dp.n_small = 0;
     for (int s = 0; s < ns; s++) {
-        dp.n_tiny += region(s) == 0;
-        dp.n_small += region(s) <= 1;
+        dp.n_mini += region(s) == 0;
+        dp.n_little += region(s) <= 1;
+        dp.n_tiny += region(s) <= 2;
+        dp.n_small += region(s) <= 3;
     }
     // split fronts (FP64): in the last kSplitTail ranks of the order (the
     // narrow top of the tree), a front of at least kSplitMin rows is factored
@@ -1188,6 +1192,8 @@ void build_dag(gp_layout *L, const gp::Symbolic &sym) {
     const int lim = gp::dag_tiny_front();
     gp::DevDag &D = L->D;
     D.nsup = ns;
+    D.n_mini = dp.n_mini;
+    D.n_little = dp.n_little;
     D.n_tiny = dp.n_tiny;
     D.n_small = dp.n_small;
     D.max_front = sym.max_front;
@@ -1763,7 +1769,7 @@ void mark(gp_layout *L, int i) {
 // own factors), and the update.
 int enqueue_solve(gp_layout *L, int variant, int *nfac_out) {
     const gp::DevDag &D = L->D;
-    const int nfac = gp::dag_factor_launches(D, 1), nfac64 = gp::dag_factor_launches(D, 0);
+    const int nfac = gp::dag_factor_launches(D, L->M, 1), nfac64 = gp::dag_factor_launches(D, L->M, 0);
     const gp::DevBlk &B = L->B;
     const int nsolve = (B.nblk + B.n_top) > 0;   // one fused kernel per direction
     int launches = 2, facs = 0;   // dag_begin, update
@@ -2022,7 +2028,7 @@ void wb_prepare(gp_layout *L, double dt) {
     }
     gp::launch_wb_setup(L->P, L->wb_W1, L->wb_W2, L->wb_Hinv, L->st);
     {
-        const int nfac = gp::dag_factor_launches(L->D, 0);
+        const int nfac = gp::dag_factor_launches(L->D, L->M, 0);
         L->launches += 14 + nfac;
         L->factor_launches += nfac;
     }

@@ -14,9 +14,8 @@
 // at once, and the kernel finishes with the scenario marked in `status`.
 //
 // Factorisation, in two launches (three for FP64):
-//  - factor_group_kernel (FP64 only): supernodes whose whole subtree has
-//    fronts of at most kTinyFront rows, 32 / kTinyLanes scenarios a warp
-//    (kTinyLanes lanes per front);
+//  - factor_tiny_kernel (FP64): supernodes whose whole subtree has fronts of
+//    at most kTinyFront rows, four or two scenarios a warp;
 //  - factor_small_kernel: supernodes whose whole subtree has fronts of at
 //    most 32 rows, one warp per task, the front in shared memory;
 //  - factor_big_kernel: the rest, one CTA per task.
@@ -39,6 +38,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "gp_internal.h"
 #include "gp_warp.cuh"
@@ -50,21 +50,13 @@ namespace {
 constexpr unsigned FULL = kFullMask;
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
-// FP64 factorisations run the subtrees whose fronts have at most
-// kTinyFront rows first, in a launch of their own with a smaller front
-// buffer: more fronts in flight, where the 32-row buffers hold an SM to 24
-// (factorisation 693 -> 670 ms per FP64 run), and several fronts a warp
-// (factor_group_kernel).  FP32 ones keep one launch: their 32-row buffers
-// already allow 48 warps, and the launch boundary would cost the overlap of
-// the two regions (74 -> 81 ms per mixed run).
-constexpr int kSmallFront = 32;
-constexpr int kTinyFront = 20;
-// lanes a tiny front gets in factor_group_kernel (32 / kTinyLanes fronts a
-// warp).  16: two fronts a warp.  8 (four fronts a warp, a quarter fewer
-// FP64 instructions by count) measured slower: the same shared memory then
-// holds half the warps, and the kernel also waits on its loads (FP64
-// factorisation 141.2 -> 144.7 ms over 0.3 s of the 70k-bus workload).
-constexpr int kTinyLanes = 16;
+constexpr int kSmallFront = 32;   // rows a warp of factor_small_kernel has room for
+// FP64 factorisations run the subtrees whose fronts have at most kTinyFront
+// rows first, in a launch of their own with smaller front buffers (more
+// fronts in flight) and several scenarios a warp (factor_tiny_kernel).  FP32
+// ones keep one launch: their 32-row buffers already allow 48 warps, and the
+// launch boundary would cost the overlap of the two regions.
+constexpr int kMiniFront = 8, kLittleFront = 14, kTinyFront = 20;
 // update-matrix entries a thread loads ahead in the extend-add: none in the
 // warp kernel, which runs at 40 registers a thread and many warps a SM
 template <class G>
@@ -149,7 +141,7 @@ __device__ __forceinline__ unsigned key_lo(double v) { return (unsigned)__double
 // whole warp calls it).  A whole warp takes the maximum by integer
 // reductions of the key's words (25 cycles each on GB300, a 64-bit shuffle
 // 38); segments by shuffles (reductions over half a warp run one half after
-// the other: factor_group_kernel 403 -> 420 us on 70,000 buses x 8).
+// the other: an FP64 kernel of two fronts a warp 403 -> 420 us on 70,000 buses x 8).
 template <class T, int LW = 32>
 __device__ __forceinline__ int warp_pivot(const T *F, int mm, int k, int ns, bool &zero) {
     using K = typename KeyOf<T>::type;
@@ -200,8 +192,9 @@ struct WarpGroup {
     __device__ bool active() const { return true; }
     __device__ void sync() const { __syncwarp(); }
 };
+template <int N>
 struct BlockGroup {
-    static constexpr int size = kThreads, lanes = 32;
+    static constexpr int size = N, lanes = 32;
     __device__ int idx() const { return threadIdx.x; }
     __device__ int lane() const { return threadIdx.x & 31; }
     __device__ bool lead_warp() const { return threadIdx.x < 32; }
@@ -1061,6 +1054,143 @@ __host__ __device__ inline int big_front_bytes(int max_front) {
     return (max_front * (max_front + 1) * (int)sizeof(T) + 15) & ~15;
 }
 
+// ---- tiny fronts: a lane a row ----------------------------------------------
+// One front of at most LW rows by LW lanes, 32 / LW scenarios of the same
+// supernode a warp (group g of the warp on its own scenario; the whole warp
+// calls it).  Lane i holds row i of a column step.  The FP64 pipe charges a
+// warp instruction the same whatever its active lanes, so the scenarios of a
+// warp share every instruction's time; and a column's chain is short: the
+// pivot search by shuffles beside the reciprocal of every candidate, the
+// multiplier, the next column's update, which stays in a register for the
+// next search.  Rows stay in place (pos: the place a row has in the
+// eliminated order, exchanged as the other kernels exchange rows) and are
+// put in order as they are stored.  Every entry receives the operations of
+// factor_front.
+template <int LW, class Wait, class Done>
+__device__ void factor_rows(const DevProblem &P, const DevWork &W, const DevSym &S, double *fronts, double *lfac,
+                            double *ufac, int s, int m, bool act, double *F, Wait wait, Done done) {
+    const int lane = threadIdx.x & (LW - 1);
+    const int start = S.sup_start[s];
+    const int ns = S.sup_start[s + 1] - start;
+    const int mm = ns + S.row_ptr[s + 1] - S.row_ptr[s], nc = mm + 1;
+    double *fr = fronts + (size_t)m * S.front_total;
+    double *x = W.xperm + (size_t)m * P.n_red;
+    double *uv = S.uvec + (size_t)m * S.uvec_total;
+    const bool row = lane < mm;
+    // ---- the front's own entries ----
+    const double xr = lane < ns ? x[start + lane] : 0.0;
+    for (int j = 0; j < mm; j++)
+        if (row) F[lane + j * mm] = 0.0;
+    if (row) F[lane + mm * mm] = xr;
+    __syncwarp();
+    for (int e = S.asmc_ptr[s] + lane; e < S.asmc_ptr[s + 1]; e += LW) F[S.asmc_pos[e]] += S.asmc_val[e];
+    __syncwarp();
+    const double *sv = W.svar + (size_t)m * P.n_var;
+    for (int e = S.asmv_ptr[s] + lane; e < S.asmv_ptr[s + 1]; e += LW) F[S.asmv_pos[e]] += sv[S.asmv_idx[e]];
+    if (S.asmt_ptr)
+        for (int e = S.asmt_ptr[s] + lane; e < S.asmt_ptr[s + 1]; e += LW) {
+            const int t = S.asmt_tr[e];
+            if (P.tr_on[t] && t >= P.tr_ptr[m] && t < P.tr_ptr[m + 1]) F[S.asmt_pos[e]] += S.asmt_val[e];
+        }
+    __syncwarp();
+    wait();   // for the children (bounded); ends with a warp barrier
+    // ---- the children's update matrices and vectors, in child order ----
+    for (int q = S.child_ptr[s]; q < S.child_ptr[s + 1]; q++) {
+        const int c = S.children[q];
+        const int ncc = S.sup_start[c + 1] - S.sup_start[c], rc = S.row_ptr[c + 1] - S.row_ptr[c], mc = ncc + rc;
+        const int *rel = S.relmap + S.relmap_ptr[c];
+        const double *Fc = fr + S.front_off[c] + (size_t)ncc * mc + ncc, *uc = uv + S.uvec_off[c];
+        const int ra = lane < rc ? rel[lane] : 0;
+        // lane a on row a of the update matrix (rc < LW); four columns' loads
+        // together
+        for (int b0 = 0; b0 <= rc; b0 += 4) {
+            double v[4];
+            int rb[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int b = b0 + u;
+                const bool in = lane < rc && b <= rc;
+                v[u] = in ? __ldcg(b < rc ? Fc + lane + (size_t)b * mc : uc + lane) : 0.0;
+                rb[u] = in && b < rc ? rel[b] : mm;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (lane < rc && b0 + u <= rc) F[ra + rb[u] * mm] += v[u];
+        }
+        __syncwarp();
+    }
+    // ---- elimination ----
+    int pos = lane;
+    double v = row ? F[lane] : 0.0;
+    for (int k = 0; k < ns; k++) {
+        const bool cand = pos >= k && pos < ns;
+        const double own = cand ? v : 1.0;
+        const bool special = recip_special(own);
+        const double rown = recip_normal(special ? 1.0 : own);
+        unsigned kh = cand ? key_hi(v) : 0u, kl = cand ? key_lo(v) : 0u;
+        unsigned pk = cand ? (unsigned)(pos * 32 + lane) : 0xffffffffu;   // (the smallest place on ties)
+#pragma unroll
+        for (int off = LW / 2; off > 0; off >>= 1) {
+            const unsigned oh = __shfl_xor_sync(FULL, kh, off, LW), ol = __shfl_xor_sync(FULL, kl, off, LW),
+                           op = __shfl_xor_sync(FULL, pk, off, LW);
+            const bool take = oh > kh || (oh == kh && (ol > kl || (ol == kl && op < pk)));
+            if (take) { kh = oh; kl = ol; pk = op; }
+        }
+        const int pv = (int)(pk >> 5), pl = (int)(pk & 31u);
+        if (lane == 0 && act && (kh | kl) == 0u) atomicOr(W.status + m, 4);
+        double inv = __shfl_sync(FULL, rown, pl, LW);
+        const bool sp = __shfl_sync(FULL, (int)special, pl, LW) != 0;
+        if (__any_sync(FULL, sp)) {
+            const double d = __shfl_sync(FULL, own, pl, LW);
+            if (sp) inv = 1.0 / d;
+        }
+        if (lane == pl) pos = k;
+        else if (pos == k) pos = pv;
+        const bool upd = row && pos > k;
+        const double l = v * inv;
+        if (upd || lane == pl) F[lane + k * mm] = upd ? l : inv;
+        {
+            const double u = F[pl + (k + 1) * mm];
+            v = row ? F[lane + (k + 1) * mm] : 0.0;
+            if (upd) {
+                v -= l * u;
+                F[lane + (k + 1) * mm] = v;
+            }
+        }
+#pragma unroll 4
+        for (int j = k + 2; j < nc; j++) {
+            const double u = F[pl + j * mm];
+            if (upd) F[lane + j * mm] -= l * u;
+        }
+        __syncwarp();
+    }
+    // ---- store: what the parent reads and the forward-solved entries, then
+    // done(), then the solve-ordered copies and the composed pivots ----
+    if (act && row) {
+        if (lane >= ns) {
+            double *out = fr + S.front_off[s];
+            for (int j = ns; j < mm; j++) out[lane + (size_t)j * mm] = F[lane + j * mm];
+            uv[S.uvec_off[s] + lane - ns] = F[lane + mm * mm];
+        } else {
+            x[start + pos] = F[lane + mm * mm];
+        }
+    }
+    __syncwarp();
+    done();
+    if (act && row) {
+        if (lfac) {
+            double *lo = lfac + (size_t)m * S.lu_total + S.lu_off[s];
+            for (int j = 0; j < ns; j++) lo[pos + (size_t)j * mm] = F[lane + j * mm];
+        }
+        if (lane < ns) {
+            double *uo = ufac + (size_t)m * S.lu_total + S.lu_off[s];
+            for (int j = 0; j < mm; j++) uo[pos + (size_t)j * ns] = F[lane + j * mm];
+            S.ipiv[(size_t)m * S.n + start + pos] = lane;
+        }
+    }
+    __syncwarp();
+}
+
 // ---- middle fronts: registers --------------------------------------------
 // Fronts above the tiny region's, up to 32 rows, four warps a front: the
 // warps take the columns in turn (column warp + 4 c), the lanes the rows,
@@ -1087,6 +1217,7 @@ constexpr int kMidThreads = 128, kMidWarps = 4;
 // us against 395, 2,000 x 64 (1,344) 144 against 108, 9,001 x 3 (261) 145
 // against 81.
 constexpr long long kMidTasks = 3000;
+constexpr int kWideFront = 64;
 
 template <class T>
 struct MidShape {
@@ -1247,15 +1378,20 @@ __device__ void factor_mid(const DevProblem &P, const DevWork &W, const DevSym &
     if (warp == 0 && lane < ns) S.ipiv[(size_t)m * S.n + start + rpos] = lane;
 }
 
-// Ranks [r0, r1) of the order, one CTA per front; tasks claimed from counter
-// ctr.  The ranks below `from` were factored by earlier launches.
-template <class T, bool RHS>
-__global__ void __launch_bounds__(kMidThreads, 6) factor_mid_kernel(
-    DevProblem P, DevWork W, DevSym S, DevDag D, T *fronts, T *lfac, T *ufac, const uint8_t *mask, int want, int r0,
-    int r1, int ctr) {
+// Ranks [r0, nsup) of the order, one CTA per front: fronts of at most 32 rows
+// in registers (factor_mid), larger ones (WIDE) in shared memory, column by
+// column over the CTA.  The ranks below r0 were factored by earlier launches.
+// With WIDE the fronts above 32 rows and the small ones above them in the
+// tree share one launch with what lies below (FP64 factorisation of 9,001
+// buses x 3 @U@).
+template <bool WIDE>
+__global__ void __launch_bounds__(kMidThreads, 6) factor_mid_kernel(DevProblem P, DevWork W, DevSym S, DevDag D,
+                                                                    double *fronts, double *lfac, double *ufac,
+                                                                    const uint8_t *mask, int want, int r0, int r1,
+                                                                    int ctr) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    T *F = reinterpret_cast<T *>(smem_raw);
-    T *colbuf = reinterpret_cast<T *>(smem_raw + MidShape<T>::front_bytes);
+    double *F = reinterpret_cast<double *>(smem_raw);
+    double *colbuf = reinterpret_cast<double *>(smem_raw + MidShape<double>::front_bytes);
     __shared__ int s_task, s_ok;
     const int tid = threadIdx.x, lane = tid & 31;
     const int M = P.M;
@@ -1280,7 +1416,16 @@ __global__ void __launch_bounds__(kMidThreads, 6) factor_mid_kernel(
         auto done = [&] {
             if (tid == 0) signal_done(D.fdone + (size_t)s * M + m, epoch);
         };
-        factor_mid<T, RHS>(P, W, S, fronts, lfac, ufac, s, m, F, colbuf, wait, done);
+        if constexpr (WIDE) {
+            const int mm = S.sup_start[s + 1] - S.sup_start[s] + S.row_ptr[s + 1] - S.row_ptr[s];
+            if (mm > MidShape<double>::rows) {
+                int *piv = reinterpret_cast<int *>(smem_raw + ((mm * (mm + 1) * 8 + 15) & ~15));
+                factor_front<double, true>(P, W, S, fronts, lfac, ufac, s, m, F, piv, BlockGroup<kMidThreads>{}, wait,
+                                           done);
+                continue;
+            }
+        }
+        factor_mid<double, true>(P, W, S, fronts, lfac, ufac, s, m, F, colbuf, wait, done);
     }
 }
 
@@ -1316,57 +1461,100 @@ __global__ void __launch_bounds__(kThreads, 6) factor_small_kernel(DevProblem P,
     }
 }
 
-// Ranks [r0, r1) of the order, G = 32 / W scenarios a warp: a task is a
-// (supernode, group of G scenarios), and each W-lane group of the warp
-// factors the front of one of them (fronts of at most cap rows, a buffer per
-// group).  The fronts belong to the same supernode, so the groups run the
-// same loops, and each instruction of a pivot column's steps (pivot search,
-// reciprocal, multipliers) serves G fronts.  The FP64 elimination of small
-// fronts is bound by the FP64 pipe, which charges a warp instruction the
-// same whatever its active lanes, and these steps, one per column whatever
-// the front's size, would otherwise occupy it once per front.  A group
-// whose scenario this launch does not factor (M not a multiple of G, or
-// masked out) follows the task's first factored scenario and stores
-// nothing.
-template <class T, bool RHS, int W>
-__global__ void __launch_bounds__(kThreads, W == 16 ? 4 : 2) factor_group_kernel(DevProblem P, DevWork W_, DevSym S, DevDag D,
-                                                                T *fronts, T *lfac, T *ufac, const uint8_t *mask,
-                                                                int want, int r0, int r1, int cap, int ctr) {
-    constexpr int G = 32 / W;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gi = lane / W;
-    unsigned char *gbase = smem_raw + (size_t)(G * warp + gi) * warp_area_bytes<T>(cap);
-    T *F = reinterpret_cast<T *>(gbase);
-    int *piv = reinterpret_cast<int *>(gbase + warp_front_bytes<T>(cap));
-    const int M = P.M, Mg = (M + G - 1) / G;
-    const int epoch = *D.epoch;
-    const int n_tasks = (r1 - r0) * Mg;
-    for (;;) {
-        int t = 0;
-        if (lane == 0) t = atomicAdd(D.ctr + ctr, 1);
-        t = __shfl_sync(FULL, t, 0);
-        if (t >= n_tasks) break;
-        const int s = D.order[r0 + t / Mg], m0 = G * (t % Mg);
-        int first = -1;
-        bool act = false;
+// The fronts of at most kTinyFront rows (ranks below n_tiny), several
+// scenarios a warp: a task is a (supernode, group of scenarios), and each
+// group of lanes factors one of them.  A group whose scenario this launch
+// does not factor (M not a multiple, or masked out) follows the task's first
+// factored scenario and stores nothing.
+//  - the mini region (fronts of at most kMiniFront rows, two thirds of the
+//    supernodes): four scenarios a warp, a lane a row (factor_rows);
+//  - the rest, up to kLittleFront rows four, above two scenarios a warp
+//    (factor_front: its flattened updates waste fewer lanes from about ten
+//    rows on; a lane a row for 9 to 16 rows measured 339 us against about
+//    300).
+// The groups belong to the same supernode, so they run the same loops, and
+// each instruction of a pivot column's steps (pivot search, reciprocal,
+// multipliers) serves all of them: the FP64 pipe, which bounds the kernel,
+// charges a warp instruction the same whatever its active lanes.
+// Measured (70,000 buses x 8): two scenarios a warp for both 360 us -> @T@.
+struct TaskGroup {
+    int s, m;      // supernode, the lane group's scenario
+    bool act;      // factored by this launch
+};
+template <int LW>
+__device__ bool claim_group(const DevDag &D, const uint8_t *mask, int want, int M, int r0, int r1, int ctr,
+                            TaskGroup &g, bool &more) {
+    constexpr int G = 32 / LW;
+    const int lane = threadIdx.x & 31, gi = lane / LW, Mg = (M + G - 1) / G;
+    int t = 0;
+    if (lane == 0) t = atomicAdd(D.ctr + ctr, 1);
+    t = __shfl_sync(FULL, t, 0);
+    more = t < (r1 - r0) * Mg;
+    if (!more) return false;
+    g.s = D.order[r0 + t / Mg];
+    const int m0 = G * (t % Mg);
+    int first = -1;
+    g.act = false;
 #pragma unroll
-        for (int g = 0; g < G; g++) {
-            const bool v = m0 + g < M && mask[m0 + g] == want;
-            if (v && first < 0) first = m0 + g;
-            if (g == gi) act = v;
-        }
-        if (first < 0) continue;
-        const int m = act ? m0 + gi : first;
-        factor_front<T, RHS>(
-            P, W_, S, fronts, lfac, ufac, s, m, F, piv, LaneGroup<W>{act},
+    for (int q = 0; q < G; q++) {
+        const bool v = m0 + q < M && mask[m0 + q] == want;
+        if (v && first < 0) first = m0 + q;
+        if (q == gi) g.act = v;
+    }
+    g.m = g.act ? m0 + gi : first;
+    return first >= 0;
+}
+
+// shared memory of a warp: four fronts of kLittleFront rows or two of kTinyFront
+constexpr int kTinyArea = 4 * warp_area_bytes<double>(kLittleFront) > 2 * warp_area_bytes<double>(kTinyFront)
+                              ? 4 * warp_area_bytes<double>(kLittleFront)
+                              : 2 * warp_area_bytes<double>(kTinyFront);
+
+__global__ void __launch_bounds__(kThreads, 4) factor_tiny_kernel(DevProblem P, DevWork W, DevSym S, DevDag D,
+                                                                  double *fronts, double *lfac, double *ufac,
+                                                                  const uint8_t *mask, int want) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned char *wbase = smem_raw + (size_t)warp * kTinyArea;
+    const int M = P.M, epoch = *D.epoch;
+    TaskGroup g;
+    bool more = true;
+    while (more) {
+        if (!claim_group<8>(D, mask, want, M, 0, D.n_mini, 7, g, more)) continue;
+        factor_rows<8>(
+            P, W, S, fronts, lfac, ufac, g.s, g.m, g.act,
+            reinterpret_cast<double *>(wbase) + (lane / 8) * kMiniFront * (kMiniFront + 1),
             [&] {
-                if (!group_wait_children<W>(S, D, D.fdone, s, m, M, epoch) && (lane & (W - 1)) == 0 && act)
-                    atomicOr(W_.status + m, 8);
+                if (!group_wait_children<8>(S, D, D.fdone, g.s, g.m, M, epoch) && (lane & 7) == 0 && g.act)
+                    atomicOr(W.status + g.m, 8);
             },
             [&] {
-                if ((lane & (W - 1)) == 0 && act) signal_done(D.fdone + (size_t)s * M + m, epoch);
+                if ((lane & 7) == 0 && g.act) signal_done(D.fdone + (size_t)g.s * M + g.m, epoch);
             });
     }
+    // (wider fronts: LW lanes each, the updates flattened over them)
+    auto rest = [&](auto width, int cap, int r0, int r1, int ctr) {
+        constexpr int LW = decltype(width)::value;
+        unsigned char *gbase = wbase + (size_t)(lane / LW) * warp_area_bytes<double>(cap);
+        double *F = reinterpret_cast<double *>(gbase);
+        int *piv = reinterpret_cast<int *>(gbase + warp_front_bytes<double>(cap));
+        bool more = true;
+        while (more) {
+            if (!claim_group<LW>(D, mask, want, M, r0, r1, ctr, g, more)) continue;
+            factor_front<double, true>(
+                P, W, S, fronts, lfac, ufac, g.s, g.m, F, piv, LaneGroup<LW>{g.act},
+                [&] {
+                    if (!group_wait_children<LW>(S, D, D.fdone, g.s, g.m, M, epoch) && (lane & (LW - 1)) == 0 &&
+                        g.act)
+                        atomicOr(W.status + g.m, 8);
+                },
+                [&] {
+                    if ((lane & (LW - 1)) == 0 && g.act) signal_done(D.fdone + (size_t)g.s * M + g.m, epoch);
+                });
+        }
+    };
+    rest(std::integral_constant<int, 8>(), kLittleFront, D.n_mini, D.n_little, 8);
+    rest(std::integral_constant<int, 16>(), kTinyFront, D.n_little, D.n_tiny, 9);
 }
 
 template <class T, bool RHS>
@@ -1430,7 +1618,7 @@ __global__ void __launch_bounds__(kThreads, 3) factor_big_kernel(DevProblem P, D
             if (!s_ok && tid == 0) atomicOr(W.status + m, 8);
         };
         if (np == 1) {
-            factor_front<T, RHS>(P, W, S, fronts, lfac, ufac, s, m, F, piv, BlockGroup{}, wait, [&] {
+            factor_front<T, RHS>(P, W, S, fronts, lfac, ufac, s, m, F, piv, BlockGroup<kThreads>{}, wait, [&] {
                 if (tid == 0) signal_done(D.fdone + (size_t)s * M + m, epoch);
             });
         } else if constexpr (kSplit) {
@@ -1472,20 +1660,22 @@ int configure_one(DagGrid &g, int nsm, int tiny_bytes, int small_bytes, int big_
         return -1;
     g.small = nsm * occ;
     if constexpr (sizeof(T) == 8) {
-        // the tiny fronts: two scenarios a warp
-        if (cudaFuncSetAttribute(factor_group_kernel<T, R, kTinyLanes>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 tiny_bytes) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, factor_group_kernel<T, R, kTinyLanes>, kThreads,
-                                                          tiny_bytes) !=
+        if (cudaFuncSetAttribute(factor_tiny_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tiny_bytes) !=
+                cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, factor_tiny_kernel, kThreads, tiny_bytes) !=
                 cudaSuccess || occ < 1)
             return -1;
         g.tiny = nsm * occ;
-        if (cudaFuncSetAttribute(factor_mid_kernel<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 MidShape<T>::bytes) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, factor_mid_kernel<T, R>, kMidThreads,
+        if (!raise_shared_limit(factor_mid_kernel<false>, MidShape<T>::bytes) ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, factor_mid_kernel<false>, kMidThreads,
                                                           MidShape<T>::bytes) != cudaSuccess || occ < 1)
             return -1;
         g.mid = nsm * occ;
+        if (!raise_shared_limit(factor_mid_kernel<true>, g.wide_bytes) ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, factor_mid_kernel<true>, kMidThreads, g.wide_bytes) !=
+                cudaSuccess || occ < 1)
+            return -1;
+        g.wide = nsm * occ;
     }
     if (cudaFuncSetAttribute(factor_big_kernel<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, big_bytes) !=
             cudaSuccess ||
@@ -1511,10 +1701,13 @@ int dag_configure(const DevDag &D, int fp32, DagGrid &g) {
     // not split whole, and the parts of the split ones
     const int mb = std::max(1, fp32 ? D.max_big_front : D.max_big_whole);
     const int small_bytes = kWarps * (fp32 ? warp_area_bytes<float>(kSmallFront) : warp_area_bytes<double>(kSmallFront));
-    const int tiny_bytes = fp32 ? 0 : (32 / kTinyLanes) * kWarps * warp_area_bytes<double>(kTinyFront);
+    const int tiny_bytes = fp32 ? 0 : kWarps * kTinyArea;
     const int whole = (fp32 ? big_front_bytes<float>(mb) : big_front_bytes<double>(mb)) + 2 * mb * 4;
     const int part = fp32 ? 0 : ((D.max_part_entries * 8 + 15) & ~15) + D.max_part_ints * 4;
     const int big_bytes = std::max(whole, part);
+    // (up to 64 rows the fronts need no split and leave room for several CTAs)
+    const int mw = D.max_front <= kWideFront ? std::max(MidShape<double>::rows, D.max_front) : MidShape<double>::rows;
+    g.wide_bytes = std::max(MidShape<double>::bytes, big_front_bytes<double>(mw) + 2 * mw * 4);
     const int rc = fp32 ? configure_one<float>(g, nsm, tiny_bytes, small_bytes, big_bytes)
                         : configure_one<double>(g, nsm, tiny_bytes, small_bytes, big_bytes);
     if (rc != 0) {
@@ -1527,10 +1720,14 @@ int dag_configure(const DevDag &D, int fp32, DagGrid &g) {
     return 0;
 }
 
-int dag_factor_launches(const DevDag &D, int fp32) {
+int dag_factor_launches(const DevDag &D, int M, int fp32) {
     if (fp32) return (D.n_small > 0) + (D.nsup > D.n_small);
+    const bool one = (long long)(D.n_small - D.n_tiny) * M <= kMidTasks && D.max_front <= kWideFront;
+    if (one) return (D.n_tiny > 0) + (D.nsup > D.n_tiny);
     return (D.n_tiny > 0) + (D.n_small > D.n_tiny) + (D.nsup > D.n_small);
 }
+int dag_mini_front() { return kMiniFront; }
+int dag_little_front() { return kLittleFront; }
 int dag_tiny_front() { return kTinyFront; }
 
 void launch_dag_begin(const DevDag &D, cudaStream_t st) { dag_begin_kernel<<<1, 32, 0, st>>>(D); }
@@ -1551,19 +1748,28 @@ void launch_dag_factor(const DevProblem &P, const DevWork &W, const DevSym &S, c
                        T *fronts, T *lfac, T *ufac, const uint8_t *mask, int want, cudaStream_t st) {
     constexpr bool R = FusedRhs<T>::value;
     if constexpr (sizeof(T) == 8) {
-        constexpr int G = 32 / kTinyLanes;
-        const long long tt = (long long)D.n_tiny * ((P.M + G - 1) / G), ts = (long long)(D.n_small - D.n_tiny) * P.M,
-                        tb = (long long)D.big_units * P.M;
+        const long long tt = std::max((long long)D.n_little * ((P.M + 3) / 4),
+                                      (long long)(D.n_tiny - D.n_little) * ((P.M + 1) / 2)),
+                        ts = (long long)(D.n_small - D.n_tiny) * P.M, tb = (long long)D.big_units * P.M;
         if (tt > 0)
-            factor_group_kernel<T, R, kTinyLanes><<<blocks_for(g.tiny, tt, kWarps), kThreads, g.tiny_bytes, st>>>(
-                P, W, S, D, fronts, lfac, ufac, mask, want, 0, D.n_tiny, kTinyFront, 7);
+            factor_tiny_kernel<<<blocks_for(g.tiny, tt, kWarps), kThreads, g.tiny_bytes, st>>>(P, W, S, D, fronts, lfac,
+                                                                                               ufac, mask, want);
+        const bool wide = D.max_front <= kWideFront;
+        const long long tw = (long long)(D.nsup - D.n_small) * P.M;
         if (ts > kMidTasks)
             factor_small_kernel<T, R><<<blocks_for(g.small, ts, kWarps), kThreads, g.small_bytes, st>>>(
                 P, W, S, D, fronts, lfac, ufac, mask, want, D.n_tiny, D.n_small, kSmallFront, 0);
-        else if (ts > 0)
-            factor_mid_kernel<T, R><<<blocks_for(g.mid, ts, 1), kMidThreads, MidShape<T>::bytes, st>>>(
+        else if (wide && tw > 0) {
+            factor_mid_kernel<true><<<blocks_for(g.wide, ts + tw, 1), kMidThreads, g.wide_bytes, st>>>(
+                P, W, S, D, fronts, lfac, ufac, mask, want, D.n_tiny, D.nsup, 0);
+            return;
+        } else if (ts > 0)
+            factor_mid_kernel<false><<<blocks_for(g.mid, ts, 1), kMidThreads, MidShape<T>::bytes, st>>>(
                 P, W, S, D, fronts, lfac, ufac, mask, want, D.n_tiny, D.n_small, 0);
-        if (tb > 0)
+        if (wide && tw > 0)
+            factor_mid_kernel<true><<<blocks_for(g.wide, tw, 1), kMidThreads, g.wide_bytes, st>>>(
+                P, W, S, D, fronts, lfac, ufac, mask, want, D.n_small, D.nsup, 1);
+        else if (tb > 0)
             factor_big_kernel<T, R><<<blocks_for(g.big, tb, 1), kThreads, g.big_bytes, st>>>(
                 P, W, S, D, fronts, lfac, ufac, mask, want);
     } else {

@@ -192,20 +192,21 @@ struct DevMixed {
 
 // Dataflow schedule of the multifrontal factorisation and solves
 // (gp_dag.cu).  order: the supernodes by region (largest front of the
-// subtree: tiny, at most 32 rows, the rest) and by level within
+// subtree: mini, little, tiny, at most 32 rows, the rest) and by level within
 // a region; a topological order of the assembly tree.
 struct DevDag {
     int nsup;
-    // ranks below n_tiny: subtrees with fronts of at most dag_tiny_front()
-    // rows; below n_small: at most 32
-    int n_tiny, n_small;
+    // ranks below n_mini: subtrees with fronts of at most dag_mini_front()
+    // rows; n_little: dag_little_front(); n_tiny: dag_tiny_front(); n_small: 32
+    int n_mini, n_little, n_tiny, n_small;
     int max_front, max_big_front;
     int max_big_whole;            // largest front of the CTA kernel that is not split (FP64)
     const int *order;       // [nsup]
     const int *rank;        // [nsup] position in order
     const int *parent;      // [nsup] parent supernode or -1
     int *ctr;               // [16] claim counters: factor up to 32 rows, big factor, forward top, backward top,
-                            //     forward blocks, backward blocks, forward lower top, tiny factor
+                            //     forward blocks, backward blocks, forward lower top, mini factor,
+                            //     little factor, tiny factor
     int *epoch;             // [1] current solve
     int *err;               // [1] a wait gave up (sticky until the host clears it)
     int *fdone, *xdone, *bdone;   // [nsup][M] epoch at which the task finished
@@ -262,15 +263,17 @@ __host__ __device__ inline int split_cols_cap(int nc, int np) {
 }
 
 struct DagGrid {
-    int tiny = 0, small = 0, mid = 0, big = 0;            // resident blocks
-    int tiny_bytes = 0, small_bytes = 0, big_bytes = 0;     // dynamic shared memory
+    int tiny = 0, small = 0, mid = 0, wide = 0, big = 0;                  // resident blocks
+    int tiny_bytes = 0, small_bytes = 0, wide_bytes = 0, big_bytes = 0;   // dynamic shared memory
 };
 
 int dag_configure(const DevDag &D, int fp32, DagGrid &g);
 // launch_dag_factor<double> also does the forward solve (the right-hand side
 // rides along as an extra front column); launch_dag_factor<float> does not.
+int dag_mini_front();
+int dag_little_front();
 int dag_tiny_front();
-int dag_factor_launches(const DevDag &D, int fp32);   // launches of one factorisation (one per region present)
+int dag_factor_launches(const DevDag &D, int M, int fp32);   // launches of one factorisation
 void launch_dag_begin(const DevDag &D, cudaStream_t st);
 // r[i] = the factorisations' reciprocal of x[i] (device arrays), i < n.
 void launch_recip_check(const double *x, double *r, int n, cudaStream_t st);
