@@ -13,11 +13,14 @@
 // D.wait_limit polls it raises the error flag, every other wait then returns
 // at once, and the kernel finishes with the scenario marked in `status`.
 //
-// Factorisation, in two launches (three for FP64):
+// Factorisation, in two or three launches, from the leaves to the root:
 //  - factor_tiny_kernel (FP64): supernodes whose whole subtree has fronts of
 //    at most kTinyFront rows, four or two scenarios a warp;
 //  - factor_small_kernel: supernodes whose whole subtree has fronts of at
 //    most 32 rows, one warp per task, the front in shared memory;
+//  - factor_mid_kernel (FP64, few such tasks): the same ones a CTA each, the
+//    front in registers, and in the same launch larger fronts up to
+//    kWideFront rows;
 //  - factor_big_kernel: the rest, one CTA per task.
 // Partial pivoting is restricted to a supernode's pivot rows.  The FP32
 // elimination is blocked (the pivot panel column by column, then one
@@ -1129,12 +1132,20 @@ __device__ void factor_rows(const DevProblem &P, const DevWork &W, const DevSym 
         const double rown = recip_normal(special ? 1.0 : own);
         unsigned kh = cand ? key_hi(v) : 0u, kl = cand ? key_lo(v) : 0u;
         unsigned pk = cand ? (unsigned)(pos * 32 + lane) : 0xffffffffu;   // (the smallest place on ties)
+        if constexpr (LW == 32) {
+            const unsigned mh = __reduce_max_sync(FULL, kh);
+            const unsigned ml = __reduce_max_sync(FULL, kh == mh ? kl : 0u);
+            pk = __reduce_min_sync(FULL, cand && kh == mh && kl == ml ? pk : 0xffffffffu);
+            kh = mh;
+            kl = ml;
+        } else {
 #pragma unroll
-        for (int off = LW / 2; off > 0; off >>= 1) {
-            const unsigned oh = __shfl_xor_sync(FULL, kh, off, LW), ol = __shfl_xor_sync(FULL, kl, off, LW),
-                           op = __shfl_xor_sync(FULL, pk, off, LW);
-            const bool take = oh > kh || (oh == kh && (ol > kl || (ol == kl && op < pk)));
-            if (take) { kh = oh; kl = ol; pk = op; }
+            for (int off = LW / 2; off > 0; off >>= 1) {
+                const unsigned oh = __shfl_xor_sync(FULL, kh, off, LW), ol = __shfl_xor_sync(FULL, kl, off, LW),
+                               op = __shfl_xor_sync(FULL, pk, off, LW);
+                const bool take = oh > kh || (oh == kh && (ol > kl || (ol == kl && op < pk)));
+                if (take) { kh = oh; kl = ol; pk = op; }
+            }
         }
         const int pv = (int)(pk >> 5), pl = (int)(pk & 31u);
         if (lane == 0 && act && (kh | kl) == 0u) atomicOr(W.status + m, 4);
@@ -1208,15 +1219,17 @@ __device__ void factor_rows(const DevProblem &P, const DevWork &W, const DevSym 
 // Rows are not exchanged: a row that was pivot at step k drops out of the
 // updates and is stored as pivot row k.  Every entry receives the operations
 // of the right-looking elimination in factor_front.
-// Measured, one warp a front (factor_small_kernel) -> this: 9,001 buses x 3
-// (261 tasks) 145 -> 81 us, 2,000 x 64 (1,344) 144 -> 108 us.
+// Measured, the kernel alone, one warp a front (factor_small_kernel) -> this:
+// 261 tasks (9,001 buses x 3) 145 -> 81 us, 1,344 (2,000 x 64) 144 -> 108 us.
 constexpr int kMidThreads = 128, kMidWarps = 4;
 // FP64 tasks of the region of 21 to 32 rows above which factor_small_kernel
 // (a warp a front, a quarter of the FP64 instructions for reciprocals and
-// multipliers, 24 fronts a SM) takes it: 70,000 buses x 8 (5,240 tasks) 294
-// us against 395, 2,000 x 64 (1,344) 144 against 108, 9,001 x 3 (261) 145
-// against 81.
-constexpr long long kMidTasks = 3000;
+// multipliers, 24 fronts a SM) takes it, and the larger fronts a launch of
+// their own.  The whole factorisation, that against the launch of this
+// kernel: 9,001 buses x 3 (114 tasks) 325 us, 231; 2,000 x 64 (320) 258,
+// 246; 70,000 x 8 (2,776) 649, 581; x 16 (5,552) 958, 939; x 32 (11,104)
+// 1,458, 1,530.
+constexpr long long kMidTasks = 6000;
 constexpr int kWideFront = 64;
 
 template <class T>
@@ -1383,7 +1396,7 @@ __device__ void factor_mid(const DevProblem &P, const DevWork &W, const DevSym &
 // column over the CTA.  The ranks below r0 were factored by earlier launches.
 // With WIDE the fronts above 32 rows and the small ones above them in the
 // tree share one launch with what lies below (FP64 factorisation of 9,001
-// buses x 3 @U@).
+// buses x 3 289 -> 276 us, of 70,000 x 8 625 -> 609).
 template <bool WIDE>
 __global__ void __launch_bounds__(kMidThreads, 6) factor_mid_kernel(DevProblem P, DevWork W, DevSym S, DevDag D,
                                                                     double *fronts, double *lfac, double *ufac,
@@ -1476,7 +1489,7 @@ __global__ void __launch_bounds__(kThreads, 6) factor_small_kernel(DevProblem P,
 // each instruction of a pivot column's steps (pivot search, reciprocal,
 // multipliers) serves all of them: the FP64 pipe, which bounds the kernel,
 // charges a warp instruction the same whatever its active lanes.
-// Measured (70,000 buses x 8): two scenarios a warp for both 360 us -> @T@.
+// Measured (70,000 buses x 8): two scenarios a warp throughout 423 us -> 356.
 struct TaskGroup {
     int s, m;      // supernode, the lane group's scenario
     bool act;      // factored by this launch
@@ -1510,6 +1523,15 @@ constexpr int kTinyArea = 4 * warp_area_bytes<double>(kLittleFront) > 2 * warp_a
                               ? 4 * warp_area_bytes<double>(kLittleFront)
                               : 2 * warp_area_bytes<double>(kTinyFront);
 
+// With at most kTinyFew tasks every one of them is in flight at once, so the
+// time of a front counts instead of the FP64 instructions: each front gets a
+// warp, a lane a row.  The whole factorisation, shared warps against a warp
+// each: 2,000 buses x 10 (6,760 tasks) 181 us, 166; 9,001 x 3 (8,910) 246,
+// 231, x 5 (14,850) 259, 250, x 6 (17,820) 259, 259; 2,000 x 24 (16,200) 200,
+// 206, x 64 (43,000) 240, 333.
+constexpr long long kTinyFew = 15000;
+
+template <bool FEW>
 __global__ void __launch_bounds__(kThreads, 4) factor_tiny_kernel(DevProblem P, DevWork W, DevSym S, DevDag D,
                                                                   double *fronts, double *lfac, double *ufac,
                                                                   const uint8_t *mask, int want) {
@@ -1519,42 +1541,57 @@ __global__ void __launch_bounds__(kThreads, 4) factor_tiny_kernel(DevProblem P, 
     const int M = P.M, epoch = *D.epoch;
     TaskGroup g;
     bool more = true;
-    while (more) {
-        if (!claim_group<8>(D, mask, want, M, 0, D.n_mini, 7, g, more)) continue;
-        factor_rows<8>(
-            P, W, S, fronts, lfac, ufac, g.s, g.m, g.act,
-            reinterpret_cast<double *>(wbase) + (lane / 8) * kMiniFront * (kMiniFront + 1),
-            [&] {
-                if (!group_wait_children<8>(S, D, D.fdone, g.s, g.m, M, epoch) && (lane & 7) == 0 && g.act)
-                    atomicOr(W.status + g.m, 8);
-            },
-            [&] {
-                if ((lane & 7) == 0 && g.act) signal_done(D.fdone + (size_t)g.s * M + g.m, epoch);
-            });
-    }
-    // (wider fronts: LW lanes each, the updates flattened over them)
-    auto rest = [&](auto width, int cap, int r0, int r1, int ctr) {
-        constexpr int LW = decltype(width)::value;
-        unsigned char *gbase = wbase + (size_t)(lane / LW) * warp_area_bytes<double>(cap);
-        double *F = reinterpret_cast<double *>(gbase);
-        int *piv = reinterpret_cast<int *>(gbase + warp_front_bytes<double>(cap));
-        bool more = true;
+    if constexpr (FEW) {
         while (more) {
-            if (!claim_group<LW>(D, mask, want, M, r0, r1, ctr, g, more)) continue;
-            factor_front<double, true>(
-                P, W, S, fronts, lfac, ufac, g.s, g.m, F, piv, LaneGroup<LW>{g.act},
+            if (!claim_group<32>(D, mask, want, M, 0, D.n_tiny, 7, g, more)) continue;
+            factor_rows<32>(
+                P, W, S, fronts, lfac, ufac, g.s, g.m, true, reinterpret_cast<double *>(wbase),
                 [&] {
-                    if (!group_wait_children<LW>(S, D, D.fdone, g.s, g.m, M, epoch) && (lane & (LW - 1)) == 0 &&
-                        g.act)
+                    if (!warp_wait_children(S, D, D.fdone, g.s, g.m, M, epoch, 0) && lane == 0)
                         atomicOr(W.status + g.m, 8);
                 },
                 [&] {
-                    if ((lane & (LW - 1)) == 0 && g.act) signal_done(D.fdone + (size_t)g.s * M + g.m, epoch);
+                    if (lane == 0) signal_done(D.fdone + (size_t)g.s * M + g.m, epoch);
                 });
         }
-    };
-    rest(std::integral_constant<int, 8>(), kLittleFront, D.n_mini, D.n_little, 8);
-    rest(std::integral_constant<int, 16>(), kTinyFront, D.n_little, D.n_tiny, 9);
+    } else {
+        while (more) {
+            if (!claim_group<8>(D, mask, want, M, 0, D.n_mini, 7, g, more)) continue;
+            factor_rows<8>(
+                P, W, S, fronts, lfac, ufac, g.s, g.m, g.act,
+                reinterpret_cast<double *>(wbase) + (lane / 8) * kMiniFront * (kMiniFront + 1),
+                [&] {
+                    if (!group_wait_children<8>(S, D, D.fdone, g.s, g.m, M, epoch) && (lane & 7) == 0 && g.act)
+                        atomicOr(W.status + g.m, 8);
+                },
+                [&] {
+                    if ((lane & 7) == 0 && g.act) signal_done(D.fdone + (size_t)g.s * M + g.m, epoch);
+                });
+        }
+        // (wider fronts: LW lanes each, the updates flattened over them)
+        auto rest = [&](auto width, int cap, int r0, int r1, int ctr) {
+            constexpr int LW = decltype(width)::value;
+            unsigned char *gbase = wbase + (size_t)(lane / LW) * warp_area_bytes<double>(cap);
+            double *F = reinterpret_cast<double *>(gbase);
+            int *piv = reinterpret_cast<int *>(gbase + warp_front_bytes<double>(cap));
+            bool more = true;
+            while (more) {
+                if (!claim_group<LW>(D, mask, want, M, r0, r1, ctr, g, more)) continue;
+                factor_front<double, true>(
+                    P, W, S, fronts, lfac, ufac, g.s, g.m, F, piv, LaneGroup<LW>{g.act},
+                    [&] {
+                        if (!group_wait_children<LW>(S, D, D.fdone, g.s, g.m, M, epoch) && (lane & (LW - 1)) == 0 &&
+                            g.act)
+                            atomicOr(W.status + g.m, 8);
+                    },
+                    [&] {
+                        if ((lane & (LW - 1)) == 0 && g.act) signal_done(D.fdone + (size_t)g.s * M + g.m, epoch);
+                    });
+            }
+        };
+        rest(std::integral_constant<int, 8>(), kLittleFront, D.n_mini, D.n_little, 8);
+        rest(std::integral_constant<int, 16>(), kTinyFront, D.n_little, D.n_tiny, 9);
+    }
 }
 
 template <class T, bool RHS>
@@ -1660,12 +1697,16 @@ int configure_one(DagGrid &g, int nsm, int tiny_bytes, int small_bytes, int big_
         return -1;
     g.small = nsm * occ;
     if constexpr (sizeof(T) == 8) {
-        if (cudaFuncSetAttribute(factor_tiny_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tiny_bytes) !=
-                cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, factor_tiny_kernel, kThreads, tiny_bytes) !=
+        if (!raise_shared_limit(factor_tiny_kernel<false>, tiny_bytes) ||
+            !raise_shared_limit(factor_tiny_kernel<true>, tiny_bytes) ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, factor_tiny_kernel<false>, kThreads, tiny_bytes) !=
                 cudaSuccess || occ < 1)
             return -1;
         g.tiny = nsm * occ;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, factor_tiny_kernel<true>, kThreads, tiny_bytes) !=
+                cudaSuccess || occ < 1)
+            return -1;
+        g.few = nsm * occ;
         if (!raise_shared_limit(factor_mid_kernel<false>, MidShape<T>::bytes) ||
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, factor_mid_kernel<false>, kMidThreads,
                                                           MidShape<T>::bytes) != cudaSuccess || occ < 1)
@@ -1751,8 +1792,12 @@ void launch_dag_factor(const DevProblem &P, const DevWork &W, const DevSym &S, c
         const long long tt = std::max((long long)D.n_little * ((P.M + 3) / 4),
                                       (long long)(D.n_tiny - D.n_little) * ((P.M + 1) / 2)),
                         ts = (long long)(D.n_small - D.n_tiny) * P.M, tb = (long long)D.big_units * P.M;
-        if (tt > 0)
-            factor_tiny_kernel<<<blocks_for(g.tiny, tt, kWarps), kThreads, g.tiny_bytes, st>>>(P, W, S, D, fronts, lfac,
+        const long long tf = (long long)D.n_tiny * P.M;
+        if (tf > 0 && tf <= kTinyFew)
+            factor_tiny_kernel<true><<<blocks_for(g.few, tf, kWarps), kThreads, g.tiny_bytes, st>>>(
+                P, W, S, D, fronts, lfac, ufac, mask, want);
+        else if (tt > 0)
+            factor_tiny_kernel<false><<<blocks_for(g.tiny, tt, kWarps), kThreads, g.tiny_bytes, st>>>(P, W, S, D, fronts, lfac,
                                                                                                ufac, mask, want);
         const bool wide = D.max_front <= kWideFront;
         const long long tw = (long long)(D.nsup - D.n_small) * P.M;

@@ -263,7 +263,7 @@ __host__ __device__ inline int split_cols_cap(int nc, int np) {
 }
 
 struct DagGrid {
-    int tiny = 0, small = 0, mid = 0, wide = 0, big = 0;                  // resident blocks
+    int tiny = 0, few = 0, small = 0, mid = 0, wide = 0, big = 0;         // resident blocks
     int tiny_bytes = 0, small_bytes = 0, wide_bytes = 0, big_bytes = 0;   // dynamic shared memory
 };
 
