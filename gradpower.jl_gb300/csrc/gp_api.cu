@@ -552,8 +552,23 @@ constexpr int kLuAlign = 4;   // 16 bytes of FP32, 32 of FP64
 
 int64_t lu_align(int64_t x) { return (x + kLuAlign - 1) / kLuAlign * kLuAlign; }
 
-void make_blocks(const gp::Symbolic &sym, HostBlk &B) {
-    constexpr long kLimSlices = 2048, kLimRows = 512, kLimSups = 64;
+// Budget of a block in factor entries for M scenarios.  One warp runs a block
+// from end to end: a large block saves hand-offs, a small one gives the chip
+// more warps to run, so the budget follows the number of tasks (supernodes x
+// scenarios).  Measured, the solves of a run in ms at 2048 / 1024 / 512 / 256
+// entries: 70,000 buses x 8 (FP32, 188,000 tasks) 21.5 / 23.6 / 30.0 / 39.9,
+// 2,000 x 256 (FP32, 174,000) 15.4 / 15.6 / 20.3 / 27.3, x 64 (FP64, 43,600)
+// 6.74 / 5.53 / 5.87 / 7.24, x 32 (shared, 21,800) 18.5 / 15.8 / 15.1 / 16.7,
+// 9,001 x 5 (FP32, 15,000) 12.2 / 9.75 / 8.89 / 8.88, 2,000 x 7 (FP32, 4,800)
+// 9.54 / 7.56 / 7.32 / 7.03, and 7.02 at 128.
+constexpr long kBlkMax = 2048, kBlkMin = 256, kBlkShare = 40;
+
+long block_budget(long nsup, long M) {
+    return std::min(kBlkMax, std::max(kBlkMin, nsup * M / kBlkShare));
+}
+
+void make_blocks(const gp::Symbolic &sym, long budget, HostBlk &B) {
+    const long kLimRows = budget / 4, kLimSups = budget / 32;
     const long kLimFront = gp::solve_block_front_limit();
     const int ns = sym.nsup;
     std::vector<long> sl(ns, 0), sv(ns, 0), sn(ns, 0), sm(ns, 0);
@@ -574,7 +589,7 @@ void make_blocks(const gp::Symbolic &sym, HostBlk &B) {
             }
         }
     auto fits = [&](int s) {
-        return sl[s] <= kLimSlices && sv[s] <= kLimRows && sn[s] <= kLimSups && sm[s] <= kLimFront;
+        return sl[s] <= budget && sv[s] <= kLimRows && sn[s] <= kLimSups && sm[s] <= kLimFront;
     };
     // levels run from the leaves (0) to the roots, so parents are visited
     // before their children here
@@ -1275,7 +1290,7 @@ void build_dag(gp_layout *L, const gp::Symbolic &sym) {
 
 void build_blocks(gp_layout *L, const gp::Symbolic &sym) {
     HostBlk H;
-    make_blocks(sym, H);
+    make_blocks(sym, block_budget(sym.nsup, L->M), H);
     DeviceArena &A = L->arena;
     gp::DevBlk &B = L->B;
     B.nblk = H.nblk;
@@ -2694,13 +2709,19 @@ int32_t gp_reduced_selftest(const gp_problem *prob, const int32_t *s_rowptr, con
     const int zp = host_factor(pl, svar, fronts, ipiv);
     std::vector<double> xl = xp;
     host_level_solve(pl.sym, fronts, ipiv, xl);
-    HostBlk hb;
-    make_blocks(pl.sym, hb);
-    host_block_solve(pl.sym, hb, fronts, ipiv, xp);
+    // (the blocks of the smallest and of the largest budget)
     double dmax = 0.0, xmax = 0.0;
-    for (int k = 0; k < n; k++) {
-        dmax = std::max(dmax, std::fabs(xp[k] - xl[k]));
-        xmax = std::max(xmax, std::fabs(xl[k]));
+    const std::vector<double> xp0 = xp;
+    HostBlk hb;
+    for (long budget : {kBlkMin, kBlkMax}) {
+        hb = HostBlk();
+        xp = xp0;
+        make_blocks(pl.sym, budget, hb);
+        host_block_solve(pl.sym, hb, fronts, ipiv, xp);
+        for (int k = 0; k < n; k++) {
+            dmax = std::max(dmax, std::fabs(xp[k] - xl[k]));
+            xmax = std::max(xmax, std::fabs(xl[k]));
+        }
     }
     for (int k = 0; k < n; k++) x[pl.sym.perm[k]] = xp[k];
     // the split fronts' elimination (factor_part, emulated) against the
