@@ -703,7 +703,10 @@ void make_blocks(const gp::Symbolic &sym, long budget, HostBlk &B) {
         }
         B.n_lower_top = 0;
         for (int s : B.top_order)
-            if (tlev[s] < lv) B.n_lower_top++;
+            if (tlev[s] < lv) {
+                B.n_lower_top++;
+                B.max_v = std::max(B.max_v, sym.front_m(s));   // (its vector lies where a block's does)
+            }
     }
     // solve-ordered factor copies: the blocks in the order they are claimed,
     // then the top supernodes
