@@ -532,9 +532,9 @@ struct HostBlk {
     std::vector<int4> ent0, ent1;
     int n_top_levels = 0, top_max_front = 1, top_max_xent = 1;
     // the first n_lower_top entries of top_order (whole levels, each front
-    // of at most solve_block_front_limit() rows) are forward-solved by one
-    // warp per task, the rest (and the whole backward pass) by one CTA per
-    // task
+    // of at most solve_block_front_limit() rows) can be forward-solved by one
+    // warp per task (build_blocks takes as many of them as do better there),
+    // the rest (and the whole backward pass) by one CTA per task
     int n_lower_top = 0;
     std::vector<int> top_order, top_rank;
     std::vector<int> top_xptr, top_xrow, top_xent;   // extend-add lists of the top region
@@ -556,11 +556,11 @@ int64_t lu_align(int64_t x) { return (x + kLuAlign - 1) / kLuAlign * kLuAlign; }
 // from end to end: a large block saves hand-offs, a small one gives the chip
 // more warps to run, so the budget follows the number of tasks (supernodes x
 // scenarios).  Measured, the solves of a run in ms at 2048 / 1024 / 512 / 256
-// entries: 70,000 buses x 8 (FP32, 188,000 tasks) 21.5 / 23.6 / 30.0 / 39.9,
-// 2,000 x 256 (FP32, 174,000) 15.4 / 15.6 / 20.3 / 27.3, x 64 (FP64, 43,600)
-// 6.74 / 5.53 / 5.87 / 7.24, x 32 (shared, 21,800) 18.5 / 15.8 / 15.1 / 16.7,
-// 9,001 x 5 (FP32, 15,000) 12.2 / 9.75 / 8.89 / 8.88, 2,000 x 7 (FP32, 4,800)
-// 9.54 / 7.56 / 7.32 / 7.03, and 7.02 at 128.
+// entries: 70,000 buses x 8 (FP32, 188,000 tasks) 18.7 / 20.7 / 27.2 / 37.1,
+// 2,000 x 256 (FP32, 174,000) 14.6 / 14.9 / 19.6 / 26.7, x 64 (FP64, 43,600)
+// 6.76 / 5.62 / 5.91 / 7.24, x 32 (shared, 21,800) 16.0 / 12.8 / 12.5 / 14.3,
+// 9,001 x 5 (FP32, 15,000) 10.4 / 7.73 / 6.81 / 6.85, 2,000 x 7 (FP32, 4,800)
+// 8.55 / 6.29 / 5.66 / 5.28, and 5.28 at 128.
 constexpr long kBlkMax = 2048, kBlkMin = 256, kBlkShare = 40;
 
 long block_budget(long nsup, long M) {
@@ -1330,6 +1330,16 @@ void build_blocks(gp_layout *L, const gp::Symbolic &sym) {
     const int sc = gp::solve_configure(B, L->SG);
     if (sc == -2) fail(GP_E_INVALID, "front of %d rows exceeds the solve kernels' staging area", B.top_max_front);
     if (sc != 0) fail(GP_E_CUDA, "could not configure the solve kernels");
+    // A CTA stages a top task's factors while it waits for the children and
+    // hands on sooner than a warp, but only the tasks that resident CTAs hold
+    // wait that way: the last ones, as many as there are CTAs, go to CTAs and
+    // only what lies below to warps.  Measured, the solves of a run with all
+    // of the lower region on warps / as many on CTAs as are resident / all on
+    // CTAs: 2,000 buses x 7 (FP32, 1,106 top tasks, so all on CTAs) 7.02 /
+    // 5.28 / 5.28 ms, x 32 (shared, 2,528) 15.2 / 12.4 / 12.2, x 256 (FP32,
+    // 5,376) 15.4 / 14.3 / 15.2, 9,001 x 5 (2,530) 8.94 / 6.57 / 6.94, 70,000 x
+    // 8 (5,680) 21.5 / 18.5 / 19.4.
+    B.n_lower_top = std::min(B.n_lower_top, std::max(0, B.n_top - std::max(1, L->SG.top_fwd / L->M)));
 }
 
 // Lists of the one-CTA path (build_small) from the plan: the fronts' places in

@@ -16,9 +16,10 @@
 //    memory (cp.async, all threads) and loads its own right-hand-side
 //    entries before it waits, bounded, on the tasks it depends on; one warp
 //    then sweeps the front from shared memory.
-//  - in the forward pass the top region's first levels (fronts of at most
-//    kBlkFront rows) are tasks of one warp each, a supernode per task
-//    waiting on its children.
+//  - in the forward pass of a large batch the lower part of the top region
+//    (fronts of at most kBlkFront rows) are tasks of one warp each, a
+//    supernode per task waiting on its children; as many tasks as there are
+//    resident CTAs stay with the CTAs (gp_api.cu, build_blocks).
 // One persistent kernel per direction runs them all: forward, the warps
 // claim the block tasks, then the lower top tasks, and the CTAs then the
 // rest of the top region; backward, the CTAs claim the top tasks, then the
@@ -535,8 +536,8 @@ __device__ void bwd_block(const DevProblem &P, const DevWork &W, const DevSym &S
 }
 
 // ---- lower top region, forward: one warp per task ---------------------------
-// In the forward pass the top supernodes of the first levels (fronts of at
-// most kBlkFront rows) are tasks of one warp each, like a block of one
+// In the forward pass the top supernodes beyond those the CTAs take (fronts of
+// at most kBlkFront rows) are tasks of one warp each, like a block of one
 // supernode that waits on its children: through tagged words on FP32
 // factors, through done flags on FP64 factors.  The warp keeps the front's
 // vector in its shared-memory area and reads the factors through L1 (pulled
