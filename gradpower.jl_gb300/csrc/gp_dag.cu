@@ -14,8 +14,8 @@
 // at once, and the kernel finishes with the scenario marked in `status`.
 //
 // Factorisation, in two or three launches, from the leaves to the root:
-//  - factor_tiny_kernel (FP64): supernodes whose whole subtree has fronts of
-//    at most kTinyFront rows, four or two scenarios a warp;
+//  - factor_tiny_kernel: supernodes whose whole subtree has fronts of at most
+//    kTinyFront rows, four or two scenarios a warp;
 //  - factor_small_kernel: supernodes whose whole subtree has fronts of at
 //    most 32 rows, one warp per task, the front in shared memory;
 //  - factor_mid_kernel (FP64, few such tasks): the same ones a CTA each, the
@@ -54,11 +54,9 @@ constexpr unsigned FULL = kFullMask;
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kSmallFront = 32;   // rows a warp of factor_small_kernel has room for
-// FP64 factorisations run the subtrees whose fronts have at most kTinyFront
-// rows first, in a launch of their own with smaller front buffers (more
-// fronts in flight) and several scenarios a warp (factor_tiny_kernel).  FP32
-// ones keep one launch: their 32-row buffers already allow 48 warps, and the
-// launch boundary would cost the overlap of the two regions.
+// The subtrees whose fronts have at most kTinyFront rows run first, in a launch
+// of their own with smaller front buffers (more fronts in flight) and several
+// scenarios a warp (factor_tiny_kernel), but for small FP32 batches.
 constexpr int kMiniFront = 8, kLittleFront = 14, kTinyFront = 20;
 // update-matrix entries a thread loads ahead in the extend-add: none in the
 // warp kernel, which runs at 40 registers a thread and many warps a SM
@@ -139,6 +137,8 @@ struct KeyOf<float> {
 
 __device__ __forceinline__ unsigned key_hi(double v) { return (unsigned)__double2hiint(v) & 0x7fffffffu; }
 __device__ __forceinline__ unsigned key_lo(double v) { return (unsigned)__double2loint(v); }
+__device__ __forceinline__ unsigned key_hi(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+__device__ __forceinline__ unsigned key_lo(float) { return 0u; }
 
 // LW < 32: the warp is LW-lane segments, each searching its own front (the
 // whole warp calls it).  A whole warp takes the maximum by integer
@@ -1069,31 +1069,31 @@ __host__ __device__ inline int big_front_bytes(int max_front) {
 // eliminated order, exchanged as the other kernels exchange rows) and are
 // put in order as they are stored.  Every entry receives the operations of
 // factor_front.
-template <int LW, class Wait, class Done>
-__device__ void factor_rows(const DevProblem &P, const DevWork &W, const DevSym &S, double *fronts, double *lfac,
-                            double *ufac, int s, int m, bool act, double *F, Wait wait, Done done) {
+template <class T, bool RHS, int LW, class Wait, class Done>
+__device__ void factor_rows(const DevProblem &P, const DevWork &W, const DevSym &S, T *fronts, T *lfac, T *ufac, int s,
+                            int m, bool act, T *F, Wait wait, Done done) {
     const int lane = threadIdx.x & (LW - 1);
     const int start = S.sup_start[s];
     const int ns = S.sup_start[s + 1] - start;
-    const int mm = ns + S.row_ptr[s + 1] - S.row_ptr[s], nc = mm + 1;
-    double *fr = fronts + (size_t)m * S.front_total;
+    const int mm = ns + S.row_ptr[s + 1] - S.row_ptr[s], nc = mm + (RHS ? 1 : 0);
+    T *fr = fronts + (size_t)m * S.front_total;
     double *x = W.xperm + (size_t)m * P.n_red;
     double *uv = S.uvec + (size_t)m * S.uvec_total;
     const bool row = lane < mm;
     // ---- the front's own entries ----
-    const double xr = lane < ns ? x[start + lane] : 0.0;
+    const T xr = RHS && lane < ns ? (T)x[start + lane] : T(0);
     for (int j = 0; j < mm; j++)
-        if (row) F[lane + j * mm] = 0.0;
-    if (row) F[lane + mm * mm] = xr;
+        if (row) F[lane + j * mm] = T(0);
+    if (RHS && row) F[lane + mm * mm] = xr;
     __syncwarp();
-    for (int e = S.asmc_ptr[s] + lane; e < S.asmc_ptr[s + 1]; e += LW) F[S.asmc_pos[e]] += S.asmc_val[e];
+    for (int e = S.asmc_ptr[s] + lane; e < S.asmc_ptr[s + 1]; e += LW) F[S.asmc_pos[e]] += (T)S.asmc_val[e];
     __syncwarp();
     const double *sv = W.svar + (size_t)m * P.n_var;
-    for (int e = S.asmv_ptr[s] + lane; e < S.asmv_ptr[s + 1]; e += LW) F[S.asmv_pos[e]] += sv[S.asmv_idx[e]];
+    for (int e = S.asmv_ptr[s] + lane; e < S.asmv_ptr[s + 1]; e += LW) F[S.asmv_pos[e]] += (T)sv[S.asmv_idx[e]];
     if (S.asmt_ptr)
         for (int e = S.asmt_ptr[s] + lane; e < S.asmt_ptr[s + 1]; e += LW) {
             const int t = S.asmt_tr[e];
-            if (P.tr_on[t] && t >= P.tr_ptr[m] && t < P.tr_ptr[m + 1]) F[S.asmt_pos[e]] += S.asmt_val[e];
+            if (P.tr_on[t] && t >= P.tr_ptr[m] && t < P.tr_ptr[m + 1]) F[S.asmt_pos[e]] += (T)S.asmt_val[e];
         }
     __syncwarp();
     wait();   // for the children (bounded); ends with a warp barrier
@@ -1102,46 +1102,49 @@ __device__ void factor_rows(const DevProblem &P, const DevWork &W, const DevSym 
         const int c = S.children[q];
         const int ncc = S.sup_start[c + 1] - S.sup_start[c], rc = S.row_ptr[c + 1] - S.row_ptr[c], mc = ncc + rc;
         const int *rel = S.relmap + S.relmap_ptr[c];
-        const double *Fc = fr + S.front_off[c] + (size_t)ncc * mc + ncc, *uc = uv + S.uvec_off[c];
+        const T *Fc = fr + S.front_off[c] + (size_t)ncc * mc + ncc;
+        const double *uc = uv + S.uvec_off[c];
+        const int cols = rc + (RHS ? 1 : 0);
         const int ra = lane < rc ? rel[lane] : 0;
         // lane a on row a of the update matrix (rc < LW); four columns' loads
         // together
-        for (int b0 = 0; b0 <= rc; b0 += 4) {
-            double v[4];
+        for (int b0 = 0; b0 < cols; b0 += 4) {
+            T v[4];
             int rb[4];
 #pragma unroll
             for (int u = 0; u < 4; u++) {
                 const int b = b0 + u;
-                const bool in = lane < rc && b <= rc;
-                v[u] = in ? __ldcg(b < rc ? Fc + lane + (size_t)b * mc : uc + lane) : 0.0;
+                const bool in = lane < rc && b < cols;
+                v[u] = !in ? T(0) : b < rc ? __ldcg(Fc + lane + (size_t)b * mc) : (T)__ldcg(uc + lane);
                 rb[u] = in && b < rc ? rel[b] : mm;
             }
 #pragma unroll
             for (int u = 0; u < 4; u++)
-                if (lane < rc && b0 + u <= rc) F[ra + rb[u] * mm] += v[u];
+                if (lane < rc && b0 + u < cols) F[ra + rb[u] * mm] += v[u];
         }
         __syncwarp();
     }
     // ---- elimination ----
     int pos = lane;
-    double v = row ? F[lane] : 0.0;
+    T v = row ? F[lane] : T(0);
     for (int k = 0; k < ns; k++) {
         const bool cand = pos >= k && pos < ns;
-        const double own = cand ? v : 1.0;
-        const bool special = recip_special(own);
-        const double rown = recip_normal(special ? 1.0 : own);
+        const T own = cand ? v : T(1);
+        const bool special = sizeof(T) == 8 && recip_special(own);
+        const T rown = recip_normal(special ? T(1) : own);
         unsigned kh = cand ? key_hi(v) : 0u, kl = cand ? key_lo(v) : 0u;
         unsigned pk = cand ? (unsigned)(pos * 32 + lane) : 0xffffffffu;   // (the smallest place on ties)
         if constexpr (LW == 32) {
             const unsigned mh = __reduce_max_sync(FULL, kh);
-            const unsigned ml = __reduce_max_sync(FULL, kh == mh ? kl : 0u);
+            const unsigned ml = sizeof(T) == 8 ? __reduce_max_sync(FULL, kh == mh ? kl : 0u) : 0u;
             pk = __reduce_min_sync(FULL, cand && kh == mh && kl == ml ? pk : 0xffffffffu);
             kh = mh;
             kl = ml;
         } else {
 #pragma unroll
             for (int off = LW / 2; off > 0; off >>= 1) {
-                const unsigned oh = __shfl_xor_sync(FULL, kh, off, LW), ol = __shfl_xor_sync(FULL, kl, off, LW),
+                const unsigned oh = __shfl_xor_sync(FULL, kh, off, LW),
+                               ol = sizeof(T) == 8 ? __shfl_xor_sync(FULL, kl, off, LW) : kl,
                                op = __shfl_xor_sync(FULL, pk, off, LW);
                 const bool take = oh > kh || (oh == kh && (ol > kl || (ol == kl && op < pk)));
                 if (take) { kh = oh; kl = ol; pk = op; }
@@ -1149,20 +1152,22 @@ __device__ void factor_rows(const DevProblem &P, const DevWork &W, const DevSym 
         }
         const int pv = (int)(pk >> 5), pl = (int)(pk & 31u);
         if (lane == 0 && act && (kh | kl) == 0u) atomicOr(W.status + m, 4);
-        double inv = __shfl_sync(FULL, rown, pl, LW);
-        const bool sp = __shfl_sync(FULL, (int)special, pl, LW) != 0;
-        if (__any_sync(FULL, sp)) {
-            const double d = __shfl_sync(FULL, own, pl, LW);
-            if (sp) inv = 1.0 / d;
+        T inv = __shfl_sync(FULL, rown, pl, LW);
+        if constexpr (sizeof(T) == 8) {
+            const bool sp = __shfl_sync(FULL, (int)special, pl, LW) != 0;
+            if (__any_sync(FULL, sp)) {
+                const double d = __shfl_sync(FULL, own, pl, LW);
+                if (sp) inv = 1.0 / d;
+            }
         }
         if (lane == pl) pos = k;
         else if (pos == k) pos = pv;
         const bool upd = row && pos > k;
-        const double l = v * inv;
+        const T l = v * inv;
         if (upd || lane == pl) F[lane + k * mm] = upd ? l : inv;
-        {
-            const double u = F[pl + (k + 1) * mm];
-            v = row ? F[lane + (k + 1) * mm] : 0.0;
+        if (RHS || k + 1 < nc) {
+            const T u = F[pl + (k + 1) * mm];
+            v = row ? F[lane + (k + 1) * mm] : T(0);
             if (upd) {
                 v -= l * u;
                 F[lane + (k + 1) * mm] = v;
@@ -1170,7 +1175,7 @@ __device__ void factor_rows(const DevProblem &P, const DevWork &W, const DevSym 
         }
 #pragma unroll 4
         for (int j = k + 2; j < nc; j++) {
-            const double u = F[pl + j * mm];
+            const T u = F[pl + j * mm];
             if (upd) F[lane + j * mm] -= l * u;
         }
         __syncwarp();
@@ -1179,22 +1184,22 @@ __device__ void factor_rows(const DevProblem &P, const DevWork &W, const DevSym 
     // done(), then the solve-ordered copies and the composed pivots ----
     if (act && row) {
         if (lane >= ns) {
-            double *out = fr + S.front_off[s];
+            T *out = fr + S.front_off[s];
             for (int j = ns; j < mm; j++) out[lane + (size_t)j * mm] = F[lane + j * mm];
-            uv[S.uvec_off[s] + lane - ns] = F[lane + mm * mm];
-        } else {
-            x[start + pos] = F[lane + mm * mm];
+            if (RHS) uv[S.uvec_off[s] + lane - ns] = (double)F[lane + mm * mm];
+        } else if (RHS) {
+            x[start + pos] = (double)F[lane + mm * mm];
         }
     }
     __syncwarp();
     done();
     if (act && row) {
         if (lfac) {
-            double *lo = lfac + (size_t)m * S.lu_total + S.lu_off[s];
+            T *lo = lfac + (size_t)m * S.lu_total + S.lu_off[s];
             for (int j = 0; j < ns; j++) lo[pos + (size_t)j * mm] = F[lane + j * mm];
         }
         if (lane < ns) {
-            double *uo = ufac + (size_t)m * S.lu_total + S.lu_off[s];
+            T *uo = ufac + (size_t)m * S.lu_total + S.lu_off[s];
             for (int j = 0; j < mm; j++) uo[pos + (size_t)j * ns] = F[lane + j * mm];
             S.ipiv[(size_t)m * S.n + start + pos] = lane;
         }
@@ -1487,8 +1492,9 @@ __global__ void __launch_bounds__(kThreads, 6) factor_small_kernel(DevProblem P,
 //    300).
 // The groups belong to the same supernode, so they run the same loops, and
 // each instruction of a pivot column's steps (pivot search, reciprocal,
-// multipliers) serves all of them: the FP64 pipe, which bounds the kernel,
-// charges a warp instruction the same whatever its active lanes.
+// multipliers) serves all of them: the FP64 pipe, which bounds the FP64 kernel,
+// charges a warp instruction the same whatever its active lanes; the FP32
+// kernel is bound by the instructions it issues.
 // Measured (70,000 buses x 8): two scenarios a warp throughout 423 us -> 356.
 struct TaskGroup {
     int s, m;      // supernode, the lane group's scenario
@@ -1519,9 +1525,12 @@ __device__ bool claim_group(const DevDag &D, const uint8_t *mask, int want, int 
 }
 
 // shared memory of a warp: four fronts of kLittleFront rows or two of kTinyFront
-constexpr int kTinyArea = 4 * warp_area_bytes<double>(kLittleFront) > 2 * warp_area_bytes<double>(kTinyFront)
-                              ? 4 * warp_area_bytes<double>(kLittleFront)
-                              : 2 * warp_area_bytes<double>(kTinyFront);
+template <class T>
+__host__ __device__ constexpr int tiny_area() {
+    return 4 * warp_area_bytes<T>(kLittleFront) > 2 * warp_area_bytes<T>(kTinyFront)
+               ? 4 * warp_area_bytes<T>(kLittleFront)
+               : 2 * warp_area_bytes<T>(kTinyFront);
+}
 
 // With at most kTinyFew tasks every one of them is in flight at once, so the
 // time of a front counts instead of the FP64 instructions: each front gets a
@@ -1530,22 +1539,29 @@ constexpr int kTinyArea = 4 * warp_area_bytes<double>(kLittleFront) > 2 * warp_a
 // 231, x 5 (14,850) 259, 250, x 6 (17,820) 259, 259; 2,000 x 24 (16,200) 200,
 // 206, x 64 (43,000) 240, 333.
 constexpr long long kTinyFew = 15000;
+// FP32: up to so many tasks one launch of factor_small_kernel takes these
+// fronts too (a warp each, the two regions overlapping).  Measured, the
+// factorisations of a run, that against this kernel: 9,001 buses x 5 (14,850
+// tasks) 3.15 ms, 4.00, x 20 (59,400) 4.70, 4.76; 2,000 x 64 (43,000) 3.76,
+// 4.03, x 128 (86,500) 4.61, 4.03, x 256 (173,000) 7.68, 5.48; 70,000 x 8
+// (186,000) 10.5, 8.22.
+constexpr long long kTinyFew32 = 60000;
 
-template <bool FEW>
+template <class T, bool RHS, bool FEW>
 __global__ void __launch_bounds__(kThreads, 4) factor_tiny_kernel(DevProblem P, DevWork W, DevSym S, DevDag D,
-                                                                  double *fronts, double *lfac, double *ufac,
-                                                                  const uint8_t *mask, int want) {
+                                                                  T *fronts, T *lfac, T *ufac, const uint8_t *mask,
+                                                                  int want) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    unsigned char *wbase = smem_raw + (size_t)warp * kTinyArea;
+    unsigned char *wbase = smem_raw + (size_t)warp * tiny_area<T>();
     const int M = P.M, epoch = *D.epoch;
     TaskGroup g;
     bool more = true;
     if constexpr (FEW) {
         while (more) {
             if (!claim_group<32>(D, mask, want, M, 0, D.n_tiny, 7, g, more)) continue;
-            factor_rows<32>(
-                P, W, S, fronts, lfac, ufac, g.s, g.m, true, reinterpret_cast<double *>(wbase),
+            factor_rows<T, RHS, 32>(
+                P, W, S, fronts, lfac, ufac, g.s, g.m, true, reinterpret_cast<T *>(wbase),
                 [&] {
                     if (!warp_wait_children(S, D, D.fdone, g.s, g.m, M, epoch, 0) && lane == 0)
                         atomicOr(W.status + g.m, 8);
@@ -1557,9 +1573,9 @@ __global__ void __launch_bounds__(kThreads, 4) factor_tiny_kernel(DevProblem P, 
     } else {
         while (more) {
             if (!claim_group<8>(D, mask, want, M, 0, D.n_mini, 7, g, more)) continue;
-            factor_rows<8>(
+            factor_rows<T, RHS, 8>(
                 P, W, S, fronts, lfac, ufac, g.s, g.m, g.act,
-                reinterpret_cast<double *>(wbase) + (lane / 8) * kMiniFront * (kMiniFront + 1),
+                reinterpret_cast<T *>(wbase) + (lane / 8) * kMiniFront * (kMiniFront + 1),
                 [&] {
                     if (!group_wait_children<8>(S, D, D.fdone, g.s, g.m, M, epoch) && (lane & 7) == 0 && g.act)
                         atomicOr(W.status + g.m, 8);
@@ -1571,13 +1587,13 @@ __global__ void __launch_bounds__(kThreads, 4) factor_tiny_kernel(DevProblem P, 
         // (wider fronts: LW lanes each, the updates flattened over them)
         auto rest = [&](auto width, int cap, int r0, int r1, int ctr) {
             constexpr int LW = decltype(width)::value;
-            unsigned char *gbase = wbase + (size_t)(lane / LW) * warp_area_bytes<double>(cap);
-            double *F = reinterpret_cast<double *>(gbase);
-            int *piv = reinterpret_cast<int *>(gbase + warp_front_bytes<double>(cap));
+            unsigned char *gbase = wbase + (size_t)(lane / LW) * warp_area_bytes<T>(cap);
+            T *F = reinterpret_cast<T *>(gbase);
+            int *piv = reinterpret_cast<int *>(gbase + warp_front_bytes<T>(cap));
             bool more = true;
             while (more) {
                 if (!claim_group<LW>(D, mask, want, M, r0, r1, ctr, g, more)) continue;
-                factor_front<double, true>(
+                factor_front<T, RHS>(
                     P, W, S, fronts, lfac, ufac, g.s, g.m, F, piv, LaneGroup<LW>{g.act},
                     [&] {
                         if (!group_wait_children<LW>(S, D, D.fdone, g.s, g.m, M, epoch) && (lane & (LW - 1)) == 0 &&
@@ -1696,15 +1712,15 @@ int configure_one(DagGrid &g, int nsm, int tiny_bytes, int small_bytes, int big_
             cudaSuccess || occ < 1)
         return -1;
     g.small = nsm * occ;
+    if (!raise_shared_limit(factor_tiny_kernel<T, R, false>, tiny_bytes) ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, factor_tiny_kernel<T, R, false>, kThreads, tiny_bytes) !=
+            cudaSuccess || occ < 1)
+        return -1;
+    g.tiny = nsm * occ;
     if constexpr (sizeof(T) == 8) {
-        if (!raise_shared_limit(factor_tiny_kernel<false>, tiny_bytes) ||
-            !raise_shared_limit(factor_tiny_kernel<true>, tiny_bytes) ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, factor_tiny_kernel<false>, kThreads, tiny_bytes) !=
-                cudaSuccess || occ < 1)
-            return -1;
-        g.tiny = nsm * occ;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, factor_tiny_kernel<true>, kThreads, tiny_bytes) !=
-                cudaSuccess || occ < 1)
+        if (!raise_shared_limit(factor_tiny_kernel<T, R, true>, tiny_bytes) ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, factor_tiny_kernel<T, R, true>, kThreads,
+                                                          tiny_bytes) != cudaSuccess || occ < 1)
             return -1;
         g.few = nsm * occ;
         if (!raise_shared_limit(factor_mid_kernel<false>, MidShape<T>::bytes) ||
@@ -1742,7 +1758,7 @@ int dag_configure(const DevDag &D, int fp32, DagGrid &g) {
     // not split whole, and the parts of the split ones
     const int mb = std::max(1, fp32 ? D.max_big_front : D.max_big_whole);
     const int small_bytes = kWarps * (fp32 ? warp_area_bytes<float>(kSmallFront) : warp_area_bytes<double>(kSmallFront));
-    const int tiny_bytes = fp32 ? 0 : kWarps * kTinyArea;
+    const int tiny_bytes = kWarps * (fp32 ? tiny_area<float>() : tiny_area<double>());
     const int whole = (fp32 ? big_front_bytes<float>(mb) : big_front_bytes<double>(mb)) + 2 * mb * 4;
     const int part = fp32 ? 0 : ((D.max_part_entries * 8 + 15) & ~15) + D.max_part_ints * 4;
     const int big_bytes = std::max(whole, part);
@@ -1762,7 +1778,10 @@ int dag_configure(const DevDag &D, int fp32, DagGrid &g) {
 }
 
 int dag_factor_launches(const DevDag &D, int M, int fp32) {
-    if (fp32) return (D.n_small > 0) + (D.nsup > D.n_small);
+    if (fp32) {
+        if ((long long)D.n_tiny * M <= kTinyFew32) return (D.n_small > 0) + (D.nsup > D.n_small);
+        return (D.n_tiny > 0) + (D.n_small > D.n_tiny) + (D.nsup > D.n_small);
+    }
     const bool one = (long long)(D.n_small - D.n_tiny) * M <= kMidTasks && D.max_front <= kWideFront;
     if (one) return (D.n_tiny > 0) + (D.nsup > D.n_tiny);
     return (D.n_tiny > 0) + (D.n_small > D.n_tiny) + (D.nsup > D.n_small);
@@ -1788,17 +1807,18 @@ template <class T>
 void launch_dag_factor(const DevProblem &P, const DevWork &W, const DevSym &S, const DevDag &D, const DagGrid &g,
                        T *fronts, T *lfac, T *ufac, const uint8_t *mask, int want, cudaStream_t st) {
     constexpr bool R = FusedRhs<T>::value;
+    const long long tt = std::max((long long)D.n_little * ((P.M + 3) / 4),
+                                  (long long)(D.n_tiny - D.n_little) * ((P.M + 1) / 2)),
+                    tf = (long long)D.n_tiny * P.M, ts = (long long)(D.n_small - D.n_tiny) * P.M;
+    const bool few = tf <= (sizeof(T) == 8 ? kTinyFew : kTinyFew32);
+    if (tf > 0 && !few)
+        factor_tiny_kernel<T, R, false><<<blocks_for(g.tiny, tt, kWarps), kThreads, g.tiny_bytes, st>>>(
+            P, W, S, D, fronts, lfac, ufac, mask, want);
     if constexpr (sizeof(T) == 8) {
-        const long long tt = std::max((long long)D.n_little * ((P.M + 3) / 4),
-                                      (long long)(D.n_tiny - D.n_little) * ((P.M + 1) / 2)),
-                        ts = (long long)(D.n_small - D.n_tiny) * P.M, tb = (long long)D.big_units * P.M;
-        const long long tf = (long long)D.n_tiny * P.M;
-        if (tf > 0 && tf <= kTinyFew)
-            factor_tiny_kernel<true><<<blocks_for(g.few, tf, kWarps), kThreads, g.tiny_bytes, st>>>(
+        const long long tb = (long long)D.big_units * P.M;
+        if (tf > 0 && few)
+            factor_tiny_kernel<T, R, true><<<blocks_for(g.few, tf, kWarps), kThreads, g.tiny_bytes, st>>>(
                 P, W, S, D, fronts, lfac, ufac, mask, want);
-        else if (tt > 0)
-            factor_tiny_kernel<false><<<blocks_for(g.tiny, tt, kWarps), kThreads, g.tiny_bytes, st>>>(P, W, S, D, fronts, lfac,
-                                                                                               ufac, mask, want);
         const bool wide = D.max_front <= kWideFront;
         const long long tw = (long long)(D.nsup - D.n_small) * P.M;
         if (ts > kMidTasks)
@@ -1818,10 +1838,10 @@ void launch_dag_factor(const DevProblem &P, const DevWork &W, const DevSym &S, c
             factor_big_kernel<T, R><<<blocks_for(g.big, tb, 1), kThreads, g.big_bytes, st>>>(
                 P, W, S, D, fronts, lfac, ufac, mask, want);
     } else {
-        const long long ts = (long long)D.n_small * P.M, tb = (long long)(D.nsup - D.n_small) * P.M;
-        if (ts > 0)
-            factor_small_kernel<T, R><<<blocks_for(g.small, ts, kWarps), kThreads, g.small_bytes, st>>>(
-                P, W, S, D, fronts, lfac, ufac, mask, want, 0, D.n_small, kSmallFront, 0);
+        const long long tb = (long long)(D.nsup - D.n_small) * P.M, tl = few ? tf + ts : ts;
+        if (tl > 0)
+            factor_small_kernel<T, R><<<blocks_for(g.small, tl, kWarps), kThreads, g.small_bytes, st>>>(
+                P, W, S, D, fronts, lfac, ufac, mask, want, few ? 0 : D.n_tiny, D.n_small, kSmallFront, 0);
         if (tb > 0)
             factor_big_kernel<T, R><<<blocks_for(g.big, tb, 1), kThreads, g.big_bytes, st>>>(
                 P, W, S, D, fronts, lfac, ufac, mask, want);

@@ -100,6 +100,7 @@ __device__ inline unsigned long long wait_tag(const unsigned long long *p, int e
 // infinite and NaN pivots take the division, so that they give the
 // division's result exactly.
 __device__ __forceinline__ float recip(float x) { return 1.0f / x; }
+__device__ __forceinline__ float recip_normal(float x) { return 1.0f / x; }
 // whether x takes the division
 __device__ __forceinline__ bool recip_special(double x) {
     const unsigned e = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
