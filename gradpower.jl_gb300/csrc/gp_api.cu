@@ -2534,25 +2534,25 @@ int32_t gp_integrate(gp_layout *L, const gp_options *opt, int32_t n_faults, cons
             for (; k < ke; k++) send_slice(k);
             if (d_traj) send_slice(k);
         } else {
-        ck(cudaMemcpyAsync(L->W.zold, L->W.z, (size_t)M * nsys * sizeof(double), cudaMemcpyDeviceToDevice, L->st),
-           "zold");
-        if (predict) {
-            gp::launch_predict(L->W.z, L->W.zold, L->zprev, L->zprev2, L->zprev3, (size_t)M * nsys,
-                               std::min(predict, smooth), L->st);
-            smooth += 1;
-        }
-        ck(cudaMemsetAsync(L->W.active, 1, M, L->st), "memset");
-        solve_step(L, opt->dt, opt->newton_tol, opt->itermax, force);
-        force = false;
-        ck(cudaMemcpyAsync(d_iters + (size_t)(2 * (k - 1)) * M, L->W.iters, M * sizeof(int),
-                           cudaMemcpyDeviceToDevice, L->st),
-           "iters");
-        if (d_traj) {
-            ck(cudaMemcpy2DAsync(d_traj + (size_t)k * nsys, tpitch, L->W.z, nsys * sizeof(double),
-                                 nsys * sizeof(double), M, cudaMemcpyDeviceToDevice, L->st),
-               "snapshot");
-            send_slice(k);
-        }
+            ck(cudaMemcpyAsync(L->W.zold, L->W.z, (size_t)M * nsys * sizeof(double), cudaMemcpyDeviceToDevice, L->st),
+               "zold");
+            if (predict) {
+                gp::launch_predict(L->W.z, L->W.zold, L->zprev, L->zprev2, L->zprev3, (size_t)M * nsys,
+                                   std::min(predict, smooth), L->st);
+                smooth += 1;
+            }
+            ck(cudaMemsetAsync(L->W.active, 1, M, L->st), "memset");
+            solve_step(L, opt->dt, opt->newton_tol, opt->itermax, force);
+            force = false;
+            ck(cudaMemcpyAsync(d_iters + (size_t)(2 * (k - 1)) * M, L->W.iters, M * sizeof(int),
+                               cudaMemcpyDeviceToDevice, L->st),
+               "iters");
+            if (d_traj) {
+                ck(cudaMemcpy2DAsync(d_traj + (size_t)k * nsys, tpitch, L->W.z, nsys * sizeof(double),
+                                     nsys * sizeof(double), M, cudaMemcpyDeviceToDevice, L->st),
+                   "snapshot");
+                send_slice(k);
+            }
         }
         if (ev_steps.count(k)) {
             ck(cudaMemsetAsync(L->W.active, 0, M, L->st), "memset");

@@ -1757,7 +1757,8 @@ int dag_configure(const DevDag &D, int fp32, DagGrid &g) {
     // FP32: every front of the CTA kernel whole; FP64: the fronts that are
     // not split whole, and the parts of the split ones
     const int mb = std::max(1, fp32 ? D.max_big_front : D.max_big_whole);
-    const int small_bytes = kWarps * (fp32 ? warp_area_bytes<float>(kSmallFront) : warp_area_bytes<double>(kSmallFront));
+    const int small_bytes =
+        kWarps * (fp32 ? warp_area_bytes<float>(kSmallFront) : warp_area_bytes<double>(kSmallFront));
     const int tiny_bytes = kWarps * (fp32 ? tiny_area<float>() : tiny_area<double>());
     const int whole = (fp32 ? big_front_bytes<float>(mb) : big_front_bytes<double>(mb)) + 2 * mb * 4;
     const int part = fp32 ? 0 : ((D.max_part_entries * 8 + 15) & ~15) + D.max_part_ints * 4;
