@@ -297,13 +297,6 @@ void launch_fault_status(const DevProblem &P, const int *fl_on_step, const int *
     if (n_fl > 0) fault_status_kernel<<<(n_fl + 255) / 256, 256, 0, st>>>(fl_on_step, fl_off_step, fl_on, n_fl, upto);
 }
 
-int adj_smem_optin(int bytes) {
-    if (cudaFuncSetAttribute(adj_cluster_back_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) !=
-        cudaSuccess) {
-        cudaGetLastError();
-        return -1;
-    }
-    return bytes;
-}
+int adj_smem_optin(int bytes) { return raise_shared_limit(adj_cluster_back_kernel, bytes) ? bytes : -1; }
 
 }  // namespace gp

@@ -1706,8 +1706,7 @@ template <class T>
 int configure_one(DagGrid &g, int nsm, int tiny_bytes, int small_bytes, int big_bytes) {
     constexpr bool R = FusedRhs<T>::value;
     int occ = 0;
-    if (cudaFuncSetAttribute(factor_small_kernel<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, small_bytes) !=
-            cudaSuccess ||
+    if (!raise_shared_limit(factor_small_kernel<T, R>, small_bytes) ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, factor_small_kernel<T, R>, kThreads, small_bytes) !=
             cudaSuccess || occ < 1)
         return -1;
@@ -1734,8 +1733,7 @@ int configure_one(DagGrid &g, int nsm, int tiny_bytes, int small_bytes, int big_
             return -1;
         g.wide = nsm * occ;
     }
-    if (cudaFuncSetAttribute(factor_big_kernel<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, big_bytes) !=
-            cudaSuccess ||
+    if (!raise_shared_limit(factor_big_kernel<T, R>, big_bytes) ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, factor_big_kernel<T, R>, kThreads, big_bytes) !=
             cudaSuccess || occ < 1)
         return -1;

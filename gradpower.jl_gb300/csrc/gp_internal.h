@@ -4,14 +4,20 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
+
 #include "gp_devices.cuh"
 
 namespace gp {
 
 // Raises a kernel's dynamic shared-memory limit to `bytes`; never lowers it
-// (the limit belongs to the kernel, and layouts of other sizes may be alive).
+// (the limit belongs to the kernel, and layouts of other sizes may be alive;
+// one thread at a time, so that two that make layouts do not lower each
+// other's).
 template <class K>
 bool raise_shared_limit(K *kernel, int bytes) {
+    static std::mutex one;
+    const std::lock_guard<std::mutex> lock(one);
     cudaFuncAttributes a;
     if (cudaFuncGetAttributes(&a, kernel) == cudaSuccess &&
         (a.maxDynamicSharedSizeBytes >= bytes ||

@@ -1006,13 +1006,8 @@ int solve_configure(const DevBlk &B, SolveGrid &g) {
     g.blk_bytes = kBlkWarps * blk_layout(B).total;
     g.top_bytes = std::max(g.blk_bytes, top_vec_bytes(std::max(1, B.top_max_front)) +
                                             top_idx_bytes(std::max(1, B.top_max_front), B.top_max_xent) + kTopStage);
-    if (cudaFuncSetAttribute(fwd_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, g.top_bytes) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(bwd_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, g.top_bytes) !=
-            cudaSuccess) {
-        cudaGetLastError();
+    if (!raise_shared_limit(fwd_solve_kernel, g.top_bytes) || !raise_shared_limit(bwd_solve_kernel, g.top_bytes))
         return -1;
-    }
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fwd_solve_kernel, kTopThreads, g.top_bytes) !=
             cudaSuccess || occ < 1)
         return -1;
