@@ -3059,12 +3059,23 @@ int32_t gp_set_line_trips(gp_layout *L, int32_t n, const gp_line_trip *trips) {
                 per_s[fe.first].push_back({(double)fe.second, (double)e, blk[q]});
             }
         }
-    std::vector<int> ap(sym.nsup + 1, 0), apos, atr;
+    std::vector<int> ap(sym.nsup + 1, 0), apos, atr, alen;
     std::vector<double> aval;
     for (int s = 0; s < sym.nsup; s++) {
-        for (const auto &t : per_s[s]) {
+        // a scenario's entries at one position (parallel circuits) together,
+        // in trip order
+        auto key = [&](const std::array<double, 3> &t) { return std::make_pair(scen[(int)t[1]], (int)t[0]); };
+        std::stable_sort(per_s[s].begin(), per_s[s].end(),
+                         [&](const std::array<double, 3> &a, const std::array<double, 3> &b) { return key(a) < key(b); });
+        size_t head = 0;
+        for (size_t i = 0; i < per_s[s].size(); i++) {
+            const auto &t = per_s[s][i];
+            const bool same = i > 0 && key(t) == key(per_s[s][i - 1]);
+            if (!same) head = apos.size();
             apos.push_back((int)t[0]);
             atr.push_back((int)t[1]);
+            alen.push_back(0);
+            alen[head]++;
             aval.push_back(t[2]);
         }
         ap[s + 1] = (int)apos.size();
@@ -3090,9 +3101,10 @@ int32_t gp_set_line_trips(gp_layout *L, int32_t n, const gp_line_trip *trips) {
         L->S.asmt_ptr = up_i(ap);
         L->S.asmt_pos = up_i(apos);
         L->S.asmt_tr = up_i(atr);
+        L->S.asmt_len = up_i(alen);
         L->S.asmt_val = A.upload(aval.empty() ? std::vector<double>{0.0} : aval);
     } else {
-        L->S.asmt_ptr = L->S.asmt_pos = L->S.asmt_tr = nullptr;
+        L->S.asmt_ptr = L->S.asmt_pos = L->S.asmt_tr = L->S.asmt_len = nullptr;
         L->S.asmt_val = nullptr;
     }
     drop_graphs(L);   // the graphs hold the problem and structure by value

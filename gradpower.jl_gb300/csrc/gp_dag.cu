@@ -43,6 +43,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "gp_front.cuh"
 #include "gp_internal.h"
 #include "gp_warp.cuh"
 
@@ -514,10 +515,7 @@ __device__ void factor_front(const DevProblem &P, const DevWork &W, const DevSym
     const double *sv = W.svar + (size_t)m * P.n_var;
     for (int e = S.asmv_ptr[s] + idx; e < S.asmv_ptr[s + 1]; e += step) F[S.asmv_pos[e]] += (T)sv[S.asmv_idx[e]];
     if (S.asmt_ptr)
-        for (int e = S.asmt_ptr[s] + idx; e < S.asmt_ptr[s + 1]; e += step) {
-            const int t = S.asmt_tr[e];
-            if (P.tr_on[t] && t >= P.tr_ptr[m] && t < P.tr_ptr[m + 1]) F[S.asmt_pos[e]] += (T)S.asmt_val[e];
-        }
+        for (int e = S.asmt_ptr[s] + idx; e < S.asmt_ptr[s + 1]; e += step) add_trips(P, S, m, e, F + S.asmt_pos[e]);
     g.sync();
     // the entries above need nothing from the children: only now wait for
     // them (bounded; wait() ends with a barrier of the group)
@@ -818,11 +816,8 @@ __device__ void factor_part(const DevProblem &P, const DevWork &W, const DevSym 
     }
     if (S.asmt_ptr)
         for (int q = S.asmt_ptr[s] + tid; q < S.asmt_ptr[s + 1]; q += nthr) {
-            const int t = S.asmt_tr[q];
-            if (P.tr_on[t] && t >= P.tr_ptr[m] && t < P.tr_ptr[m + 1]) {
-                const int e = local(S.asmt_pos[q]);
-                if (e >= 0) Fl[e] += (T)S.asmt_val[q];
-            }
+            const int e = local(S.asmt_pos[q]);
+            if (e >= 0) add_trips(P, S, m, q, Fl + e);
         }
     __syncthreads();
     wait();
@@ -1091,10 +1086,7 @@ __device__ void factor_rows(const DevProblem &P, const DevWork &W, const DevSym 
     const double *sv = W.svar + (size_t)m * P.n_var;
     for (int e = S.asmv_ptr[s] + lane; e < S.asmv_ptr[s + 1]; e += LW) F[S.asmv_pos[e]] += (T)sv[S.asmv_idx[e]];
     if (S.asmt_ptr)
-        for (int e = S.asmt_ptr[s] + lane; e < S.asmt_ptr[s + 1]; e += LW) {
-            const int t = S.asmt_tr[e];
-            if (P.tr_on[t] && t >= P.tr_ptr[m] && t < P.tr_ptr[m + 1]) F[S.asmt_pos[e]] += (T)S.asmt_val[e];
-        }
+        for (int e = S.asmt_ptr[s] + lane; e < S.asmt_ptr[s + 1]; e += LW) add_trips(P, S, m, e, F + S.asmt_pos[e]);
     __syncwarp();
     wait();   // for the children (bounded); ends with a warp barrier
     // ---- the children's update matrices and vectors, in child order ----
@@ -1269,10 +1261,8 @@ __device__ void factor_mid(const DevProblem &P, const DevWork &W, const DevSym &
     for (int e = S.asmv_ptr[s] + tid; e < S.asmv_ptr[s + 1]; e += kMidThreads)
         F[S.asmv_pos[e]] += (T)sv[S.asmv_idx[e]];
     if (S.asmt_ptr)
-        for (int e = S.asmt_ptr[s] + tid; e < S.asmt_ptr[s + 1]; e += kMidThreads) {
-            const int t = S.asmt_tr[e];
-            if (P.tr_on[t] && t >= P.tr_ptr[m] && t < P.tr_ptr[m + 1]) F[S.asmt_pos[e]] += (T)S.asmt_val[e];
-        }
+        for (int e = S.asmt_ptr[s] + tid; e < S.asmt_ptr[s + 1]; e += kMidThreads)
+            add_trips(P, S, m, e, F + S.asmt_pos[e]);
     // sources of each entry: where its list starts, its length, the offsets
     // of the next kSrc of them
     constexpr int kSrc = 2;

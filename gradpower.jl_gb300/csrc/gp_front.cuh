@@ -1,11 +1,25 @@
-// Backward substitution of one front by a warp, shared by the triangular
-// solves (gp_solve.cu) and the small-system kernel (gp_small.cu).
+// Parts of one front's work that several kernels share: the tripped lines'
+// entries (gp_dag.cu, gp_small.cu) and the backward substitution by a warp
+// (gp_solve.cu, gp_small.cu).
 #pragma once
 #include <cuda_runtime.h>
 
+#include "gp_internal.h"
 #include "gp_warp.cuh"
 
 namespace gp {
+
+// Line-trip entry e of scenario m's front into its place *a.  Threads take
+// entries in any order and at once, so the entries of one scenario at one
+// place (parallel circuits) are all added by the thread of the first
+// (asmt_len; 0 at the others).
+template <class T>
+__device__ __forceinline__ void add_trips(const DevProblem &P, const DevSym &S, int m, int e, T *a) {
+    for (int q = e; q < e + S.asmt_len[e]; q++) {
+        const int t = S.asmt_tr[q];
+        if (P.tr_on[t] && t >= P.tr_ptr[m] && t < P.tr_ptr[m + 1]) *a += (T)S.asmt_val[q];
+    }
+}
 
 template <class T, int J>
 __device__ __forceinline__ T pick(const T (&r)[J], int j) {

@@ -102,8 +102,10 @@ struct DevSym {
     const int *asmv_ptr, *asmv_pos, *asmv_idx;   // variable entries: front position, svar index
     // line-trip entries of the off-diagonal bus blocks: front position,
     // trip entry (its scenario and status in DevProblem), value added while
-    // the line is tripped; null without trips
-    const int *asmt_ptr, *asmt_pos, *asmt_tr;
+    // the line is tripped; asmt_len: how many entries from here on are the
+    // same scenario's at the same position (0: counted by an earlier one);
+    // null without trips
+    const int *asmt_ptr, *asmt_pos, *asmt_tr, *asmt_len;
     const double *asmt_val;
     double *fronts;                   // [M][front_total]
     // solve-ordered copies of the factors, written by the factorisation for

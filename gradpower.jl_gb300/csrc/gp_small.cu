@@ -222,11 +222,8 @@ __global__ void __launch_bounds__(kSmallThreads) small_newton_kernel(DevProblem 
             if (S.asmt_ptr) {
                 // tripped lines' off-diagonal entries
                 for (int s = warp; s < S.nsup; s += kSmallWarps)
-                    for (int e = S.asmt_ptr[s] + lane; e < S.asmt_ptr[s + 1]; e += 32) {
-                        const int t = S.asmt_tr[e];
-                        if (P.tr_on[t] && t >= P.tr_ptr[m] && t < P.tr_ptr[m + 1])
-                            fronts[D.desc[s].w + S.asmt_pos[e]] += S.asmt_val[e];
-                    }
+                    for (int e = S.asmt_ptr[s] + lane; e < S.asmt_ptr[s + 1]; e += 32)
+                        add_trips(P, S, m, e, fronts + D.desc[s].w + S.asmt_pos[e]);
                 __syncthreads();
             }
             for (int l = 0; l < D.n_levels; l++) {
