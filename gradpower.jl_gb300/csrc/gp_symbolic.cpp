@@ -10,6 +10,8 @@
 #include <future>
 #include <queue>
 #include <stdexcept>
+#include <system_error>
+#include <thread>
 
 namespace gp {
 namespace {
@@ -63,6 +65,10 @@ struct ND {
     // sets of at least PAR nodes give one half to another thread (analysis of
     // 70,000 buses on eight cores 630 -> 295 ms, of 2,000 20 -> 10)
     static constexpr int PAR = 200;
+    // threads that may be started beside the caller's: a core each, and as
+    // many again for those that wait for their half; the rest runs inline,
+    // as where a thread cannot be had
+    std::atomic<int> spare{2 * (int)std::max(1u, std::thread::hardware_concurrency())};
     int set_of(int v) const { return set_id[v].load(std::memory_order_relaxed); }
     void assign(const std::vector<int> &V, int id) {
         for (int v : V) set_id[v].store(id, std::memory_order_relaxed);
@@ -308,14 +314,23 @@ struct ND {
         assign(A, ida);
         assign(B, idb);
         assign(S, ids);
+        std::vector<int> ob;
+        std::future<void> half;
         if ((int)V.size() >= PAR) {
-            std::vector<int> ob;
-            auto half = std::async(std::launch::async, [&] { run(B, idb, pass_id, ob); });
-            run(A, ida, pass_id, order);
+            if (spare.fetch_sub(1) > 0) {
+                try {
+                    half = std::async(std::launch::async, [&] { run(B, idb, pass_id, ob); });
+                } catch (const std::system_error &) {   // (the process may start no more threads)
+                }
+            }
+            if (!half.valid()) spare.fetch_add(1);
+        }
+        run(A, ida, pass_id, order);
+        if (half.valid()) {
             half.get();
+            spare.fetch_add(1);
             order.insert(order.end(), ob.begin(), ob.end());
         } else {
-            run(A, ida, pass_id, order);
             run(B, idb, pass_id, order);
         }
         // separator nodes: order them by minimum degree in chunks
