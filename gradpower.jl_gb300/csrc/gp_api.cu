@@ -131,10 +131,12 @@ struct gp_layout {
     size_t traj_cap = 0;
     cudaStream_t st_copy = nullptr;
     cudaEvent_t ev_snap = nullptr;
-    // workspace of gp_adjoint (kept between calls, grown on demand)
+    // workspace of gp_adjoint (kept between calls, grown on demand), and the
+    // caller's limit on it (gp_set_adjoint_memory; negative: none)
     DeviceArena adj_arena;
     double *adj_buf = nullptr;
     size_t adj_bytes = 0;
+    int64_t adj_limit = -1;
     double *d_zl_k = nullptr;   // DevProblem::zl_k
     int *d_state_maps = nullptr;   // state_bus then red_of
     int *d_gen_w = nullptr;        // z index of every machine's speed deviation
@@ -2199,6 +2201,16 @@ std::map<int, std::vector<uint8_t>> event_masks(const gp_layout *L) {
     return ev;
 }
 
+// Gives back an adjoint workspace larger than the layout may keep between
+// calls.
+void trim_adjoint(gp_layout *L) {
+    constexpr size_t kAdjKeep = size_t(4) << 30;
+    if (L->adj_bytes <= (L->adj_limit < 0 ? kAdjKeep : std::min(kAdjKeep, (size_t)L->adj_limit))) return;
+    cudaStreamSynchronize(L->st);
+    L->adj_arena.release();
+    L->adj_bytes = 0;
+}
+
 // One transposed Newton-Jacobian solve of the adjoint for the active
 // scenarios at the state z (time step dt, current fault status):
 // g holds the right-hand side on entry and E lambda on exit; lambda and the
@@ -2807,10 +2819,14 @@ int32_t gp_adjoint(gp_layout *L, const gp_options *opt, int32_t n_faults, const 
     // device copies of the re-solve masks
     std::map<int, uint8_t *> d_mask;
     for (const auto &kv : ev) d_mask[kv.first] = L->call.upload(kv.second);
-    // the states of every solve are kept when they fit a quarter of the free
-    // device memory; else the checkpoints (at steps 0, K, 2K, ...) and one
-    // segment's.  The workspace stays with the layout, up to kAdjKeep bytes
-    constexpr size_t kAdjKeep = size_t(4) << 30;
+    // the states of every solve are kept when they fit the caller's limit, by
+    // default a quarter of the free device memory; else the checkpoints (at
+    // steps 0, K, 2K, ...) and one segment's.  What the layout may not keep
+    // goes at the end, on every path
+    struct Trim {
+        gp_layout *L;
+        ~Trim() { trim_adjoint(L); }
+    } trim{L};
     const int nck = (ns + K - 1) / K;
     std::map<int, int> ev_slot;   // event step -> its re-solve state's slot
     for (const auto &kv : ev) {
@@ -2820,7 +2836,8 @@ int32_t gp_adjoint(gp_layout *L, const gp_options *opt, int32_t n_faults, const 
     const size_t n_all = (size_t)ns + ev.size(), n_seg = nck + (size_t)2 * K;
     size_t mem_free = 0, mem_total = 0;
     ck(cudaMemGetInfo(&mem_free, &mem_total), "memory info");
-    const bool keep_all = n_all <= n_seg || n_all * blk * sizeof(double) <= (mem_free + L->adj_bytes) / 4;
+    const size_t state_limit = L->adj_limit < 0 ? (mem_free + L->adj_bytes) / 4 : (size_t)L->adj_limit;
+    const bool keep_all = n_all <= n_seg || n_all * blk * sizeof(double) <= state_limit;
     DevClu Cs = L->C;
     Cs.n_save = 1;
     for (int v : L->cplan.rhs_base) Cs.n_save = std::max(Cs.n_save, v);
@@ -2966,10 +2983,15 @@ int32_t gp_adjoint(gp_layout *L, const gp_options *opt, int32_t n_faults, const 
     if (grad_p && L->n_par > 0)
         to_host(L, grad_p, A.grad, (size_t)M * L->n_par * sizeof(double), "grad copy");
     if (grad_z0) to_host(L, grad_z0, A.g, blk * sizeof(double), "grad z0 copy");
-    if (L->adj_bytes > kAdjKeep) {
-        L->adj_arena.release();
-        L->adj_bytes = 0;
-    }
+    API_END
+}
+
+int32_t gp_set_adjoint_memory(gp_layout *L, int64_t bytes) {
+    API_BEGIN
+    if (!L) fail(GP_E_INVALID, "null argument");
+    DeviceScope dev(L);
+    L->adj_limit = bytes;
+    trim_adjoint(L);
     API_END
 }
 

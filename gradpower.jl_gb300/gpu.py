@@ -60,12 +60,13 @@ def library():
         L.gp_set_device_disconnects.argtypes = [vp, C.c_int32, vp]
         L.gp_initialize.argtypes = [vp] * 7
         L.gp_adjoint.argtypes = [vp, vp, C.c_int32, vp, vp, C.c_int32, vp, vp, vp, vp]
+        L.gp_set_adjoint_memory.argtypes = [vp, C.c_int64]
         L.gp_recip_check.argtypes = [C.c_int32, vp, vp]
         for f in ("gp_layout_create", "gp_layout_destroy", "gp_layout_stats", "gp_set_state",
                   "gp_get_state", "gp_integrate", "gp_residual", "gp_last_timing",
                   "gp_restore_initial_state", "gp_reduced_selftest", "gp_cluster_selftest",
                   "gp_residual_static", "gp_set_mixed_policy", "gp_set_profiling", "gp_set_wait_limit",
-                  "gp_set_line_trips",
+                  "gp_set_adjoint_memory", "gp_set_line_trips",
                   "gp_set_device_disconnects", "gp_initialize", "gp_adjoint", "gp_recip_check"):
             getattr(L, f).restype = C.c_int32
         _lib = L
@@ -170,6 +171,13 @@ class GpuBatchedLayout:
         in include/gradpower_gb300.h); the call then raises GradPowerError
         with GP_E_TIMEOUT and the waiting scenarios get status bit 8."""
         _check(library().gp_set_wait_limit(self._h, int(polls)))
+
+    def set_adjoint_memory(self, limit_bytes: Optional[int] = None):
+        """Device memory adjoint() may take for the forward run's states (see
+        gp_set_adjoint_memory in include/gradpower_gb300.h): above it, or
+        with 0, it keeps the states every `checkpoint_every` steps and
+        recomputes the others.  None: a quarter of the free memory."""
+        _check(library().gp_set_adjoint_memory(self._h, -1 if limit_bytes is None else max(0, int(limit_bytes))))
 
     def set_profiling(self, on: bool = True):
         """Host-driven Newton loop with CUDA events around every phase (for

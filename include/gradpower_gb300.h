@@ -338,9 +338,10 @@ typedef struct gp_objective {
  * backwards with one transposed Newton-Jacobian solve per forward solve
  * (regular steps and dt = 0 event re-solves) at its converged state and
  * fault status.  The states of every solve are kept when they fit
- * a quarter of the free device memory; else the state every
- * checkpoint_every steps, and the sweep recomputes the steps between (the
- * same values either way).
+ * a quarter of the free device memory (or gp_set_adjoint_memory's limit);
+ * else the state every checkpoint_every steps, and the sweep recomputes the
+ * steps between (the same values either way).  The workspace stays with the
+ * layout up to 4 GiB.
  *   J        [M] objective value
  *   grad_p   [M][n_par] dJ/dp at the fixed initial state: filled for the
  *            machine inertia H and damping D (GENROU/GENSAL), the exciter
@@ -357,6 +358,14 @@ typedef struct gp_objective {
 int32_t gp_adjoint(gp_layout *L, const gp_options *opt, int32_t n_faults, const gp_fault *faults,
                    const gp_objective *obj, int32_t checkpoint_every, double *J, double *grad_p, double *grad_z0,
                    int32_t *status);
+
+/* Device memory of gp_adjoint's states: with bytes >= 0 the states of every
+ * solve are kept only when they take at most so many bytes (0: checkpoints
+ * alone, whenever those take less), and a larger workspace does not stay
+ * with the layout after a call.  Negative (the default): a quarter of the
+ * free device memory, and up to 4 GiB stay.  No counterpart in the
+ * reference. */
+int32_t gp_set_adjoint_memory(gp_layout *L, int64_t bytes);
 
 /* Policy of GP_SOLVER_SCHUR_MIXED (no counterpart in the reference, whose
  * solvers refactor every iteration):
