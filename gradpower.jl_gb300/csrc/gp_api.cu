@@ -67,7 +67,10 @@ struct DeviceArena {
     void *raw(size_t bytes) {
         void *p = nullptr;
         const cudaError_t e = cudaMalloc(&p, bytes);
-        if (e != cudaSuccess) fail(GP_E_NOMEM, "cudaMalloc of %zu bytes: %s", bytes, cudaGetErrorString(e));
+        if (e != cudaSuccess) {
+            cudaGetLastError();   // told here: a later call's launch check must not find it
+            fail(GP_E_NOMEM, "cudaMalloc of %zu bytes: %s", bytes, cudaGetErrorString(e));
+        }
         ptrs.push_back(p);
         return p;
     }
