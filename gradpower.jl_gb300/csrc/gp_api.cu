@@ -106,6 +106,19 @@ struct DeviceArena {
     }
 };
 
+// An arena's new contents: they take the place of the old ones at commit();
+// without it (an allocation failed) the old ones stay.
+struct ArenaSwap {
+    DeviceArena fresh;
+    DeviceArena &into;
+    explicit ArenaSwap(DeviceArena &a) : into(a) { fresh.st = a.st; }
+    ~ArenaSwap() { fresh.release(); }
+    void commit() {
+        into.release();
+        std::swap(into, fresh);
+    }
+};
+
 std::vector<int> vec(const int32_t *p, int n) {
     std::vector<int> v(n > 0 ? n : 0);
     if (n > 0 && p) std::copy(p, p + n, v.begin());
@@ -1757,9 +1770,11 @@ void set_faults(gp_layout *L, int n_faults, const gp_fault *faults) {
     // the captured graphs hold those addresses, and stay valid across calls
     const int cap = std::max(1, L->n_fl);
     if (!L->d_fl_ptr || cap > L->fl_cap) {
+        drop_graphs(L);
         L->fault_arena.release();
+        L->d_fl_ptr = nullptr;   // (nothing to go back to if an allocation fails)
         DeviceArena &A = L->fault_arena;
-        L->d_fl_ptr = A.alloc<int>(M + 1);
+        int *fl_ptr = A.alloc<int>(M + 1);
         L->d_fl_bus = A.alloc<int>(cap);
         L->d_fl_yf = A.alloc<double>(cap);
         L->d_fl_on = A.alloc<uint8_t>(cap);
@@ -1767,11 +1782,10 @@ void set_faults(gp_layout *L, int n_faults, const gp_fault *faults) {
         L->d_fl_off_step = A.alloc<int>(cap);
         L->d_fl_scen = A.alloc<int>(cap);
         L->fl_cap = cap;
-        L->P.fl_ptr = L->d_fl_ptr;
+        L->P.fl_ptr = L->d_fl_ptr = fl_ptr;
         L->P.fl_bus = L->d_fl_bus;
         L->P.fl_yf = L->d_fl_yf;
         L->P.fl_on = L->d_fl_on;
-        drop_graphs(L);
     }
     auto put = [&](void *d, const void *h, size_t bytes) {
         if (bytes) to_device(L, d, h, bytes, "fault table");
@@ -2018,7 +2032,7 @@ void ensure_mixed(gp_layout *L) {
 
 // Buffers of the shared-factor Woodbury path, allocated on its first use.
 void ensure_woodbury(gp_layout *L) {
-    if (L->wb_W1) return;
+    if (L->d_only0) return;
     DeviceArena &A = L->arena;
     const size_t M = L->M, nr = std::max(1, L->P.n_red);
     L->wb_W1 = A.alloc<double>(M * nr);
@@ -2463,6 +2477,7 @@ int32_t gp_integrate(gp_layout *L, const gp_options *opt, int32_t n_faults, cons
     const size_t n_it = (size_t)2 * std::max(ns, 1) * M;
     if (n_it > L->iters_cap) {
         L->iters_arena.release();
+        L->iters_cap = 0;
         L->d_iters_buf = L->iters_arena.alloc<int>(n_it);
         L->iters_cap = n_it;
     }
@@ -2476,6 +2491,7 @@ int32_t gp_integrate(gp_layout *L, const gp_options *opt, int32_t n_faults, cons
         const size_t need = (size_t)M * (ns + 1) * nsys;
         if (need > L->traj_cap) {
             L->traj_arena.release();
+            L->traj_cap = 0;
             L->d_traj = L->traj_arena.alloc<double>(need);
             L->traj_cap = need;
         }
@@ -3105,33 +3121,41 @@ int32_t gp_set_line_trips(gp_layout *L, int32_t n, const gp_line_trip *trips) {
         }
         ap[s + 1] = (int)apos.size();
     }
-    L->trip_arena.release();
-    DeviceArena &A = L->trip_arena;
+    ArenaSwap swap(L->trip_arena);
+    DeviceArena &A = swap.fresh;
     auto up_i = [&](const std::vector<int> &v) { return A.upload(v.empty() ? std::vector<int>{0} : v); };
-    L->n_tr = (int)fb.size();
-    L->P.n_tr = L->n_tr;
-    L->P.tr_ptr = up_i(ptr);
-    L->P.tr_from = up_i(fb);
-    L->P.tr_to = up_i(tb);
-    L->P.tr_y = A.upload(y.empty() ? std::vector<double>{0.0} : y);
-    L->d_tr_on = A.alloc<uint8_t>(std::max(1, L->n_tr));
-    fill(L, L->d_tr_on, 0, std::max(1, L->n_tr));
-    L->P.tr_on = L->d_tr_on;
-    L->d_tr_on_step = up_i(on);
-    L->d_tr_off_step = up_i(off);
-    L->d_tr_scen = up_i(scen);
+    const int n_tr = (int)fb.size();
+    gp::DevProblem P = L->P;
+    gp::DevSym S = L->S;
+    P.n_tr = n_tr;
+    P.tr_ptr = up_i(ptr);
+    P.tr_from = up_i(fb);
+    P.tr_to = up_i(tb);
+    P.tr_y = A.upload(y.empty() ? std::vector<double>{0.0} : y);
+    uint8_t *tr_on = A.alloc<uint8_t>(std::max(1, n_tr));
+    fill(L, tr_on, 0, std::max(1, n_tr));
+    P.tr_on = tr_on;
+    int *on_step = up_i(on), *off_step = up_i(off), *tr_scen = up_i(scen);
+    if (n_tr > 0) {
+        S.asmt_ptr = up_i(ap);
+        S.asmt_pos = up_i(apos);
+        S.asmt_tr = up_i(atr);
+        S.asmt_len = up_i(alen);
+        S.asmt_val = A.upload(aval.empty() ? std::vector<double>{0.0} : aval);
+    } else {
+        S.asmt_ptr = S.asmt_pos = S.asmt_tr = S.asmt_len = nullptr;
+        S.asmt_val = nullptr;
+    }
+    swap.commit();
+    L->P = P;
+    L->S = S;
+    L->n_tr = n_tr;
+    L->d_tr_on = tr_on;
+    L->d_tr_on_step = on_step;
+    L->d_tr_off_step = off_step;
+    L->d_tr_scen = tr_scen;
     L->h_tr_on_step = on;
     L->h_tr_off_step = off;
-    if (L->n_tr > 0) {
-        L->S.asmt_ptr = up_i(ap);
-        L->S.asmt_pos = up_i(apos);
-        L->S.asmt_tr = up_i(atr);
-        L->S.asmt_len = up_i(alen);
-        L->S.asmt_val = A.upload(aval.empty() ? std::vector<double>{0.0} : aval);
-    } else {
-        L->S.asmt_ptr = L->S.asmt_pos = L->S.asmt_tr = L->S.asmt_len = nullptr;
-        L->S.asmt_val = nullptr;
-    }
     drop_graphs(L);   // the graphs hold the problem and structure by value
     API_END
 }
@@ -3213,27 +3237,29 @@ int32_t gp_set_device_disconnects(gp_layout *L, int32_t n, const gp_device_disco
             idx.push_back((int)(base + (size_t)m * stride + row));
         }
     }
-    L->dc_arena.release();
-    DeviceArena &A = L->dc_arena;
-    L->n_dc = (int)on.size();
-    L->h_dc_on_step = on;
-    if (L->n_dc > 0) {
-        auto up_i = [&](const std::vector<int> &v) { return A.upload(v); };
-        L->dc_bytes = bytes;
-        L->d_dc_flags = A.alloc<uint8_t>(std::max<size_t>(1, bytes));
-        fill(L, L->d_dc_flags, 0, std::max<size_t>(1, bytes));
-        L->d_dc_on_step = up_i(on);
-        L->d_dc_scen = up_i(scen);
-        L->d_dc_idx = up_i(idx);
-        L->P.zl_off = L->d_dc_flags + o_zl;
-        L->P.sg_off = L->d_dc_flags + o_sg;
-        L->P.exc_off = L->d_dc_flags + o_cl;
-    } else {
-        L->dc_bytes = 0;
-        L->d_dc_flags = nullptr;
-        L->d_dc_on_step = L->d_dc_scen = L->d_dc_idx = nullptr;
-        L->P.zl_off = L->P.sg_off = L->P.exc_off = nullptr;
+    ArenaSwap swap(L->dc_arena);
+    DeviceArena &A = swap.fresh;
+    const int n_dc = (int)on.size();
+    uint8_t *flags = nullptr;
+    int *on_step = nullptr, *dc_scen = nullptr, *dc_idx = nullptr;
+    if (n_dc > 0) {
+        flags = A.alloc<uint8_t>(std::max<size_t>(1, bytes));
+        fill(L, flags, 0, std::max<size_t>(1, bytes));
+        on_step = A.upload(on);
+        dc_scen = A.upload(scen);
+        dc_idx = A.upload(idx);
     }
+    swap.commit();
+    L->n_dc = n_dc;
+    L->h_dc_on_step = on;
+    L->dc_bytes = n_dc > 0 ? bytes : 0;
+    L->d_dc_flags = flags;
+    L->d_dc_on_step = on_step;
+    L->d_dc_scen = dc_scen;
+    L->d_dc_idx = dc_idx;
+    L->P.zl_off = flags ? flags + o_zl : nullptr;
+    L->P.sg_off = flags ? flags + o_sg : nullptr;
+    L->P.exc_off = flags ? flags + o_cl : nullptr;
     drop_graphs(L);   // the graphs hold the problem by value
     API_END
 }

@@ -1,9 +1,12 @@
-"""A call that asks for more memory than the device has (the checkpoints of
-10^9 steps) ends with that error, and the calls after it are not told of it."""
+"""A call that asks for more memory than the device has (checkpoints,
+trajectories or counts of 10^6 to 2 10^9 steps) ends with that error, and the
+calls after it are not told of it."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
-from helpers import DT, synthetic_case
+from helpers import DT, LY, synthetic_case
 
 pytestmark = pytest.mark.gpu
 
@@ -28,3 +31,27 @@ def test_call_after_a_failed_allocation():
             gbl.restore_initial_state()
     finally:
         gbl.close()
+
+
+@pytest.mark.parametrize("name,M_,steps,want_traj", [("planar2k", 6, 10 ** 6, True),
+                                                     ("two_bus", 40, 2 * 10 ** 9, False)])
+def test_shorter_call_after_a_buffer_could_not_grow(name, M_, steps, want_traj):
+    """The trajectory buffer (550 GB asked for) or the Newton counts' (640 GB)
+    fails to grow; a call that had fitted before still has its buffer."""
+    from gradpower_gb300 import build, gpu
+    build.build()
+    c, _ = synthetic_case(name, M_)
+    gbl = gpu.GpuBatchedLayout(c.dp, c.ps, c.M)
+    try:
+        ref = gbl.integrate(6 * DT, DT, scenario_faults=c.faults)
+        fa, nf = c.fault_array(DT)
+        opt = LY.GpOptions(DT, steps, 1e-10, 30, LY.SOLVER_SCHUR_FP64)
+        traj = np.zeros(16)
+        gbl.restore_initial_state()
+        rc = gpu.library().gp_integrate(gbl._h, C.byref(opt), nf, C.addressof(fa),
+                                        traj.ctypes.data if want_traj else None, None, None)
+        assert rc == -3 and np.all(traj == 0.0)
+        r = gbl.integrate(6 * DT, DT, scenario_faults=c.faults)
+    finally:
+        gbl.close()
+    assert np.array_equal(r["traj"], ref["traj"]) and np.array_equal(r["iters"], ref["iters"])
