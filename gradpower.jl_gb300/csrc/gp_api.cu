@@ -1657,10 +1657,8 @@ void build_clusters(gp_layout *L, const gp_problem *pr, const double *z0, const 
     C.slot_of = A.upload(cp.slot_of);
     C.prog_ptr = A.upload(cp.prog_ptr);
     C.prog_mid = A.upload(cp.prog_mid);
-    C.prog_sol = A.upload(cp.prog_sol);
     C.ops = A.upload(cp.ops);
     C.rhs_base = A.upload(cp.rhs_base);
-    C.nslot = A.upload(cp.nslot);
     C.perm_col = A.upload(cp.perm_col);
     C.pos3 = A.upload(cp.pos3);
     {

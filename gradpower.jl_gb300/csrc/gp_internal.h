@@ -139,10 +139,8 @@ struct DevClu {
     const short *slot_of;       // [class][32*32] slot of local entry (r, c); c = 29/30 B, 31 f
     const int *prog_ptr;        // [n_class+1]
     const int *prog_mid;        // [n_class] first op of the factorisation part
-    const int *prog_sol;        // [n_class] first op of the solve part (after the factorisation)
     const CluOp *ops;
     const int *rhs_base;        // [n_class] first right-hand-side slot
-    const int *nslot;           // [n_class] slots used (values + pivots + 3 W)
     const int *perm_col;        // [class][32] state (local) of solution position j
     const int *pos3;            // [class][3] solution positions of delta, i_q, i_d
     const int *row_pos;         // [class][32] position of local row r in the program
@@ -414,7 +412,6 @@ void launch_predict(double *z, const double *zold, double *zprev, double *zprev2
 void launch_update(const DevProblem &P, const DevWork &W, const DevSym &S, const int *perm, cudaStream_t st);
 void launch_events(const DevProblem &P, const DevWork &W, const int *fl_on_step, const int *fl_off_step,
                    const int *fl_scen, uint8_t *fl_on, int n_fl, int step, cudaStream_t st);
-void launch_snapshot(const double *z, double *traj, int M, int n_sys, int n_steps, int k, cudaStream_t st);
 int cluster_smem_optin(int bytes);
 
 // Small systems, one CTA a scenario (gp_small.cu).
