@@ -1474,8 +1474,9 @@ __global__ void __launch_bounds__(kThreads, 6) factor_small_kernel(DevProblem P,
 // group of lanes factors one of them.  A group whose scenario this launch
 // does not factor (M not a multiple, or masked out) follows the task's first
 // factored scenario and stores nothing.
-//  - the mini region (fronts of at most kMiniFront rows, two thirds of the
-//    supernodes): four scenarios a warp, a lane a row (factor_rows);
+//  - the mini region (fronts of at most kMiniFront rows; 257 of the 681
+//    supernodes of 2,000 buses, 8,491 of the 23,565 of 70,000): four
+//    scenarios a warp, a lane a row (factor_rows);
 //  - the rest, up to kLittleFront rows four, above two scenarios a warp
 //    (factor_front: its flattened updates waste fewer lanes from about ten
 //    rows on; a lane a row for 9 to 16 rows measured 339 us against about

@@ -76,7 +76,7 @@ struct ND {
     // sets of at most LEAF nodes are ordered by minimum degree as a whole;
     // separators and sets that do not split, in chunks of CHUNK.  LEAF 6
     // against 48: the tree of the 39-bus ring has 4 levels instead of 6, the
-    // one of 70,000 buses 23,567 supernodes instead of 26,477 and 14 levels
+    // one of 70,000 buses 23,565 supernodes instead of 26,477 and 13 levels
     // instead of 16; FP64 runs of 70,000 buses x 8 57.0 -> 50.6 ms, 2,000 x
     // 64 39.2 -> 34.6.  (8: 4 and 23,775; 4 and 3 have fewer flops but more
     // supernodes.)

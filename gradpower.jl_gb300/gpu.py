@@ -217,7 +217,10 @@ class GpuBatchedLayout:
                   scenario_trips: Optional[Sequence[Sequence[Mdl.TripLineEvent]]] = None,
                   disconnect_events: Sequence[Mdl.DisconnectDeviceEvent] = (),
                   scenario_disconnects: Optional[Sequence[Sequence[Mdl.DisconnectDeviceEvent]]] = None):
-        """Integrate every scenario from the current state.  `traj_out`, if
+        """Integrate every scenario from the current state.  `solver`: exact
+        FP64 Newton steps (the default, the fastest for a few dozen buses) or
+        LY.SOLVER_SCHUR_MIXED (the fastest for grids of thousands of buses:
+        1.4 to 1.8 times FP64 over a window with a fault).  `traj_out`, if
         given, is a C-contiguous float64 array [M, n_steps+1, n_sys] (for
         example a pinned buffer) that receives the trajectories.
         `trip_events` (every scenario, the reference's ps.dynamic.trip_events)

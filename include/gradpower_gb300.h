@@ -304,7 +304,9 @@ int32_t gp_set_profiling(gp_layout *L, int32_t on);
  * GP_E_TIMEOUT.  The next call clears the flag and starts afresh.  polls >=
  * 1; GP_E_INVALID otherwise.  No counterpart in the reference (cuDSS has no
  * such wait); a failure-detection hook: a tiny limit makes the waits run
- * out without anything on the GPU hanging. */
+ * out without anything on the GPU hanging.  Without effect where there are
+ * no such waits: small systems' FP64 integrations (and the adjoint's forward
+ * run), whose scenarios run in one CTA each while profiling is off. */
 int32_t gp_set_wait_limit(gp_layout *L, int32_t polls);
 
 /* Time of the last gp_integrate call split by phase, milliseconds between
